@@ -17,6 +17,7 @@
 #include "local.cuh"
 #include "mpnn.cuh"
 #include "rap.cuh"
+#include "dcg_plan.h"
 #include "solver.h"
 #include "structure.h"
 
@@ -693,6 +694,32 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
       std::memcpy(contrib_idx, g.contrib_idx.data(), sizeof(int32_t) * g.contrib_idx.size());
       std::memcpy(contrib_off, g.contrib_off.data(), sizeof(int32_t) * g.contrib_off.size());
     }
+  });
+}
+
+int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv,
+                               const float* x_ref, const int32_t* prob, int32_t n_prob,
+                               int32_t n_blocks, int32_t cluster, int32_t threads,
+                               int32_t smem_limit, const float* gradC, const float* invm,
+                               const float* alpha, const float* x, double* y, int32_t* info) {
+  if (!t_i || nt <= 0 || n4 < 0 || n4 > nt || nv <= 0 || !x_ref || n_prob <= 0 || n_blocks <= 0 ||
+      n_blocks > (cluster ? mgpbd::kDMaxCluster : 255) || threads < 128 ||
+      threads > mgpbd::kDMaxThreads || threads % 128 != 0 || !gradC || !invm || !alpha || !x || !y ||
+      !info)
+    return MGPBD_EINVAL;
+  return guarded([&] {
+    mgpbd::DcgPlan p;
+    mgpbd::require(mgpbd::build_dcg_plan(t_i, nt, n4, nv, x_ref, prob, n_prob, n_blocks, cluster != 0,
+                                         threads, smem_limit, p),
+                   MGPBD_ERANGE, "a block's vectors do not fit");
+    mgpbd::dcg_plan_apply(p, gradC, invm, alpha, x, y);
+    int32_t least = nt, most = 0;
+    for (const mgpbd::DBlock& b : p.blocks) {
+      least = std::min(least, 4 * b.nT + 2 * b.nE);
+      most = std::max(most, 4 * b.nT + 2 * b.nE);
+    }
+    const int32_t v[6] = {p.onchip, p.smem, p.srows, p.kT, least, most};
+    std::memcpy(info, v, sizeof v);
   });
 }
 

@@ -10,16 +10,9 @@
 // warp 0 of every block sums all partials in the same fixed order, so all
 // blocks hold bit-identical scalars and take the same branch.
 //
-// Staging: when the mesh is small enough (up to ~400k tets on 152 SMs),
-// each block owns a contiguous range of vertices (balanced by incident
-// entries plus a per-vertex weight) and of tets (32-aligned), and copies
-// their constant operator data into shared memory once per solve: the
-// vertex-major entries (gradient, tet id), the incidence offsets and
-// weights, and the tet indices.  A phase then issues only the gathers of the vector it applies
-// A to (x_t in the vertex phase, u_v in the tet phase) plus the coalesced
-// per-tet loads, instead of two or three dependent L2 round trips.
-// Larger meshes run the same phases reading everything from L2, with tets
-// and vertices strided over the grid.
+// Every phase reads the operator from L2, tets and vertices strided over the
+// grid.  Meshes whose partition fits the kernel of dcg.cu run that one, which
+// keeps the operator on the chip; this one takes the others.
 //
 // Arithmetic is float32 per element (GB300's float64 rate is a small
 // fraction of its float32 rate).  Dot products sum in float32 within a warp
@@ -44,17 +37,11 @@ namespace {
 using namespace jdev;
 using namespace pdev;
 
-// Staged: one block of kPT threads per SM, up to 112 registers a thread,
-// so each thread can issue the gathers of several tets (vertices) before
-// it uses them, and 152 arrivals per grid barrier.  Unstaged: two blocks
-// per SM (56 registers a thread): the phases wait on L2 gathers, and twice
-// the resident warps hide more of that latency than the extra registers
-// would.
+// Two blocks per SM (56 registers a thread): the phases wait on L2 gathers,
+// and twice the resident warps hide more of that latency than the extra
+// registers would.
 constexpr int kPT = 576;
 constexpr int kTB = 4;   // tets a thread handles per round of a tet phase
-constexpr int kVS = 4;   // lanes per vertex in the staged vertex phase
-constexpr int kVE = 6;   // entries a lane gathers per vertex and round
-constexpr int kVB = 4;   // vertices a lane group handles per round
 constexpr int kVertexCost = 64;  // per-vertex weight of the work split
 
 struct PArgs {
@@ -76,9 +63,6 @@ struct PArgs {
   GridSync* gs;
   CgState* st;
   const JState* js;
-  const int32_t* part_v;  // staged: block vertex ranges (grid + 1)
-  const int32_t* part_t;  // staged: block tet ranges (grid + 1)
-  int32_t emax, tmax, vmax;
   double tol_abs, tol_rel;
   int32_t maxiter, degree;
   int32_t warm;  // 1: start from the x on entry instead of 0
@@ -88,24 +72,13 @@ struct PArgs {
   const JcgCtl* ctl;  // device-side tolerance / limit / start, or null
 };
 
-// (the staged kernel keeps the loads: the flag's test spills a register
-// there, and its operator sits in shared memory anyway)
-template <bool STAGED>
 __device__ __forceinline__ float dinv_of(const PArgs& a, int64_t t) {
-  return (!STAGED && a.unit_dinv) ? 1.0f : __ldg(a.ta.dinv + t);
+  return a.unit_dinv ? 1.0f : __ldg(a.ta.dinv + t);
 }
 
-// This block's share of the work: tets from tbeg to tend in steps of tstep
-// (staged: the block's own range; otherwise strided over the whole grid),
-// and, when staged, its vertex range and the shared-memory copies.
+// This thread's share of the tets: from tbeg to tend in steps of tstep
 struct Own {
   int64_t tbeg, tend, tstep;
-  int32_t tb0;
-  int32_t vb0, nvb;
-  const float4* e;     // entries of the block's vertices
-  const int4* q;       // indices of the block's tets
-  const int32_t* off;  // nvb + 1 entry offsets
-  const float* w;      // nvb vertex weights
 };
 
 __device__ __forceinline__ bool grid_sync(const PArgs& a, unsigned long long& gen) {
@@ -122,21 +95,11 @@ __device__ __forceinline__ float tdot(const TArgs& a, int64_t t, int4 q) {
          (g1.z * u2.x + g1.w * u2.y + g2.x * u2.z) + (g2.y * u3.x + g2.z * u3.y + g2.w * u3.z);
 }
 
-// A t of constraint t: staged blocks use their shared copy of the indices;
-// unstaged, length constraints (t >= n4) take the compact two-vertex path
-template <bool STAGED>
-__device__ __forceinline__ float tdot_any(const PArgs& a, const Own& o, int64_t t);
-
-template <bool STAGED>
-__device__ __forceinline__ int4 tet_q(const PArgs& a, const Own& o, int64_t t) {
-  if (STAGED) return o.q[t - o.tb0];
-  return a.ta.t_i[t];
-}
-
-template <bool STAGED>
-__device__ __forceinline__ float tdot_any(const PArgs& a, const Own& o, int64_t t) {
-  if (!STAGED && t >= a.ta.n4) return jt_edge(a.ta, t);
-  return tdot(a.ta, t, tet_q<STAGED>(a, o, t));
+// (A t) of constraint t; length constraints (t >= n4) take the compact
+// two-vertex path
+__device__ __forceinline__ float tdot_any(const PArgs& a, int64_t t) {
+  if (t >= a.ta.n4) return jt_edge(a.ta, t);
+  return tdot(a.ta, t, a.ta.t_i[t]);
 }
 
 // Warm start, vertex phase in float64: u_v = w_v sum x_t g_{t,l} summed in
@@ -144,37 +107,22 @@ __device__ __forceinline__ float tdot_any(const PArgs& a, const Own& o, int64_t 
 // The residual b - A x of a good start x is a small difference of large
 // terms; float32 sums would bury it in their rounding (~1e-7 of the terms),
 // and CG would then converge to the wrong target.  Runs once per solve.
-template <bool STAGED>
-__device__ __forceinline__ void vphase_warm(const PArgs& a, const Own& o) {
+__device__ __forceinline__ void vphase_warm(const PArgs& a) {
   const int lane = threadIdx.x % 4;
-  int64_t gidx, ngroups, nloop;
-  if (STAGED) {
-    gidx = threadIdx.x / 4;
-    ngroups = blockDim.x / 4;
-    nloop = o.nvb;
-  } else {
-    gidx = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 4;
-    ngroups = (int64_t)gridDim.x * blockDim.x / 4;
-    nloop = a.nv;
-  }
-  for (int64_t base = 0; base < nloop; base += ngroups) {
-    const int64_t lv = base + gidx;
+  const int64_t gidx = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 4;
+  const int64_t ngroups = (int64_t)gridDim.x * blockDim.x / 4;
+  for (int64_t base = 0; base < a.nv; base += ngroups) {
+    const int64_t v = base + gidx;
     float w = 0.0f;
     int32_t k0 = 0, k1 = 0;
-    if (lv < nloop) {
-      if (STAGED) {
-        w = o.w[lv];
-        k0 = o.off[lv];
-        k1 = o.off[lv + 1] - 1;
-      } else {
-        w = a.invm[lv];
-        k0 = a.inc_ptr[lv];
-        k1 = a.inc_ptr[lv + 1];
-      }
+    if (v < a.nv) {
+      w = a.invm[v];
+      k0 = a.inc_ptr[v];
+      k1 = a.inc_ptr[v + 1];
     }
     double sx = 0.0, sy = 0.0, sz = 0.0;
     for (int32_t k = k0 + lane; k < k1; k += 4) {
-      const float4 g = STAGED ? o.e[k] : __ldg(a.gV + k);
+      const float4 g = __ldg(a.gV + k);
       const double xt = a.x[__float_as_int(g.w)];
       sx += xt * g.x;
       sy += xt * g.y;
@@ -186,8 +134,7 @@ __device__ __forceinline__ void vphase_warm(const PArgs& a, const Own& o) {
       sy += __shfl_xor_sync(0xffffffffu, sy, sh, 4);
       sz += __shfl_xor_sync(0xffffffffu, sz, sh, 4);
     }
-    if (lane == 0 && lv < nloop) {
-      const int64_t v = STAGED ? o.vb0 + lv : lv;
+    if (lane == 0 && v < a.nv) {
       sx *= w;
       sy *= w;
       sz *= w;
@@ -199,9 +146,8 @@ __device__ __forceinline__ void vphase_warm(const PArgs& a, const Own& o) {
 }
 
 // (A x)_t in float64 from the float pair u + ulo (warm start)
-template <bool STAGED>
-__device__ __forceinline__ double tdot_warm(const PArgs& a, const Own& o, int64_t t) {
-  const int4 q = tet_q<STAGED>(a, o, t);
+__device__ __forceinline__ double tdot_warm(const PArgs& a, int64_t t) {
+  const int4 q = a.ta.t_i[t];
   const int32_t vs[4] = {q.x, q.y, q.z, q.w};
   const float4 g0 = __ldg(a.ta.gradC + t), g1 = __ldg(a.ta.gradC + a.ta.nt + t),
                g2 = __ldg(a.ta.gradC + 2LL * a.ta.nt + t);
@@ -217,97 +163,24 @@ __device__ __forceinline__ double tdot_warm(const PArgs& a, const Own& o, int64_
 }
 
 // Vertex phase: u_v = w_v sum x_t g_{t,l} with x_t = src_t (+ beta p_t).
-template <int SRC, bool STAGED>
-__device__ __forceinline__ void vphase(const PArgs& a, const Own& o, float beta, const float* src) {
-  if (!STAGED) {
-    const int lane = threadIdx.x % kVG;
-    constexpr int kPerWarp = 32 / kVG;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kPerWarp;
-    for (int64_t base = warp * kPerWarp; base < a.nv; base += stride) {
-      const int64_t v = base + (threadIdx.x & 31) / kVG;
-      const bool valid = v < a.nv;
-      float w;
-      const float3 s = jv_group<SRC>(v, valid, lane, a.inc_ptr, a.gV, a.invm, src, a.p, beta, &w);
-      if (valid && lane == 0) a.u[v] = make_float4(w * s.x, w * s.y, w * s.z, 0.0f);
-    }
-    return;
-  }
-  // staged: kVS lanes per vertex, kVB vertices per lane group and round;
-  // the entries (shared memory, one pad slot after each vertex's run so
-  // consecutive vertices start 4 banks apart) give the tet ids, and all
-  // gathers of a round are issued before any is consumed
-  const int lane = threadIdx.x % kVS;
-  const int grp = threadIdx.x / kVS;
-  const int ngrp = blockDim.x / kVS;
-  for (int base = 0; base < o.nvb; base += kVB * ngrp) {
-    int k0[kVB], k1[kVB];
-    float wv[kVB];
-#pragma unroll
-    for (int i = 0; i < kVB; ++i) {
-      const int lv = base + grp + i * ngrp;
-      k0[i] = k1[i] = 0;
-      wv[i] = 0.0f;
-      if (lv < o.nvb) {
-        wv[i] = o.w[lv];
-        if (wv[i] != 0.0f) {
-          k0[i] = o.off[lv];
-          k1[i] = o.off[lv + 1] - 1;
-        }
-      }
-    }
-    float xs[kVB][kVE];
-#pragma unroll
-    for (int i = 0; i < kVB; ++i) {
-#pragma unroll
-      for (int c = 0; c < kVE; ++c) {
-        const int k = k0[i] + lane + kVS * c;
-        float xt = 0.0f;
-        if (k < k1[i]) {
-          const int32_t t = __float_as_int(o.e[k].w);
-          xt = SRC == kSrcZbP ? src[t] + beta * a.p[t] : src[t];
-        }
-        xs[i][c] = xt;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kVB; ++i) {
-      float ax = 0.f, ay = 0.f, az = 0.f;
-#pragma unroll
-      for (int c = 0; c < kVE; ++c) {
-        const int k = k0[i] + lane + kVS * c;
-        if (k < k1[i]) {
-          const float4 g = o.e[k];
-          ax += xs[i][c] * g.x;
-          ay += xs[i][c] * g.y;
-          az += xs[i][c] * g.z;
-        }
-      }
-      // vertices with more than kVS * kVE incident tets
-      for (int k = k0[i] + lane + kVS * kVE; k < k1[i]; k += kVS) {
-        const float4 g = o.e[k];
-        const int32_t t = __float_as_int(g.w);
-        const float xt = SRC == kSrcZbP ? src[t] + beta * a.p[t] : src[t];
-        ax += xt * g.x;
-        ay += xt * g.y;
-        az += xt * g.z;
-      }
-#pragma unroll
-      for (int sh = kVS / 2; sh > 0; sh >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, sh, kVS);
-        ay += __shfl_xor_sync(0xffffffffu, ay, sh, kVS);
-        az += __shfl_xor_sync(0xffffffffu, az, sh, kVS);
-      }
-      const int lv = base + grp + i * ngrp;
-      if (lane == 0 && lv < o.nvb)
-        a.u[o.vb0 + lv] = make_float4(wv[i] * ax, wv[i] * ay, wv[i] * az, 0.0f);
-    }
+template <int SRC>
+__device__ __forceinline__ void vphase(const PArgs& a, float beta, const float* src) {
+  const int lane = threadIdx.x % kVG;
+  constexpr int kPerWarp = 32 / kVG;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kPerWarp;
+  for (int64_t base = warp * kPerWarp; base < a.nv; base += stride) {
+    const int64_t v = base + (threadIdx.x & 31) / kVG;
+    const bool valid = v < a.nv;
+    float w;
+    const float3 s = jv_group<SRC>(v, valid, lane, a.inc_ptr, a.gV, a.invm, src, a.p, beta, &w);
+    if (valid && lane == 0) a.u[v] = make_float4(w * s.x, w * s.y, w * s.z, 0.0f);
   }
 }
 
 // Chebyshev step: rr = D^-1 (r - A z); d = c1 d + c2 rr; z += d.  LAST also
 // writes this block's partial of r.z.
-template <bool LAST, bool STAGED>
+template <bool LAST>
 __device__ __forceinline__ void tphase_cheb(const PArgs& a, const Own& o, float c1, float c2,
                                             double* slot) {
   float acc = 0.0f;
@@ -316,7 +189,7 @@ __device__ __forceinline__ void tphase_cheb(const PArgs& a, const Own& o, float 
 #pragma unroll
     for (int i = 0; i < kTB; ++i) {
       const int64_t t = tb + i * o.tstep;
-      y[i] = t < o.tend ? tdot_any<STAGED>(a, o, t) : 0.0f;
+      y[i] = t < o.tend ? tdot_any(a, t) : 0.0f;
     }
 #pragma unroll
     for (int i = 0; i < kTB; ++i) {
@@ -325,7 +198,7 @@ __device__ __forceinline__ void tphase_cheb(const PArgs& a, const Own& o, float 
         const float zt = a.z[t];
         const float yt = y[i] + __ldg(a.ta.alpha + t) * zt;
         const float rt = a.r[t];
-        const float rrv = dinv_of<STAGED>(a, t) * (rt - yt);
+        const float rrv = dinv_of(a, t) * (rt - yt);
         const float dt = c1 * a.d[t] + c2 * rrv;
         a.d[t] = dt;
         const float zn = zt + dt;
@@ -338,7 +211,6 @@ __device__ __forceinline__ void tphase_cheb(const PArgs& a, const Own& o, float 
 }
 
 // p = z + beta p; ap = A p; this block's partial of p.Ap
-template <bool STAGED>
 __device__ __forceinline__ void tphase_ap(const PArgs& a, const Own& o, float bf, double* slot) {
   float acc = 0.0f;
   for (int64_t tb = o.tbeg; tb < o.tend; tb += kTB * o.tstep) {
@@ -346,7 +218,7 @@ __device__ __forceinline__ void tphase_ap(const PArgs& a, const Own& o, float bf
 #pragma unroll
     for (int i = 0; i < kTB; ++i) {
       const int64_t t = tb + i * o.tstep;
-      y[i] = t < o.tend ? tdot_any<STAGED>(a, o, t) : 0.0f;
+      y[i] = t < o.tend ? tdot_any(a, t) : 0.0f;
     }
 #pragma unroll
     for (int i = 0; i < kTB; ++i) {
@@ -363,12 +235,10 @@ __device__ __forceinline__ void tphase_ap(const PArgs& a, const Own& o, float bf
   put_partial(acc, slot);
 }
 
-template <bool STAGED>
-__global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
+__global__ void __launch_bounds__(kPT, 2) k_jcg(PArgs a) {
   // a skipped launch leaves before its first barrier in every block (every
   // thread reads the same flag)
   if (a.ctl && a.ctl->skip) return;
-  extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ float s_c1[kMaxCheb], s_c2[kMaxCheb];
   __shared__ float s_scal;  // alpha or beta, broadcast from thread 0
   __shared__ int s_stop;
@@ -402,53 +272,15 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
   unsigned long long gen = 0;
 
   Own o;
-  if (STAGED) {
-    const int32_t tb0 = a.part_t[blockIdx.x], tb1 = a.part_t[blockIdx.x + 1];
-    const int32_t vb0 = a.part_v[blockIdx.x], vb1 = a.part_v[blockIdx.x + 1];
-    const int32_t e0 = a.inc_ptr[vb0], ne = a.inc_ptr[vb1] - e0;
-    o.tbeg = tb0 + threadIdx.x;
-    o.tend = tb1;
-    o.tstep = blockDim.x;
-    o.tb0 = tb0;
-    o.vb0 = vb0;
-    o.nvb = vb1 - vb0;
-    float4* se = reinterpret_cast<float4*>(s_dyn);
-    int4* sq = reinterpret_cast<int4*>(se + a.emax + a.vmax);
-    int32_t* soff = reinterpret_cast<int32_t*>(sq + a.tmax);
-    float* sw = reinterpret_cast<float*>(soff + a.vmax + 1);
-    // vertex lv's entries go to [off + lv, off + lv + n): one pad slot per vertex
-    const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5, ln = threadIdx.x & 31;
-    for (int lv = wid; lv < o.nvb; lv += nw) {
-      const int32_t k0 = a.inc_ptr[vb0 + lv], n = a.inc_ptr[vb0 + lv + 1] - k0;
-      const int32_t dst = k0 - e0 + lv;
-      for (int j = ln; j < n; j += 32) se[dst + j] = __ldg(a.gV + k0 + j);
-    }
-    for (int k = threadIdx.x; k < tb1 - tb0; k += blockDim.x) sq[k] = a.ta.t_i[tb0 + k];
-    for (int k = threadIdx.x; k <= o.nvb; k += blockDim.x) soff[k] = a.inc_ptr[vb0 + k] - e0 + k;
-    for (int k = threadIdx.x; k < o.nvb; k += blockDim.x) sw[k] = a.invm[vb0 + k];
-    (void)ne;
-    o.e = se;
-    o.q = sq;
-    o.off = soff;
-    o.w = sw;
-  } else {
-    o.tbeg = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    o.tend = a.ta.nt;
-    o.tstep = (int64_t)G * blockDim.x;
-    o.tb0 = 0;
-    o.vb0 = 0;
-    o.nvb = 0;
-    o.e = nullptr;
-    o.q = nullptr;
-    o.off = nullptr;
-    o.w = nullptr;
-  }
+  o.tbeg = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  o.tend = a.ta.nt;
+  o.tstep = (int64_t)G * blockDim.x;
   __syncthreads();
 
   // x = 0 (or the warm start x0), r = b - A x, p = 0, z = d = D^-1 r / theta;
   // partials of b.b and r.z
   if (warm) {
-    vphase_warm<STAGED>(a, o);
+    vphase_warm(a);
     if (!grid_sync(a, gen)) return;
   }
   {
@@ -457,14 +289,14 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
       const float bt = a.b[t];
       float rt = bt;
       if (warm) {
-        rt = (float)((double)bt - tdot_warm<STAGED>(a, o, t));
+        rt = (float)((double)bt - tdot_warm(a, t));
       } else {
         a.x[t] = 0.0f;
       }
       a.xc[t] = 0.0f;
       a.r[t] = rt;
       a.p[t] = 0.0f;
-      const float zt = dinv_of<STAGED>(a, t) * rt * it;
+      const float zt = dinv_of(a, t) * rt * it;
       a.z[t] = zt;
       a.d[t] = zt;
       bb += bt * bt;
@@ -503,10 +335,10 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
   // remaining Chebyshev steps of z = M^-1 r
   if (!done && m > 1) {
     for (int i = 1; i < m; ++i) {
-      vphase<kSrcX, STAGED>(a, o, 0.0f, a.z);
+      vphase<kSrcX>(a, 0.0f, a.z);
       if (!grid_sync(a, gen)) return;
-      if (i == m - 1) tphase_cheb<true, STAGED>(a, o, s_c1[i], s_c2[i], P2);
-      else tphase_cheb<false, STAGED>(a, o, s_c1[i], s_c2[i], P2);
+      if (i == m - 1) tphase_cheb<true>(a, o, s_c1[i], s_c2[i], P2);
+      else tphase_cheb<false>(a, o, s_c1[i], s_c2[i], P2);
       if (!grid_sync(a, gen)) return;
     }
     if (threadIdx.x < 32) {
@@ -528,10 +360,10 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
   float bf = 0.0f;  // beta
   while (!done) {
     // u = W J^T (z + beta p)
-    vphase<kSrcZbP, STAGED>(a, o, bf, a.z);
+    vphase<kSrcZbP>(a, bf, a.z);
     if (!grid_sync(a, gen)) return;
     // p = z + beta p; ap = A p; partials of p.Ap
-    tphase_ap<STAGED>(a, o, bf, P0);
+    tphase_ap(a, o, bf, P0);
     if (!grid_sync(a, gen)) return;
     if (threadIdx.x < 32) {
       const double sp = warp_sum_partials(P0, G);
@@ -565,7 +397,7 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
         a.x[t] = sn;
         const float rt = a.r[t] - al * apt;
         a.r[t] = rt;
-        const float zt = dinv_of<STAGED>(a, t) * rt * it;
+        const float zt = dinv_of(a, t) * rt * it;
         a.z[t] = zt;
         a.d[t] = zt;
         acc_rr += rt * rt;
@@ -594,10 +426,10 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
     if (s_stop) break;
     if (m > 1) {
       for (int i = 1; i < m; ++i) {
-        vphase<kSrcX, STAGED>(a, o, 0.0f, a.z);
+        vphase<kSrcX>(a, 0.0f, a.z);
         if (!grid_sync(a, gen)) return;
-        if (i == m - 1) tphase_cheb<true, STAGED>(a, o, s_c1[i], s_c2[i], P2);
-        else tphase_cheb<false, STAGED>(a, o, s_c1[i], s_c2[i], P2);
+        if (i == m - 1) tphase_cheb<true>(a, o, s_c1[i], s_c2[i], P2);
+        else tphase_cheb<false>(a, o, s_c1[i], s_c2[i], P2);
         if (!grid_sync(a, gen)) return;
       }
     }
@@ -660,7 +492,7 @@ __global__ void __launch_bounds__(kPT, STAGED ? 1 : 2) k_jcg(PArgs a) {
 // each converges as its own CG would.  A body that meets its bound keeps
 // its x and r (its chunks are skipped); the launch ends when every body has
 // stopped.  The Chebyshev preconditioner (one polynomial) and the vertex
-// and tet phases are those of k_jcg, unstaged.
+// and tet phases are those of k_jcg.
 //
 // Per iteration: vertex phase, A p (chunked), body alphas, update
 // (chunked), body residuals, the Chebyshev steps (the last chunked), body
@@ -739,13 +571,6 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
   o.tbeg = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   o.tend = a.ta.nt;
   o.tstep = (int64_t)gridDim.x * blockDim.x;
-  o.tb0 = 0;
-  o.vb0 = 0;
-  o.nvb = 0;
-  o.e = nullptr;
-  o.q = nullptr;
-  o.off = nullptr;
-  o.w = nullptr;
   __syncthreads();
   // every block reads whether all bodies have stopped after a barrier
   auto all_stopped = [&]() {
@@ -757,7 +582,7 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
   // x = 0 (or the warm start), r = b - A x, p = 0, z = d = D^-1 r / theta;
   // chunk partials of b.b, r.z and r.r
   if (warm) {
-    vphase_warm<false>(a, o);
+    vphase_warm(a);
     if (!grid_sync(a, gen)) return;
   }
   for (int64_t c = gwarp(); c < b.nch; c += nwarps()) {
@@ -767,14 +592,14 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
       const float bt = a.b[t];
       float rt = bt;
       if (warm) {
-        rt = (float)((double)bt - tdot_warm<false>(a, o, t));
+        rt = (float)((double)bt - tdot_warm(a, t));
       } else {
         a.x[t] = 0.0f;
       }
       a.xc[t] = 0.0f;
       a.r[t] = rt;
       a.p[t] = 0.0f;
-      const float zt = dinv_of<false>(a, t) * rt * it;
+      const float zt = dinv_of(a, t) * rt * it;
       a.z[t] = zt;
       a.d[t] = zt;
       bb += bt * bt;
@@ -821,10 +646,10 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
   // of r.z into plane 2
   auto cheb_steps = [&]() -> bool {
     for (int i = 1; i < m; ++i) {
-      vphase<kSrcX, false>(a, o, 0.0f, a.z);
+      vphase<kSrcX>(a, 0.0f, a.z);
       if (!grid_sync(a, gen)) return false;
       if (i < m - 1) {
-        tphase_cheb<false, false>(a, o, s_c1[i], s_c2[i], nullptr);
+        tphase_cheb<false>(a, o, s_c1[i], s_c2[i], nullptr);
       } else {
         const float c1 = s_c1[i], c2 = s_c2[i];
         for (int64_t c = gwarp(); c < b.nch; c += nwarps()) {
@@ -835,7 +660,7 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
 #pragma unroll
             for (int q = 0; q < kTB; ++q) {
               const int64_t t = tb + 32 * q;
-              y[q] = t < r.y ? tdot_any<false>(a, o, t) : 0.0f;
+              y[q] = t < r.y ? tdot_any(a, t) : 0.0f;
             }
 #pragma unroll
             for (int q = 0; q < kTB; ++q) {
@@ -844,7 +669,7 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
                 const float zt = a.z[t];
                 const float yt = y[q] + __ldg(a.ta.alpha + t) * zt;
                 const float rt = a.r[t];
-                const float rrv = dinv_of<false>(a, t) * (rt - yt);
+                const float rrv = dinv_of(a, t) * (rt - yt);
                 const float dt = c1 * a.d[t] + c2 * rrv;
                 a.d[t] = dt;
                 const float zn = zt + dt;
@@ -897,7 +722,7 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
 #pragma unroll
         for (int q = 0; q < kTB; ++q) {
           const int64_t t = tb + 32 * q;
-          y[q] = t < r.y ? tdot_any<false>(a, o, t) : 0.0f;
+          y[q] = t < r.y ? tdot_any(a, t) : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < kTB; ++q) {
@@ -950,7 +775,7 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
         a.x[t] = sn;
         const float rt = a.r[t] - al * apt;
         a.r[t] = rt;
-        const float zt = dinv_of<false>(a, t) * rt * it;
+        const float zt = dinv_of(a, t) * rt * it;
         a.z[t] = zt;
         a.d[t] = zt;
         acc_rr += rt * rt;
@@ -1041,11 +866,6 @@ __global__ void __launch_bounds__(kPT, 2) k_jcg_bodies(PArgs a, BodyCg b) {
   }
 }
 
-int64_t staged_smem_bytes(int32_t emax, int32_t tmax, int32_t vmax) {
-  const int64_t b = 16LL * (emax + vmax) + 16LL * tmax + 4LL * (vmax + 1) + 4LL * vmax;
-  return (b + 15) / 16 * 16;
-}
-
 }  // namespace
 
 JcgPlan jcg_plan(const std::vector<int32_t>& inc_ptr, int32_t nv, int32_t nt, bool allow_staged) {
@@ -1057,6 +877,9 @@ JcgPlan jcg_plan(const std::vector<int32_t>& inc_ptr, int32_t nv, int32_t nt, bo
   require(coop != 0, MGPBD_ENOTSUP, "device does not support cooperative launch");
   MGPBD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   MGPBD_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  int occ = 0;
+  MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jcg, kPT, 0));
+  require(occ >= 1, MGPBD_ENOTSUP, "persistent CG kernel does not fit on an SM");
   const int64_t ne = inc_ptr[nv];
   if (allow_staged) {
     JcgPlan p;
@@ -1084,29 +907,17 @@ JcgPlan jcg_plan(const std::vector<int32_t>& inc_ptr, int32_t nv, int32_t nt, bo
       p.tmax = std::max(p.tmax, p.tb[b + 1] - p.tb[b]);
       p.emax = std::max(p.emax, inc_ptr[p.vb[b + 1]] - inc_ptr[p.vb[b]]);
     }
-    const int64_t smem = staged_smem_bytes(p.emax, p.tmax, p.vmax);
+    const int64_t smem = jcg_staged_bytes(p.emax, p.tmax, p.vmax);
     if (smem <= optin) {
-      MGPBD_CUDA(cudaFuncSetAttribute(k_jcg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
-      int occ = 0;
-      MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jcg<true>, kPT,
-                                                               static_cast<size_t>(smem)));
-      if (occ >= 1) {
-        p.staged = true;
-        p.grid = G;
-        p.smem = static_cast<int>(smem);
-        return p;
-      }
+      p.staged = true;
+      p.grid = G;
+      p.dual_grid = sms * occ;
+      return p;
     }
   }
   // too large to stage: every phase reads from L2, work strided over the grid
   JcgPlan p;
-  int occ = 0;
-  MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jcg<false>, kPT, 0));
-  require(occ >= 1, MGPBD_ENOTSUP, "persistent CG kernel does not fit on an SM");
-  p.staged = false;
-  p.grid = sms * occ;
-  p.smem = 0;
+  p.grid = p.dual_grid = sms * occ;
   return p;
 }
 
@@ -1144,9 +955,6 @@ static PArgs pargs_of(const JView& j, const JcgVecs& v, const JState* js, CgStat
   a.gs = v.gs;
   a.st = st;
   a.js = js;
-  a.part_v = nullptr;
-  a.part_t = nullptr;
-  a.emax = a.tmax = a.vmax = 0;
   a.tol_abs = tol_abs;
   a.tol_rel = tol_rel;
   a.maxiter = maxiter;
@@ -1160,31 +968,18 @@ static PArgs pargs_of(const JView& j, const JcgVecs& v, const JState* js, CgStat
 }
 
 void launch_jcg_persistent(const JView& j, const JcgVecs& v, const JcgPlan& plan,
-                           const int32_t* part_dev, const JState* js, CgState* st, double tol_abs,
-                           double tol_rel, int maxiter, int degree, bool warm, double spin_limit_s,
-                           cudaStream_t s, const JcgCtl* ctl) {
+                           const JState* js, CgState* st, double tol_abs, double tol_rel,
+                           int maxiter, int degree, bool warm, double spin_limit_s, cudaStream_t s,
+                           const JcgCtl* ctl) {
   require(degree >= 1 && degree <= kMaxCheb, MGPBD_EINVAL, "Chebyshev degree out of range");
-  require(plan.grid > 0, MGPBD_ESTATE, "persistent CG plan not built");
-  require(3LL * plan.grid <= v.partials_capacity, MGPBD_ERANGE, "partials buffer too small");
-  require(!plan.staged || part_dev != nullptr, MGPBD_ESTATE, "staged plan without partition");
+  require(plan.dual_grid > 0, MGPBD_ESTATE, "persistent CG plan not built");
+  require(3LL * plan.dual_grid <= v.partials_capacity, MGPBD_ERANGE, "partials buffer too small");
   PArgs a = pargs_of(j, v, js, st, tol_abs, tol_rel, maxiter, degree, warm, spin_limit_s, ctl);
-  a.part_v = plan.staged ? part_dev : nullptr;
-  a.part_t = plan.staged ? part_dev + plan.grid + 1 : nullptr;
-  a.emax = plan.emax;
-  a.tmax = plan.tmax;
-  a.vmax = plan.vmax;
   MGPBD_CUDA(cudaMemsetAsync(v.gs, 0, sizeof(GridSync), s));
   MGPBD_CUDA(cudaMemsetAsync(st, 0, sizeof(CgState), s));
   void* args[] = {&a};
-  const void* fn = plan.staged ? reinterpret_cast<const void*>(k_jcg<true>)
-                               : reinterpret_cast<const void*>(k_jcg<false>);
-  // the dynamic shared-memory limit is a per-function attribute shared by
-  // every handle in the process: set this plan's before each staged launch
-  if (plan.staged)
-    MGPBD_CUDA(cudaFuncSetAttribute(k_jcg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    plan.smem));
-  MGPBD_CUDA(cudaLaunchCooperativeKernel(fn, dim3(plan.grid), dim3(kPT), args,
-                                         static_cast<size_t>(plan.smem), s));
+  MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_jcg), dim3(plan.dual_grid),
+                                         dim3(kPT), args, 0, s));
   MGPBD_CHECK_LAUNCH();
 }
 

@@ -132,14 +132,15 @@ struct JcgVecs {
   GridSync* gs = nullptr;
   float4* ulo = nullptr;  // warm start: nv float4 scratch
 };
-// Work split of the persistent kernel for one mesh on the current device:
-// the cooperative grid, and, when the block data fits in shared memory
-// (staged), each block's vertex range (balanced by incident entries) and
-// 32-aligned tet range with the largest per-block counts.
+// Work split of the persistent kernels for one mesh on the current device:
+// the cooperative grids, and, when a block's share of the operator fits in
+// shared memory (staged: what the primal kernel holds there), each block's
+// vertex range (balanced by incident entries) and 32-aligned tet range with
+// the largest per-block counts.
 struct JcgPlan {
   bool staged = false;
-  int grid = 0;   // resident blocks of the cooperative launch
-  int smem = 0;   // dynamic shared memory per block (staged)
+  int grid = 0;       // resident blocks of the primal kernel's launch
+  int dual_grid = 0;  // ... and of the dual kernel's
   int32_t vmax = 0, tmax = 0, emax = 0;
   std::vector<int32_t> vb, tb;  // grid + 1 boundaries each (staged)
 };
@@ -147,10 +148,13 @@ struct JcgPlan {
 // the staged one would fit
 JcgPlan jcg_plan(const std::vector<int32_t>& inc_ptr, int32_t nv, int32_t nt,
                  bool allow_staged = true);
+inline int64_t jcg_staged_bytes(int32_t emax, int32_t tmax, int32_t vmax) {
+  const int64_t b = 16LL * (emax + vmax) + 16LL * tmax + 4LL * (vmax + 1) + 4LL * vmax;
+  return (b + 15) / 16 * 16;
+}
 // The whole CG solve (init, iterations to the tolerance or maxiter, the
 // Chebyshev preconditioner of `degree`) as one cooperative kernel; st is
-// zeroed and then filled like the per-phase path fills it.  part_dev holds
-// plan.vb then plan.tb on the device (staged plans).  warm: start from the
+// zeroed and then filled like the per-phase path fills it.  warm: start from the
 // x on entry (r = b - A x) instead of 0; the tolerance stays relative to
 // |b|.  A barrier wait longer than spin_limit_s sets
 // MGPBD_STATUS_SYNC_TIMEOUT in st->status.
@@ -166,9 +170,9 @@ struct JcgCtl {
   int32_t pad;
 };
 void launch_jcg_persistent(const JView& j, const JcgVecs& v, const JcgPlan& plan,
-                           const int32_t* part_dev, const JState* js, CgState* st, double tol_abs,
-                           double tol_rel, int maxiter, int degree, bool warm, double spin_limit_s,
-                           cudaStream_t s, const JcgCtl* ctl = nullptr);
+                           const JState* js, CgState* st, double tol_abs, double tol_rel,
+                           int maxiter, int degree, bool warm, double spin_limit_s, cudaStream_t s,
+                           const JcgCtl* ctl = nullptr);
 
 // Packed bodies: the per-body CG of launch_jcg_bodies (A block diagonal
 // over the bodies).  Device arrays; the chunks and body lists are constant

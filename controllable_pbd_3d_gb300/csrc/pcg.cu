@@ -778,16 +778,11 @@ __global__ void __launch_bounds__(kPT, 1) k_pcg(QArgs a) {
   }
 }
 
-int64_t staged_smem_bytes(int32_t emax, int32_t tmax, int32_t vmax) {
-  const int64_t b = 16LL * (emax + vmax) + 16LL * tmax + 4LL * (vmax + 1) + 4LL * vmax;
-  return (b + 15) / 16 * 16;
-}
-
 }  // namespace
 
 bool pcg_plan_fits(JcgPlan& plan) {
   if (!plan.staged) return true;
-  const int64_t smem = staged_smem_bytes(plan.emax, plan.tmax, plan.vmax);
+  const int64_t smem = jcg_staged_bytes(plan.emax, plan.tmax, plan.vmax);
   int dev = 0, optin = 0;
   MGPBD_CUDA(cudaGetDevice(&dev));
   MGPBD_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -865,7 +860,7 @@ void launch_pcg_primal(const JView& j, const PcgVecs& v, const JcgPlan& plan,
   void* args[] = {&a};
   const void* fn = plan.staged ? reinterpret_cast<const void*>(k_pcg<true>)
                                : reinterpret_cast<const void*>(k_pcg<false>);
-  const size_t smem = plan.staged ? static_cast<size_t>(staged_smem_bytes(plan.emax, plan.tmax,
+  const size_t smem = plan.staged ? static_cast<size_t>(jcg_staged_bytes(plan.emax, plan.tmax,
                                                                            plan.vmax))
                                   : 0;
   // per-function attribute shared by every handle: set this plan's limit

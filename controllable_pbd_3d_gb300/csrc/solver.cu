@@ -440,7 +440,7 @@ void Solver::init() {
         pplan_.grid = pcg_unstaged_grid();
       }
     }
-    if (jplan_.staged) {
+    if (jplan_.staged && primal()) {
       std::vector<int32_t> part(jplan_.vb);
       part.insert(part.end(), jplan_.tb.begin(), jplan_.tb.end());
       upload(jpart_, part, s);
@@ -461,7 +461,7 @@ void Solver::init() {
     stats_.cg_path = jplan_.staged ? MGPBD_CGPATH_STAGED : MGPBD_CGPATH_PERSISTENT;
     if (primal())
       stats_.cg_path = pplan_.staged ? MGPBD_CGPATH_PRIMAL_STAGED : MGPBD_CGPATH_PRIMAL;
-    stats_.cg_grid = jplan_.grid;
+    stats_.cg_grid = jplan_.dual_grid;
   }
   for (int32_t l = 0; l < n_levels() && l < 8; ++l) {
     stats_.rows[l] = levels_[l].n;
@@ -472,6 +472,126 @@ void Solver::init() {
     init_bodies(t_host);
     inited_ = true;
   }
+  dcg_ready_ = false;
+  if (cheb() && p_.persistent == 1) build_dcg(t_host);
+  if (dcg_ready_) {
+    stats_.cg_grid = dplan_.nprob * dplan_.nblk;
+  }
+}
+
+// The partition of the dual CG and its device arrays.
+void Solver::build_dcg(const std::vector<int32_t>& t_host) {
+  cudaStream_t s = stream_;
+  int dev = 0, sms = 0;
+  MGPBD_CUDA(cudaGetDevice(&dev));
+  MGPBD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int limit = dcg_smem_limit();
+  std::vector<float> xr(3LL * nv_);
+  MGPBD_CUDA(cudaMemcpyAsync(xr.data(), x_ref_, sizeof(float) * xr.size(), cudaMemcpyDeviceToHost, s));
+  MGPBD_CUDA(cudaStreamSynchronize(s));
+  const int32_t* prob = nullptr;
+  std::vector<int32_t> body;
+  const bool per_body = nb_ > 0 && p_.body_cg;
+  const double entries = 4.0 * n4_ + 2.0 * (nt_ - n4_);
+  // candidates in order of preference: blocks per problem, cluster or grid
+  std::vector<std::pair<int32_t, bool>> shapes;
+  if (per_body) {
+    body.resize(nt_);
+    std::vector<double> size(nb_, 0.0);
+    for (size_t k = 0; k < body_segs_.size(); k += 3)
+      for (int32_t t = body_segs_[k]; t < body_segs_[k + 1]; ++t) {
+        body[t] = body_segs_[k + 2];
+        size[body[t]] += t < n4_ ? 4.0 : 2.0;
+      }
+    prob = body.data();
+    shapes = dcg_body_shapes(size);
+  } else {
+    if (entries <= kDClusterEntries) shapes.push_back({kDMaxCluster, true});
+    shapes.push_back({std::min(sms, 255), false});
+  }
+  bool built = false;
+  for (const auto& sh : shapes) {
+    const double per_block = static_cast<double>(nt_) / ((per_body ? nb_ : 1) * sh.first);
+    const int threads = per_body || per_block >= kDWideConstraints ? kDMaxThreads : 512;
+    if (build_dcg_plan(t_host.data(), nt_, n4_, nv_, xr.data(), prob, per_body ? nb_ : 1, sh.first,
+                       sh.second, threads, limit, dplan_) &&
+        (!sh.second || dcg_max_clusters(sh.first, threads, dplan_.smem) >= 1)) {
+      built = true;
+      break;
+    }
+  }
+  if (!built) return;
+  const int32_t nblk = dplan_.nblk;
+  upload(d_blocks_, dplan_.blocks, s);
+  upload(d_perm_, dplan_.perm, s);
+  upload(d_ti_, dplan_.ti, s);
+  upload(d_pos_v_, dplan_.pos_v, s);
+  upload(d_pos_info_, dplan_.pos_info, s);
+  upload(d_tgt_, dplan_.tgt, s);
+  upload(d_slice_, dplan_.slice, s);
+  upload(d_row_ent_, dplan_.row_ent, s);
+  upload(d_row_idx_, dplan_.row_idx, s);
+  upload(d_warps_, dplan_.warps, s);
+  d_rows_.alloc(kDRow * dplan_.n_rows);
+  MGPBD_CUDA(cudaStreamSynchronize(s));
+  d_tg_.alloc(3LL * nt_);
+  d_exch_.alloc(2 * dplan_.n_slots + 6LL * nblk);
+  d_vecs_.alloc(7LL * nt_);
+  d_gflag_.alloc(1);
+  DcgDev& d = ddev_;
+  d.blocks = d_blocks_.p;
+  d.perm = d_perm_.p;
+  d.ti = reinterpret_cast<const uint2*>(d_ti_.p);
+  d.pos_v = d_pos_v_.p;
+  d.pos_info = reinterpret_cast<const uint2*>(d_pos_info_.p);
+  d.tgt = d_tgt_.p;
+  d.slice = reinterpret_cast<const uint2*>(d_slice_.p);
+  d.row_ent = d_row_ent_.p;
+  d.row_idx = d_row_idx_.p;
+  d.warps = d_warps_.p;
+  d.rows = d_rows_.p;
+  d.tg = d_tg_.p;
+  float* v = d_vecs_.p;
+  d.ad = reinterpret_cast<float2*>(v);
+  v += 2LL * nt_;
+  for (float** f : {&d.x, &d.xc, &d.r, &d.d, &d.p}) {
+    *f = v;
+    v += nt_;
+  }
+  d.exch = d_exch_.p;
+  d.n_slots = dplan_.n_slots;
+  d.partials = reinterpret_cast<uint4*>(d_exch_.p + 2 * dplan_.n_slots);
+  d.gflag = d_gflag_.p;
+  d.nc = nt_;
+  d.n4 = n4_;
+  // the host arrays are not needed any more
+  for (auto* h : {&dplan_.perm, &dplan_.pos_v, &dplan_.row_ent})
+    std::vector<int32_t>().swap(*h);
+  for (auto* h : {&dplan_.pos_info, &dplan_.tgt, &dplan_.slice}) std::vector<uint32_t>().swap(*h);
+  for (auto* h : {&dplan_.ti, &dplan_.row_idx}) std::vector<uint16_t>().swap(*h);
+  dcg_ready_ = true;
+}
+
+// One dual CG solve over the whole mesh on stream s.
+void Solver::launch_dual(const JcgVecs& v, double tol_abs, double tol_rel, int32_t maxit,
+                         bool warm, cudaStream_t s, const JcgCtl* ctl) {
+  if (dcg_ready_ && dplan_.nprob == 1)
+    launch_dcg(jview(), v, dplan_, ddev_, jst_.p, cg_state_.p, tol_abs, tol_rel, maxit,
+               p_.cheb_degree, warm, false, nullptr, barrier_limit_s_, s, ctl);
+  else
+    launch_jcg_persistent(jview(), v, jplan_, jst_.p, cg_state_.p, tol_abs, tol_rel, maxit,
+                          p_.cheb_degree, warm, barrier_limit_s_, s, ctl);
+}
+
+// One CG per packed body on stream s.
+void Solver::launch_dual_bodies(const JcgVecs& v, int32_t maxit, bool warm, cudaStream_t s,
+                                const JcgCtl* ctl) {
+  if (dcg_ready_)
+    launch_dcg(jview(), v, dplan_, ddev_, jst_.p, cg_state_.p, p_.tol_cg, p_.rel_tol_cg, maxit,
+               p_.cheb_degree, warm, true, bcg_iters_.p, barrier_limit_s_, s, ctl);
+  else
+    launch_jcg_bodies(jview(), v, body_cg(), jst_.p, cg_state_.p, p_.tol_cg, p_.rel_tol_cg, maxit,
+                      p_.cheb_degree, warm, barrier_limit_s_, s, ctl);
 }
 
 // Transfer maps of level l (aggregate id per row, the members of each
@@ -736,6 +856,7 @@ void Solver::jform_setup(uint32_t* dev_status) {
   JView j = jview();
   launch_jform_prepare(j, inc_ent_.p, gV_.p, jdinv_.p, gT_.p,
                        p_.cheb_scale == MGPBD_CHEB_UNSCALED, stream_);
+  if (dcg_ready_) launch_dcg_pack(j, ddev_, dplan_.n_rows, stream_);
   launch_jform_lanczos(j, pw_v_.p, jd_.p, pw_w_.p, partials_.p, jst_.p, kSteps, stream_);
   launch_cheb_coefficients(jst_.p, kSteps, p_.cheb_degree, p_.cheb_lo, dev_status, stream_);
   if (dev_status) return;  // captured: the status word is read after the graph
@@ -1503,8 +1624,7 @@ int32_t Solver::run_dual(const float* b, float* x, double tol_abs, double tol_re
   v.ulo = ulo;
   MGPBD_CUDA(cudaEventRecord(ev_[0], outer));
   dual_x_ = nullptr;
-  launch_jcg_persistent(jview(), v, jplan_, jpart_.p, jst_.p, cg_state_.p, tol_abs, tol_rel, maxit,
-                        p_.cheb_degree, warm, barrier_limit_s_, outer);
+  launch_dual(v, tol_abs, tol_rel, maxit, warm, outer, nullptr);
   dual_x_ = x;
   MGPBD_CUDA(cudaEventRecord(ev_[1], outer));
   sync_read(h_state_, cg_state_.p, sizeof(CgState));
@@ -1732,8 +1852,7 @@ int32_t Solver::run_dual_bodies(const float* b, float* x, int32_t maxit, bool wa
   const JcgVecs v = dual_vecs(b, x);
   MGPBD_CUDA(cudaEventRecord(ev_[0], outer));
   dual_x_ = nullptr;
-  launch_jcg_bodies(jview(), v, body_cg(), jst_.p, cg_state_.p, p_.tol_cg, p_.rel_tol_cg, maxit,
-                    p_.cheb_degree, warm, barrier_limit_s_, outer);
+  launch_dual_bodies(v, maxit, warm, outer, nullptr);
   dual_x_ = x;
   MGPBD_CUDA(cudaEventRecord(ev_[1], outer));
   sync_read(h_state_, cg_state_.p, sizeof(CgState));
@@ -1983,15 +2102,13 @@ void Solver::capture_body_graph() {
     if (p_.body_cg) {
       if (p_.warm_substep)
         launch_bodies_warm_in(L, body_have_prev_.p, dlam_.p, dlam_prev_.p, nt_, bs);
-      launch_jcg_bodies(jview(), v, body_cg(), jst_.p, cg_state_.p, p_.tol_cg, p_.rel_tol_cg,
-                        p_.maxiter_cg, p_.cheb_degree, false, barrier_limit_s_, bs, &L->jc);
+      launch_dual_bodies(v, p_.maxiter_cg, false, bs, &L->jc);
       launch_bodies_verify(ba, L, cg_state_.p, lim, bs);
       if (p_.warm_substep)
         launch_bodies_warm_out(L, body_have_prev_.p, dlam_.p, dlam_prev_.p, nt_, bs);
     } else {
       for (int pass = 0; pass < 6; ++pass) {
-        launch_jcg_persistent(jview(), v, jplan_, jpart_.p, jst_.p, cg_state_.p, p_.tol_cg, 0.0,
-                              p_.maxiter_cg, p_.cheb_degree, false, barrier_limit_s_, bs, &L->jc);
+        launch_dual(v, p_.tol_cg, 0.0, p_.maxiter_cg, false, bs, &L->jc);
         launch_chunk_dual_sq(jrf_.p, nullptr, nullptr, chunks_.p, n_ch, chunk_partials_.p, bs);
         launch_bodies_verify(ba, L, cg_state_.p, lim, bs);
       }

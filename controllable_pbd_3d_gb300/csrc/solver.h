@@ -10,6 +10,7 @@
 
 #include "bodies.cuh"
 #include "common.h"
+#include "dcg.cuh"
 #include "jform.cuh"
 #include "kernels.cuh"
 #include "mpnn.cuh"
@@ -279,6 +280,24 @@ class Solver {
   DevBuf<float> ps_;       // primal CG tet scratch
   bool primal() const { return cheb() && p_.persistent && p_.primal; }
   DevBuf<int32_t> jpart_;  // jplan_.vb then jplan_.tb
+  // the partitioned dual CG (dcg.cuh): of the whole mesh, or of each body
+  bool dcg_ready_ = false;
+  DcgPlan dplan_;
+  DcgDev ddev_;
+  DevBuf<DBlock> d_blocks_;
+  DevBuf<int32_t> d_perm_, d_pos_v_, d_row_ent_;
+  DevBuf<uint32_t> d_pos_info_, d_tgt_, d_slice_;
+  DevBuf<uint16_t> d_ti_, d_row_idx_;
+  DevBuf<DWarp> d_warps_;
+  DevBuf<unsigned char> d_rows_;
+  DevBuf<float4> d_tg_, d_exch_;
+  DevBuf<float> d_vecs_;
+  DevBuf<uint32_t> d_gflag_;
+  void build_dcg(const std::vector<int32_t>& t_host);
+  void launch_dual(const JcgVecs& v, double tol_abs, double tol_rel, int32_t maxit, bool warm,
+                   cudaStream_t s, const JcgCtl* ctl);
+  void launch_dual_bodies(const JcgVecs& v, int32_t maxit, bool warm, cudaStream_t s,
+                          const JcgCtl* ctl);
   cudaGraphExec_t jcg_exec_ = nullptr;
   const float* jcg_b_ = nullptr;
   float* jcg_x_ = nullptr;

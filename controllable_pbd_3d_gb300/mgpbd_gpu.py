@@ -106,10 +106,10 @@ class MGPBDSolverGPU:
                    and one volume constraint det F - 1 per tet, alpha~ =
                    compliance / dt^2; n_tets then counts constraints, the
                    mesh's tets are in mesh_t_i / n_mesh_tets);
-    persistent     FAST + 'cheb': each CG solve is one cooperative persistent
-                   kernel (False: one kernel per phase, per use_graph; 2: the
-                   persistent kernel reading the operator from L2 instead of
-                   staging it in shared memory);
+    persistent     FAST + 'cheb': each CG solve is one persistent kernel that
+                   keeps the operator on the chip as far as it fits (False:
+                   one kernel per phase, per use_graph; 2: one cooperative
+                   kernel reading the operator from L2);
     primal         FAST + 'cheb' + persistent: warm-start each solve through
                    the vertex-space system K y = J^T alpha~^-1 b (Woodbury)
                    to a dual residual of primal_tol |b|, then CG on A;

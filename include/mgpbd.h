@@ -119,11 +119,12 @@ typedef struct mgpbd_params {
    * kernels from the host loop; both give the same results bit for bit. */
   int32_t use_graph;
   /* FAST mode with MGPBD_PRECOND_CHEB: 1 (default) runs each CG solve as ONE
-   * cooperative persistent kernel (grid barriers between its phases, float32
-   * vectors, compensated solution sum); 2 the same without staging the
-   * operator in shared memory (read from L2, as for meshes too large to
-   * stage); 0 runs the per-phase kernels (use_graph selects graph or host
-   * loop for those). */
+   * persistent kernel (float32 vectors, compensated solution sum) whose
+   * blocks own compact parts of the mesh and keep them on the chip as far as
+   * they fit; 2 as one cooperative kernel that reads the operator from L2,
+   * with grid barriers between its phases (also taken for meshes whose parts
+   * are too large: above 2.4 M constraints on 152 SMs); 0 runs the per-phase
+   * kernels (use_graph selects graph or host loop for those). */
   int32_t persistent;
   /* FAST mode, MGPBD_PRECOND_CHEB, persistent: 1 warm-starts each solve
    * through the primal system K y = J^T alpha~^-1 b with K = W^-1 +
@@ -230,10 +231,11 @@ typedef struct mgpbd_stats {
 } mgpbd_stats;
 
 #define MGPBD_CGPATH_KERNELS 0      /* one kernel (or graph node) per operation */
-#define MGPBD_CGPATH_PERSISTENT 1   /* one cooperative kernel per solve, the
-                                       operator read from L2                   */
-#define MGPBD_CGPATH_STAGED 2       /* the same with each block's operator data
-                                       staged in shared memory                 */
+#define MGPBD_CGPATH_PERSISTENT 1   /* one persistent kernel per solve, the
+                                       operator (persistent 1: what does not
+                                       fit on the chip) read from L2           */
+#define MGPBD_CGPATH_STAGED 2       /* the same, an SM's share of the operator
+                                       fits in its shared memory               */
 #define MGPBD_CGPATH_PRIMAL 3       /* primal system, one cooperative kernel    */
 #define MGPBD_CGPATH_PRIMAL_STAGED 4 /* the same, operator data staged         */
 
@@ -630,6 +632,23 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
                         int64_t* c_nnz, int64_t* n_contrib, int32_t* c_indptr,
                         int32_t* c_indices, int32_t* contrib_idx,
                         int32_t* contrib_off);
+
+/* y = (J W J^T + alpha~) x in float64 by way of the spatial partition that
+ * the persistent dual CG runs on: nt constraints t_i (nt,4), the length
+ * constraints from n4 on, rest positions x_ref (nv,3), prob (nt, or NULL) the
+ * body of each of n_prob bodies, n_blocks blocks each (cluster: exchanging
+ * within a cluster), `threads` a block, smem_limit bytes of shared memory.
+ * info (6): whether every block's operator stays on the chip, shared memory a
+ * block, rows in it, rounds of 4-slot constraints in tensor memory, fewest
+ * and most vertex entries of a block.  Host arrays; MGPBD_ERANGE when a
+ * block's vectors do not fit. */
+int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4,
+                               int32_t nv, const float* x_ref, const int32_t* prob,
+                               int32_t n_prob, int32_t n_blocks, int32_t cluster,
+                               int32_t threads, int32_t smem_limit,
+                               const float* gradC, const float* invm,
+                               const float* alpha, const float* x, double* y,
+                               int32_t* info);
 
 /* The same Galerkin build on the GPU (one warp per coarse row, a float64
  * hash accumulation in the host build's summation order): bit-identical
