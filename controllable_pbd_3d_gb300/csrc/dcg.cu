@@ -50,6 +50,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "cheb_dev.cuh"
 #include "common.h"
 #include "dcg.cuh"
 #include "jform_dev.cuh"
@@ -69,12 +70,13 @@ struct DArgs {
   float* xc;
   float* r;
   const float* invm;
-  const JState* js;
+  JState* js;
   CgState* st;
   GridSync* gs;
   const JcgCtl* ctl;
   int32_t* iters;
-  double tol_abs, tol_rel;
+  double tol_abs, tol_rel, lo_ratio;
+  int32_t estimate;  // 1: the Chebyshev interval is estimated first, 0: from js
   int32_t maxiter, degree, warm, per_problem, unit_dinv;
   int32_t nblk, nprob, rmax, kT, kE;
   DcgSmem o;  // byte offsets of the shared-memory parts (u is at 0)
@@ -320,6 +322,7 @@ __device__ __forceinline__ float edge_dot(float x, float y, float z, uint32_t e)
 // The loops are rolled and the code of an application of A appears once: the
 // body of an iteration then stays in the instruction cache, which a version
 // with the gradients in registers (unrolled, 3 times the code) did not.
+constexpr int kLanczosSteps = 24;
 constexpr int kColR = 12, kColP = 9, kColX = 14;  // 4-slot: g 0-8, p, q 10-11, r, d, x, xc
 constexpr int kEdgeR = 4, kEdgeP = 6;             // length: n 0-2, e 3, r, d, p
 
@@ -329,9 +332,10 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   // cluster: exchange barriers, sum barriers (two of each alternate)
   __shared__ __align__(8) unsigned long long s_bar[4];
   __shared__ double s_sum[CLUSTER ? 2 : 1][3][kDMaxCluster];  // cluster: the blocks' partials
-  __shared__ float s_c1[kMaxCheb], s_c2[kMaxCheb];
+  __shared__ float s_c1[kMaxCheb], s_c2[kMaxCheb], s_it;
+  __shared__ double s_la[kLanczosSteps], s_lb[kLanczosSteps];
   __shared__ double s_red[3][kDMaxWarps];
-  __shared__ float s_scal;
+  __shared__ float s_scal, s_inv, s_bprev;
   __shared__ int s_ok, s_stop;  // s_ok: 0 once a wait of this block has given up
   __shared__ uint32_t s_tmem;
   __shared__ DBlock s_B;  // (read where needed: registers are short)
@@ -359,10 +363,11 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid < kMaxCheb) {
+  if (tid < kMaxCheb && !a.estimate) {
     s_c1[tid] = a.js->cf.c1[tid];
     s_c2[tid] = a.js->cf.c2[tid];
   }
+  if (tid == 0 && !a.estimate) s_it = a.js->cf.inv_theta;
   if (tid == nthr - 32) {
     bbs = tol2 = rz = rr = pap = alpha = beta = 0.0;
     iters = 0;
@@ -376,7 +381,6 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
     }
   }
   const int warm = a.ctl ? a.ctl->warm : a.warm;
-  const float it = a.js->cf.inv_theta;
   const int deg = a.degree;
 
   // stage the tables and rows (u.w of a position holds its vertex weight)
@@ -699,7 +703,225 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
     return stop;
   };
 
+  // epi(c, r, d, (J u)_c) -> d: the rounds on private vertices (half 0), the
+  // others (half 1), and what is not held
+  auto held = [&](int half, auto epi) {
+#pragma unroll 1
+    for (int k = half ? kTi : 0; k < (half ? kT : kTi); ++k) {
+      const int c = k * nthr + tid;
+      const uint32_t t = tm0 + 16 * k;
+      uint32_t v[16];
+      tm_ld16(t, v);
+      float g[9];
+#pragma unroll
+      for (int m = 0; m < 9; ++m) g[m] = __uint_as_float(v[m]);
+      float d = __uint_as_float(v[kColR + 1]);
+      if (c < nTr) d = epi(c, __uint_as_float(v[kColR]), d, tet_dot(g, make_uint2(v[10], v[11])));
+      tm_st1(t + kColR + 1, d);
+    }
+#pragma unroll 1
+    for (int k = half ? kEi : 0; k < (half ? kE : kEi); ++k) {
+      const int e = k * nthr + tid;
+      const uint32_t t = tme + 8 * k;
+      uint32_t v[8];
+      tm_ld8(t, v);
+      float d = __uint_as_float(v[kEdgeR + 1]);
+      if (e < nEr)
+        d = epi(nT + e, __uint_as_float(v[kEdgeR]), d,
+                edge_dot(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), v[3]));
+      tm_st1(t + kEdgeR + 1, d);
+    }
+    tm_wait_st();
+  };
+  auto rest_ju = [&](auto epi) {
+#pragma unroll 2
+    for (int c = nTr + tid; c < nT; c += nthr)
+      gd(c) = epi(c, gr(c), gd(c), tet_dot12(tg(0, c), tg(1, c), tg(2, c), ti(c)));
+#pragma unroll 2
+    for (int c = nT + nEr + tid; c < nC; c += nthr) {
+      const float4 g = tg(0, c);
+      gd(c) = epi(c, gr(c), gd(c), edge_dot(g.x, g.y, g.z, __float_as_uint(g.w)));
+    }
+  };
+  // A x of the x in shared memory: the vertex sums, the other blocks' and the
+  // constraints; between() runs while the partials travel, arrived() in the
+  // last warp once they are there (before the others go on).  False when a
+  // wait gave up or `stop` and s_stop is set.
+  auto apply = [&](bool stop, auto epi, auto between, auto arrived) {
+    if (CLUSTER && tid == nthr - 32) expect_bytes(smem_u32(&s_bar[(gen + 1) & 1]), 16 * B.nrecv);
+    sums(++gen);
+    between();
+    __syncthreads();
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      if (half) {
+        if (CLUSTER) {
+          if (tid == nthr - 32) {
+            const uint32_t bar = smem_u32(&s_bar[gen & 1]), parity = (gen - 1) >> 1 & 1;
+            if (!bounded_wait(a, [&]() { return test_phase(bar, parity); })) s_ok = 0;
+          }
+          __syncthreads();
+        }
+        collect(gen);
+        if (syncw) arrived();
+        __syncthreads();
+        if (!s_ok || (stop && s_stop)) return false;
+      }
+      held(half, epi);
+    }
+    rest_ju(epi);
+    return true;
+  };
+
+  // The Chebyshev interval of this problem: lambda_max of S = D^-1/2 A D^-1/2
+  // by Lanczos steps from a fixed start vector (Golub & Van Loan, sec. 10.1).
+  // One application and one sum a step: with q.w, w.w and q.q of
+  // w = S q - b q_prev, a = q.w / q.q and b = |w - a q| follow together.  As
+  // kernels of their own the 24 steps and the interval took 730 us a Newton
+  // iteration, here 245 us (72,000 ARAP constraints on the grid): a step costs
+  // two meetings, not four launches.
+  auto estimate = [&]() {
+    auto sqd = [&](int c) { return a.unit_dinv ? 1.0f : sqrtf(ad(c).y); };
+    {
+      float qq = 0.0f;
+      auto seed = [&](int c) {
+        uint32_t h = static_cast<uint32_t>(perm(c)) * 2654435761u;
+        h ^= h >> 15;
+        const float v = 0.5f + (h & 0xffff) * (1.0f / 65536.0f);
+        qq += v * v;
+        return v;
+      };
+      rounds([&](int c, bool ok, uint32_t t, uint32_t) { tm_st2(t, 0.0f, ok ? seed(c) : 0.0f); });
+      rest([&](int c) {
+        gr(c) = 0.0f;
+        gd(c) = seed(c);
+      });
+      tm_wait_st();
+      put(2, qq);
+      if (!syncw) {
+        bar_arrive1();
+      } else {
+        publish(4, true);
+        bool ok = true;
+        const double v = total(2, ok);
+        if (lane == 0) {
+          if (!ok) s_ok = 0;
+          s_scal = 0.0f;
+          s_inv = v > 0.0 ? static_cast<float>(1.0 / sqrt(v)) : 1.0f;
+          s_bprev = 0.0f;
+        }
+      }
+      __syncthreads();
+      if (!s_ok) return false;
+    }
+#pragma unroll 1
+    for (int j = 0; j < kLanczosSteps; ++j) {
+      const float aj = s_scal, inv = s_inv, bprev = s_bprev;
+      // q_prev = q, q = (w - a q) / b
+      auto next = [&](int c, float& r, float& d) {
+        const float q = (d - aj * r) * inv;
+        d = r;
+        r = q;
+        sm_f(a.o.x, c) = sqd(c) * q;
+      };
+      rounds([&](int c, bool ok, uint32_t t, uint32_t) {
+        float2 v = tm_ld2(t);
+        if (ok) next(c, v.x, v.y);
+        tm_st2(t, v.x, v.y);
+      });
+      rest([&](int c) { next(c, gr(c), gd(c)); });
+      tm_wait_st();
+      __syncthreads();
+      float qw = 0.0f, ww = 0.0f, qq = 0.0f;
+      auto epi = [&](int c, float q, float d, float y) {
+        const float w = sqd(c) * (y + ad(c).x * sm_f(a.o.x, c)) - bprev * d;
+        qw += q * w;
+        ww += w * w;
+        qq += q * q;
+        return w;
+      };
+      if (!apply(false, epi, []() {}, []() {})) return false;
+      put(0, qw);
+      put(1, ww);
+      put(2, qq);
+      if (!syncw) {
+        bar_arrive1();
+      } else {
+        publish(7, true);
+        bool ok = true;
+        const double tqw = total(0, ok), tww = total(1, ok), tqq = total(2, ok);
+        if (lane == 0) {
+          if (!ok) s_ok = 0;
+          const double av = tqq > 0.0 ? tqw / tqq : 0.0;
+          // below 1e-5 w.w the difference is the rounding of the float32
+          // vectors: the space is exhausted
+          const double b2 = tww - 2.0 * av * tqw + av * av * tqq;
+          const double bv = b2 > 1e-5 * tww ? sqrt(b2) : (b2 == b2 ? 0.0 : b2);
+          s_la[j] = av;
+          s_lb[j] = bv;
+          s_scal = static_cast<float>(av);
+          s_inv = bv > 0.0 ? static_cast<float>(1.0 / bv) : 0.0f;
+          s_bprev = static_cast<float>(bv);
+        }
+      }
+      __syncthreads();
+      if (!s_ok) return false;
+    }
+    if (syncw) {
+      const double lmax = lanczos_lmax(s_la, s_lb, kLanczosSteps);
+      if (lane == 0) {
+        double theta;
+        float it;
+        const bool ok = cheb_interval(lmax, deg, a.lo_ratio, s_c1, s_c2, &theta, &it);
+        if (!ok) status |= MGPBD_STATUS_NAN;
+        s_it = it;
+        if (blockIdx.x == 0) {
+          ChebCoef& f = a.js->cf;
+          for (int i = 0; i < kMaxCheb; ++i) {
+            f.c1[i] = s_c1[i];
+            f.c2[i] = s_c2[i];
+          }
+          f.theta = theta;
+          f.lmax = ok ? lmax : (isfinite(lmax) ? lmax : NAN);
+          f.inv_theta = it;
+          f.degree = deg;
+        }
+      }
+    }
+    __syncthreads();
+    return true;
+  };
+
   auto run = [&]() {
+    if (a.estimate) {
+      bool need = true;
+      if (a.per_problem) {  // a body whose Newton loop has ended needs none
+        float bb = 0.0f;
+        for (int c = tid; c < nC; c += nthr) {
+          const float bt = a.b[perm(c)];
+          bb += bt * bt;
+        }
+        put(0, bb);
+        if (!syncw) {
+          bar_arrive1();
+        } else {
+          publish(1, true);
+          bool ok = true;
+          const double v = total(0, ok);
+          if (lane == 0) {
+            if (!ok) s_ok = 0;
+            s_stop = v == 0.0;
+          }
+        }
+        __syncthreads();
+        if (!s_ok) return;
+        need = s_stop == 0;
+      }
+      if (need && !estimate()) return;
+      if (!need && tid == 0) s_it = 0.0f;
+      __syncthreads();
+    }
+    const float it = s_it;
     // x = 0 (or the warm start), r = b - A x, p = 0, z = d = D^-1 r / theta
     {
       float bb = 0.0f, bz = 0.0f, br = 0.0f;
@@ -844,70 +1066,22 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         acc += r * zn;
         return dn;
       };
-      if (CLUSTER && tid == nthr - 32) expect_bytes(smem_u32(&s_bar[(gen + 1) & 1]), 16 * B.nrecv);
       if (test && syncw) publish(2, false);
-      sums(++gen);
-      if (test) x_update(al);
-      __syncthreads();
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        if (half) {
-          if (CLUSTER) {
-            if (tid == nthr - 32) {
-              const uint32_t bar = smem_u32(&s_bar[gen & 1]), parity = (gen - 1) >> 1 & 1;
-              if (!bounded_wait(a, [&]() { return test_phase(bar, parity); })) s_ok = 0;
-            }
-            __syncthreads();
-          }
-          collect(gen);
-          if (test && syncw) {
+      const bool on = apply(
+          test, epi,
+          [&]() {
+            if (test) x_update(al);
+          },
+          [&]() {
+            if (!test) return;
             bool ok = true;
             const double sr = total(1, ok);
             if (lane == 0) {
               if (!ok) s_ok = 0;
               s_stop = rr_test(sr);
             }
-          }
-          __syncthreads();
-          if (!s_ok || (test && s_stop)) return;
-        }
-        // (J u)_c: rounds on private vertices before the wait, the others after
-#pragma unroll 1
-        for (int k = half ? kTi : 0; k < (half ? kT : kTi); ++k) {
-          const int c = k * nthr + tid;
-          const uint32_t t = tm0 + 16 * k;
-          uint32_t v[16];
-          tm_ld16(t, v);
-          float g[9];
-#pragma unroll
-          for (int m = 0; m < 9; ++m) g[m] = __uint_as_float(v[m]);
-          float d = __uint_as_float(v[kColR + 1]);
-          if (c < nTr) d = epi(c, __uint_as_float(v[kColR]), d, tet_dot(g, make_uint2(v[10], v[11])));
-          tm_st1(t + kColR + 1, d);
-        }
-#pragma unroll 1
-        for (int k = half ? kEi : 0; k < (half ? kE : kEi); ++k) {
-          const int e = k * nthr + tid;
-          const uint32_t t = tme + 8 * k;
-          uint32_t v[8];
-          tm_ld8(t, v);
-          float d = __uint_as_float(v[kEdgeR + 1]);
-          if (e < nEr)
-            d = epi(nT + e, __uint_as_float(v[kEdgeR]), d,
-                    edge_dot(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), v[3]));
-          tm_st1(t + kEdgeR + 1, d);
-        }
-        tm_wait_st();
-      }
-      // what is not held
-#pragma unroll 2
-      for (int c = nTr + tid; c < nT; c += nthr)
-        gd(c) = epi(c, gr(c), gd(c), tet_dot12(tg(0, c), tg(1, c), tg(2, c), ti(c)));
-#pragma unroll 2
-      for (int c = nT + nEr + tid; c < nC; c += nthr) {
-        const float4 g = tg(0, c);
-        gd(c) = epi(c, gr(c), gd(c), edge_dot(g.x, g.y, g.z, __float_as_uint(g.w)));
-      }
+          });
+      if (!on) return;
       if (!ap) {
         if (i == deg - 1) put(2, acc);
         else __syncthreads();
@@ -1190,9 +1364,9 @@ void launch_dcg_pack(const JView& j, const DcgDev& d, int64_t n_rows, cudaStream
 }
 
 void launch_dcg(const JView& j, const JcgVecs& v, const DcgPlan& plan, const DcgDev& d,
-                const JState* js, CgState* st, double tol_abs, double tol_rel, int maxiter,
-                int degree, bool warm, bool per_problem, int32_t* iters, double spin_limit_s,
-                cudaStream_t s, const JcgCtl* ctl) {
+                JState* js, CgState* st, double tol_abs, double tol_rel, int maxiter, int degree,
+                double lo_ratio, bool estimate, bool warm, bool per_problem, int32_t* iters,
+                double spin_limit_s, cudaStream_t s, const JcgCtl* ctl) {
   require(degree >= 1 && degree <= kMaxCheb, MGPBD_EINVAL, "Chebyshev degree out of range");
   require(plan.nblk > 0 && d.nc == j.nt, MGPBD_ESTATE, "dual CG partition not built");
   require(!(warm || ctl) || v.ulo != nullptr, MGPBD_EINVAL, "warm start needs the ulo scratch");
@@ -1212,6 +1386,8 @@ void launch_dcg(const JView& j, const JcgVecs& v, const DcgPlan& plan, const Dcg
   a.tol_rel = tol_rel;
   a.maxiter = maxiter;
   a.degree = degree;
+  a.lo_ratio = lo_ratio;
+  a.estimate = estimate ? 1 : 0;
   a.warm = warm ? 1 : 0;
   a.per_problem = per_problem ? 1 : 0;
   a.unit_dinv = j.unit_dinv ? 1 : 0;

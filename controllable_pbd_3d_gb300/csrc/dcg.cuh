@@ -53,11 +53,13 @@ void launch_dcg_pack(const JView& j, const DcgDev& d, int64_t n_rows, cudaStream
 // The whole solve; b, x, r and xc as in launch_jcg_persistent (original
 // order: x + xc is the solution, r its residual).  iters (nprob): each
 // problem's iterations, or null.  per_problem: a problem with b = 0 has
-// x = 0 at once (a body whose Newton loop has ended).
+// x = 0 at once (a body whose Newton loop has ended).  estimate: each problem's
+// Chebyshev interval [1.02 lmax lo_ratio, 1.02 lmax] comes from Lanczos steps of
+// its own first (problem 0's is left in js->cf); otherwise it is that of js->cf.
 void launch_dcg(const JView& j, const JcgVecs& v, const DcgPlan& plan, const DcgDev& d,
-                const JState* js, CgState* st, double tol_abs, double tol_rel, int maxiter,
-                int degree, bool warm, bool per_problem, int32_t* iters, double spin_limit_s,
-                cudaStream_t s, const JcgCtl* ctl = nullptr);
+                JState* js, CgState* st, double tol_abs, double tol_rel, int maxiter, int degree,
+                double lo_ratio, bool estimate, bool warm, bool per_problem, int32_t* iters,
+                double spin_limit_s, cudaStream_t s, const JcgCtl* ctl = nullptr);
 
 // A mesh of at most this many vertex entries (4 per 4-slot, 2 per length
 // constraint) runs on one cluster of 16 blocks, a larger one on the whole

@@ -185,6 +185,7 @@ class Solver {
   JView jview();
   JVecs jvecs(const float* b, float* x);
   void jform_setup(uint32_t* dev_status = nullptr);
+  void estimate_interval(uint32_t* dev_status);
   int32_t pcg_cheb(const float* b, float* x);
   void sync_read(void* host, const void* dev, size_t bytes);
   double finalize_read(const double* partials, int blocks);
@@ -282,6 +283,7 @@ class Solver {
   DevBuf<int32_t> jpart_;  // jplan_.vb then jplan_.tb
   // the partitioned dual CG (dcg.cuh): of the whole mesh, or of each body
   bool dcg_ready_ = false;
+  bool estimate_next_ = false;  // the next solve is the first with these gradients
   DcgPlan dplan_;
   DcgDev ddev_;
   DevBuf<DBlock> d_blocks_;

@@ -174,3 +174,24 @@ def test_solve_residual(cuda, dims, edges, kw, change):
   assert 1 <= it < 4000
   rel, floor = residual(s, n4)
   assert rel <= 1e-6 + floor, (rel, floor)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('dims,edges,kw', [((1, 1, 1), False, {}), ((6, 7, 5), True, dict(cheb_scale='jacobi')),
+                                           ((19, 20, 18), False, {})])
+def test_interval_of_one_fill(cuda, dims, edges, kw):
+  """Only the first solve after a fill estimates the Chebyshev interval; the
+  others of that fill use the same one: the same solution, bit for bit."""
+  torch = cuda
+  s = solver(torch, dims, edges, **kw)
+  s._compute_C_and_gradC()
+  s._compute_rhs_gpu()
+  out = []
+  for fill in (True, False, True):
+    if fill:
+      s._fill_A_and_update_gpu()
+    its = s._gpu_solver.solve(s._b_gpu, s._dlam_gpu)
+    out.append((its, s._dlam_gpu.cpu()))
+  assert out[0][0] > 0
+  for its, x in out[1:]:
+    assert its == out[0][0] and torch.equal(x, out[0][1])
