@@ -51,6 +51,7 @@
 #include <type_traits>
 
 #include "cheb_dev.cuh"
+#include "cluster_dev.cuh"
 #include "common.h"
 #include "dcg.cuh"
 #include "jform_dev.cuh"
@@ -62,6 +63,7 @@ namespace {
 
 using namespace jdev;
 using namespace pdev;
+using namespace cdev;
 
 struct DArgs {
   DcgDev d;
@@ -109,10 +111,6 @@ __device__ __forceinline__ uint16_t& sm_h(int off, int k) {
   return reinterpret_cast<uint16_t*>(s_dyn + off)[k];
 }
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // Named barrier 1: the other warps arrive and the last one waits
 __device__ __forceinline__ void bar_arrive1() {
   asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory");
@@ -142,48 +140,6 @@ __device__ __forceinline__ uint4 get_tagged(const void* p) {
       : "l"(p)
       : "memory");
   return v;
-}
-
-// The address of this block's shared address in block `rank` of the cluster
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-
-// Stores into another block's shared memory that complete there by counting
-// their bytes on its barrier: data and signal travel together, so neither
-// side needs a fence
-__device__ __forceinline__ void send_f4(uint32_t addr, uint32_t bar, float x, float y, float z) {
-  asm volatile(
-      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-      ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(0.0f), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void send_f64(uint32_t addr, uint32_t bar, double v) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr),
-               "d"(v), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void expect_bytes(uint32_t bar, uint32_t n) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
-}
-
-__device__ __forceinline__ bool test_phase(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ void cluster_meet() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
-               ::: "memory");
 }
 
 // Tensor memory as a second register file: a thread's lane and the columns

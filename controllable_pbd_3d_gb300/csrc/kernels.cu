@@ -700,12 +700,13 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kRowShapeG[kNumRowShapes] = {4, 4, 4, 2, 2, 4, 8, 8};
 constexpr int kRowShapeU[kNumRowShapes] = {6, 4, 8, 4, 8, 2, 2, 4};
 
+// (kSpmvDot writes one partial per block of its grid; the launches return it)
 template <int OP>
-void launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b, float* y,
+int launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b, float* y,
                       float w, double* partials, const CgState* st, cudaStream_t s,
                       const float* wp) {
   const int G = kRowShapeG[idx];
-  const int grid = OP == kSpmvDot ? reduce_blocks(a.n) : grid_for(a.n, kThreads / G);
+  const int grid = grid_for(a.n, kThreads / G);
   switch (idx) {
 #define MGPBD_VEC_CASE(I, GG, UU)                                                            \
   case I:                                                                                    \
@@ -725,23 +726,22 @@ void launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b,
       throw Error(MGPBD_EINVAL, "unknown row-kernel shape");
   }
   MGPBD_CHECK_LAUNCH();
+  return grid;
 }
 
 template <int OP>
-void rows_dispatch(const CsrView& a, const float* x, const float* b, float* y, float w,
+int rows_dispatch(const CsrView& a, const float* x, const float* b, float* y, float w,
                    double* partials, const CgState* st, cudaStream_t s, const float* wp = nullptr) {
-  if (a.n <= 0) return;
+  if (a.n <= 0) return 0;
   double avg = a.n ? (double)a.nnz / a.n : 0.0;
   if (a.padded && OP != kJacobiZero) {
     const int idx = a.shape >= 0 ? a.shape : (avg >= 40 ? 0 : 1);
-    launch_vec_shape<OP>(idx, a, x, b, y, w, partials, st, s, wp);
-    return;
+    return launch_vec_shape<OP>(idx, a, x, b, y, w, partials, st, s, wp);
   }
   int G = avg >= 48 ? 32 : (avg >= 20 ? 16 : (avg >= 8 ? 8 : 4));
   if (OP == kJacobiZero) G = 1;
   int rows_per_block = kThreads / G;
   int grid = grid_for(a.n, rows_per_block);
-  if (OP == kSpmvDot) grid = reduce_blocks(a.n);
   switch (G) {
 #define MGPBD_ROWS_CASE(GG)                                                                  \
   case GG:                                                                                   \
@@ -756,6 +756,7 @@ void rows_dispatch(const CsrView& a, const float* x, const float* b, float* y, f
 #undef MGPBD_ROWS_CASE
   }
   MGPBD_CHECK_LAUNCH();
+  return grid;
 }
 
 // P^T r for piecewise-constant P: sum of the members of each aggregate in
@@ -1004,7 +1005,10 @@ __global__ void k_chol_solve(const CgState* __restrict__ st, const double* __res
 }  // namespace
 
 // ===========================================================================
-int reduce_blocks(int64_t n) { return grid_for(n, kThreads * 4); }
+// One item a thread, up to the most blocks: with four, the reductions of a few
+// thousand items ran on 5 to 30 SMs (the line search of 5,000 constraints
+// 26 us); one more partial costs the sum nothing.
+int reduce_blocks(int64_t n) { return grid_for(n, kThreads); }
 
 void launch_rest_shape(const float* x_ref, const int32_t* t_i, const int32_t* ctype, int32_t nt,
                        float mu, float dt, float* dm_inv, float* rest_vol, float* alpha,
@@ -1154,9 +1158,6 @@ void launch_diag_inv_scan(const int32_t* indptr, const int32_t* indices, const f
 void launch_spmv(const CsrView& a, const float* x, float* y, cudaStream_t s) {
   rows_dispatch<kSpmv>(a, x, nullptr, y, 0.0f, nullptr, nullptr, s);
 }
-void launch_spmv_dot(const CsrView& a, const float* x, float* y, double* partials, cudaStream_t s) {
-  rows_dispatch<kSpmvDot>(a, x, nullptr, y, 0.0f, partials, nullptr, s);
-}
 void launch_jacobi(const CsrView& a, const float* b, const float* x, float* x_new, float w,
                    cudaStream_t s) {
   if (x) rows_dispatch<kJacobi>(a, x, b, x_new, w, nullptr, nullptr, s);
@@ -1199,9 +1200,9 @@ void launch_prolong_add_g(const CgState* st, const int32_t* agg, const float* xc
   k_prolong_add<<<grid_for(n, kThreads), kThreads, 0, s>>>(agg, xc, n, x, st);
   MGPBD_CHECK_LAUNCH();
 }
-void launch_spmv_dot_g(const CgState* st, const CsrView& a, const float* x, float* y, double* partials,
-                       cudaStream_t s) {
-  rows_dispatch<kSpmvDot>(a, x, nullptr, y, 0.0f, partials, st, s);
+int launch_spmv_dot_g(const CgState* st, const CsrView& a, const float* x, float* y, double* partials,
+                      cudaStream_t s) {
+  return rows_dispatch<kSpmvDot>(a, x, nullptr, y, 0.0f, partials, st, s);
 }
 void launch_dot_partials_g(const CgState* st, const float* a, const float* b, int64_t n,
                            double* partials, cudaStream_t s) {

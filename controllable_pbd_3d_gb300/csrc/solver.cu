@@ -1311,8 +1311,8 @@ void Solver::cg_body(const float* b, float* x) {
   CgState* st = cg_state_.p;
   int64_t n = nt_;
   int blocks = reduce_blocks(n);
-  launch_spmv_dot_g(st, levels_[0].view(), cg_p_.p, cg_ap_.p, partials_.p, s);
-  launch_cg_alpha(st, partials_.p, blocks, s);
+  const int dot_blocks = launch_spmv_dot_g(st, levels_[0].view(), cg_p_.p, cg_ap_.p, partials_.p, s);
+  launch_cg_alpha(st, partials_.p, dot_blocks, s);
   launch_cg_update_xr(st, cg_p_.p, cg_ap_.p, x, cg_r_.p, n, partials_.p, s);
   launch_cg_check(st, partials_.p, blocks, s);
   precondition(st);
