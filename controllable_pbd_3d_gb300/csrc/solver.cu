@@ -685,6 +685,15 @@ void Solver::alloc_work() {
     k_fill_f32<<<1, 32, 0, s>>>(L.omega.p, p_.omega_jacobi, 1);
     MGPBD_CHECK_LAUNCH();
   }
+  // the coarsest level's rows on a cluster
+  sweep_ = SweepPlan();
+  if (!cheb()) {
+    std::vector<int32_t> ip(levels_.back().n + 1);
+    MGPBD_CUDA(cudaMemcpyAsync(ip.data(), levels_.back().indptr.p, sizeof(int32_t) * ip.size(),
+                               cudaMemcpyDeviceToHost, s));
+    MGPBD_CUDA(cudaStreamSynchronize(s));
+    build_sweep_plan(ip, levels_.back().n, sweep_, s);
+  }
   cg_r_.alloc(nt_);
   cg_z_.alloc(nt_);
   cg_p_.alloc(nt_);
@@ -1141,6 +1150,24 @@ void Solver::smooth_level(int32_t l, const float* b, float*& cur, float*& nxt, i
   if (sweeps == 0 && from_zero) MGPBD_CUDA(cudaMemsetAsync(cur, 0, sizeof(float) * L.n, stream_));
 }
 
+int Solver::n_coarse_sweeps() const {
+  return p_.coarse_sweeps > 0 ? p_.coarse_sweeps : std::min(50, levels_.back().n);
+}
+
+// Whether the coarsest level's sweeps run as one kernel: where its matrix fits
+// into a cluster, from four sweeps on (the kernel's start is about that many
+// launches).
+bool Solver::fused_sweeps() const {
+  return sweep_.blocks > 0 && p_.coarse_solver != MGPBD_COARSE_DENSE_F64 && n_coarse_sweeps() >= 4;
+}
+
+// The coarsest level's correction into its xa (launch_sweeps)
+void Solver::coarse_sweeps(const float* b, const SweepTransfer& t, const CgState* guard) {
+  Level& L = levels_.back();
+  launch_sweeps(guard, L.view(), sweep_, b, p_.omega_jacobi, L.omega.p, n_coarse_sweeps(),
+                p_.mode == MGPBD_MODE_FAST, L.xa.p, t, &cg_state_.p->status, stream_);
+}
+
 // GPUMultigridSolver.vcycle (cons/mgpcg_gpu.py:214-259) with a zero initial
 // guess; the result ends in levels_[l].xa.
 void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
@@ -1152,8 +1179,11 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
       launch_dense_chol_solve(guard, chol_.p, L.n, b, L.xa.p, stream_);
       return;
     }
-    int sweeps = p_.coarse_sweeps > 0 ? p_.coarse_sweeps : std::min(50, L.n);
-    smooth_level(l, b, cur, nxt, sweeps, true, guard);
+    if (fused_sweeps()) {
+      coarse_sweeps(b, SweepTransfer(), guard);
+      return;
+    }
+    smooth_level(l, b, cur, nxt, n_coarse_sweeps(), true, guard);
   } else {
     smooth_level(l, b, cur, nxt, p_.n_smooth, true, guard);
     Level& C = levels_[l + 1];
@@ -1161,12 +1191,27 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
     // in the reference (cons/mgpcg_gpu.py:239-240 with :275)
     float* res = (l == 0 && p_.cg_alias) ? cg_r_.p : L.r.p;
     launch_residual_g(guard, L.view(), b, cur, res, stream_);
-    launch_restrict_g(guard, L.mem_ptr.p, L.mem_rows.p, res, C.n, C.b.p, stream_);
-    if (l == 0)
-      coarse_correction(guard);
-    else
-      vcycle(l + 1, C.b.p, guard);
-    launch_prolong_add_g(guard, L.agg.p, C.xa.p, L.n, cur, stream_);
+    // (a level-0 correction that is judged, learned or recorded is not only
+    // the sweeps)
+    const bool plain = l > 0 || !(judge_pending_ || net_active_ || rec_count_ < rec_cap_);
+    if (l + 1 == n_levels() - 1 && fused_sweeps() && plain) {
+      SweepTransfer t;
+      t.r = res;
+      t.b_out = C.b.p;
+      t.mem_ptr = L.mem_ptr.p;
+      t.mem_rows = L.mem_rows.p;
+      t.agg = L.agg.p;
+      t.xf = cur;
+      t.nf = L.n;
+      coarse_sweeps(nullptr, t, guard);
+    } else {
+      launch_restrict_g(guard, L.mem_ptr.p, L.mem_rows.p, res, C.n, C.b.p, stream_);
+      if (l == 0)
+        coarse_correction(guard);
+      else
+        vcycle(l + 1, C.b.p, guard);
+      launch_prolong_add_g(guard, L.agg.p, C.xa.p, L.n, cur, stream_);
+    }
     smooth_level(l, b, cur, nxt, p_.n_smooth, false, guard);
   }
   if (cur != L.xa.p)

@@ -16,6 +16,7 @@
 #include "mpnn.cuh"
 #include "rap.cuh"
 #include "structure.h"
+#include "sweep.cuh"
 
 namespace mgpbd {
 
@@ -162,6 +163,9 @@ class Solver {
   void alloc_work();
   // V-cycle on `l` with rhs b_l (device) and zero initial guess; the result
   // is left in levels_[l].xa.
+  int n_coarse_sweeps() const;
+  bool fused_sweeps() const;
+  void coarse_sweeps(const float* b, const SweepTransfer& t, const CgState* guard);
   void vcycle(int32_t l, const float* b, const CgState* guard);
   void smooth_level(int32_t l, const float* b, float*& cur, float*& nxt, int sweeps,
                     bool from_zero, const CgState* guard);
@@ -281,6 +285,7 @@ class Solver {
   DevBuf<float> ps_;       // primal CG tet scratch
   bool primal() const { return cheb() && p_.persistent && p_.primal; }
   DevBuf<int32_t> jpart_;  // jplan_.vb then jplan_.tb
+  SweepPlan sweep_;  // of the coarsest level
   // the partitioned dual CG (dcg.cuh): of the whole mesh, or of each body
   bool dcg_ready_ = false;
   bool estimate_next_ = false;  // the next solve is the first with these gradients

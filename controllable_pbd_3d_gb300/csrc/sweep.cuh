@@ -1,0 +1,46 @@
+// Jacobi sweeps on the coarsest multigrid level by one thread-block cluster
+// (sweep.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <vector>
+
+#include "common.h"
+#include "kernels.cuh"
+
+namespace mgpbd {
+
+// How a matrix is spread over the cluster.  blocks == 0: it is not (it does
+// not fit into the blocks' shared memory).
+struct SweepPlan {
+  int32_t blocks = 0, lanes = 0;  // blocks of the cluster, lanes of a row
+  int32_t rows = 0, quads = 0;    // the most rows and 4-element groups of a block
+  int32_t smem = 0;
+  DevBuf<int32_t> dev;  // first row of each block and the end, first group of each row
+};
+
+// indptr: the matrix's n + 1 row offsets (host)
+void build_sweep_plan(const std::vector<int32_t>& indptr, int32_t n, SweepPlan& plan, cudaStream_t s);
+
+// What surrounds the sweeps: r (not null): their b is the sum of r over each
+// row's members (k_restrict), left in b_out; xf (not null): xf[i] += x[agg[i]]
+// for the nf fine rows afterwards (k_prolong_add).
+struct SweepTransfer {
+  const float* r = nullptr;
+  float* b_out = nullptr;
+  const int32_t *mem_ptr = nullptr, *mem_rows = nullptr, *agg = nullptr;
+  float* xf = nullptr;
+  int32_t nf = 0;
+};
+
+// x = `sweeps` sweeps x += w D^-1 (b - A x) from x = 0, w from w_dev when not
+// null; zero_first: the first sweep is written down as w D^-1 b.  A no-op
+// once st->done.  A wait that gave up leaves NaN in x (and xf) and
+// MGPBD_STATUS_SYNC_TIMEOUT in *status.
+void launch_sweeps(const CgState* st, const CsrView& a, const SweepPlan& plan, const float* b, float w,
+                   const float* w_dev, int32_t sweeps, bool zero_first, float* x,
+                   const SweepTransfer& t, int32_t* status, cudaStream_t s);
+
+}  // namespace mgpbd
