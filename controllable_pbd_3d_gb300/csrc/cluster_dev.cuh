@@ -51,6 +51,20 @@ __device__ __forceinline__ bool test_phase(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same, but the warp may be suspended for a (bounded) while first: it leaves
+// the issue slots to the others
+__device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 __device__ __forceinline__ void cluster_meet() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
                ::: "memory");

@@ -687,12 +687,15 @@ void Solver::alloc_work() {
   }
   // the coarsest level's rows on a cluster
   sweep_ = SweepPlan();
-  if (!cheb()) {
-    std::vector<int32_t> ip(levels_.back().n + 1);
-    MGPBD_CUDA(cudaMemcpyAsync(ip.data(), levels_.back().indptr.p, sizeof(int32_t) * ip.size(),
+  if (!cheb() && levels_.back().nnz <= kSweepMaxNnz) {
+    const Level& L = levels_.back();
+    std::vector<int32_t> ip(L.n + 1), ix(L.nnz);
+    MGPBD_CUDA(cudaMemcpyAsync(ip.data(), L.indptr.p, sizeof(int32_t) * ip.size(),
+                               cudaMemcpyDeviceToHost, s));
+    MGPBD_CUDA(cudaMemcpyAsync(ix.data(), L.indices.p, sizeof(int32_t) * ix.size(),
                                cudaMemcpyDeviceToHost, s));
     MGPBD_CUDA(cudaStreamSynchronize(s));
-    build_sweep_plan(ip, levels_.back().n, sweep_, s);
+    build_sweep_plan(ip, ix, L.n, sweep_, s);
   }
   cg_r_.alloc(nt_);
   cg_z_.alloc(nt_);
@@ -1200,9 +1203,7 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
       t.b_out = C.b.p;
       t.mem_ptr = L.mem_ptr.p;
       t.mem_rows = L.mem_rows.p;
-      t.agg = L.agg.p;
       t.xf = cur;
-      t.nf = L.n;
       coarse_sweeps(nullptr, t, guard);
     } else {
       launch_restrict_g(guard, L.mem_ptr.p, L.mem_rows.p, res, C.n, C.b.p, stream_);

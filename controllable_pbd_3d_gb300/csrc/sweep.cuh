@@ -15,24 +15,30 @@ namespace mgpbd {
 // How a matrix is spread over the cluster.  blocks == 0: it is not (it does
 // not fit into the blocks' shared memory).
 struct SweepPlan {
-  int32_t blocks = 0, lanes = 0;  // blocks of the cluster, lanes of a row
-  int32_t rows = 0, quads = 0;    // the most rows and 4-element groups of a block
+  int32_t blocks = 0, lanes = 0;       // blocks of the cluster, lanes of a row
+  int32_t rows = 0, groups = 0, nx = 0;  // the most rows, 4-element groups and x of a block
   int32_t smem = 0;
-  DevBuf<int32_t> dev;  // first row of each block and the end, first group of each row
+  // first row of each block and the end, quads of x that a block receives,
+  // first group of each block; first group of each row in its block
+  DevBuf<int32_t> dev;
+  DevBuf<uint16_t> cols;  // columns of the groups, as positions in the block's x
+  DevBuf<uint16_t> pos;   // where each block keeps a quad of rows (kSweepNone: nowhere)
 };
+constexpr uint16_t kSweepNone = 0xffff;
+constexpr int64_t kSweepMaxNnz = 1 << 20;  // the values of more exceed 16 blocks' shared memory
 
-// indptr: the matrix's n + 1 row offsets (host)
-void build_sweep_plan(const std::vector<int32_t>& indptr, int32_t n, SweepPlan& plan, cudaStream_t s);
+// The plan of a matrix of n rows (host structure).
+void build_sweep_plan(const std::vector<int32_t>& indptr, const std::vector<int32_t>& indices,
+                      int32_t n, SweepPlan& plan, cudaStream_t s);
 
 // What surrounds the sweeps: r (not null): their b is the sum of r over each
-// row's members (k_restrict), left in b_out; xf (not null): xf[i] += x[agg[i]]
-// for the nf fine rows afterwards (k_prolong_add).
+// row's members (k_restrict), left in b_out; xf (not null): x of each row is
+// added to xf of its members afterwards (k_prolong_add).
 struct SweepTransfer {
   const float* r = nullptr;
   float* b_out = nullptr;
-  const int32_t *mem_ptr = nullptr, *mem_rows = nullptr, *agg = nullptr;
+  const int32_t *mem_ptr = nullptr, *mem_rows = nullptr;
   float* xf = nullptr;
-  int32_t nf = 0;
 };
 
 // x = `sweeps` sweeps x += w D^-1 (b - A x) from x = 0, w from w_dev when not
