@@ -40,15 +40,18 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Block-wide float64 sum in a fixed pattern; result valid in thread 0.
+// Sum over the block (at most kThreads), in thread 0.  One warp adds: float64
+// additions are slow here (2 a clock and SM), and a tree in every warp takes
+// four times as many.
 __device__ __forceinline__ double block_sum(double v) {
-  __shared__ double sh[32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  v = warp_sum(v);
-  if (lane == 0) sh[wid] = v;
+  __shared__ double sh[kThreads];
+  sh[threadIdx.x] = v;
   __syncthreads();
-  int nw = (blockDim.x + 31) >> 5;
-  v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
-  if (wid == 0) v = warp_sum(v);
+  v = 0.0;
+  if (threadIdx.x < 32) {
+    for (int i = threadIdx.x; i < blockDim.x; i += 32) v += sh[i];
+    v = warp_sum(v);
+  }
   __syncthreads();
   return v;
 }
@@ -565,9 +568,88 @@ __global__ void k_diag_inv_scan(const int32_t* __restrict__ indptr, const int32_
   }
 }
 
+// Sum of the partials of a launch, in their order, by one warp: in all threads
+__device__ double sum_partials(const double* __restrict__ p, int blocks) {
+  __shared__ double sum;
+  if (threadIdx.x < 32) {
+    double acc = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < blocks; i += 32) acc += p[i];
+    acc = warp_sum(acc);
+    if (threadIdx.x == 0) sum = acc;
+  }
+  __syncthreads();
+  const double v = sum;
+  __syncthreads();
+  return v;
+}
+
+// ---------------------------------------------------------------------------
+// CG scalar steps (GPUMultigridSolver.solve, cons/mgpcg_gpu.py:289-327).  Each
+// block of the kernel that needs a scalar adds the partials of the launch
+// before it; block 0 leaves the result in the state.  (As one-block kernels of
+// their own these steps were three of the 16 launches of an iteration; made by
+// the last block of the launch before, the tickets and fences took 6 us each.)
+// True: go on.  A block that starts late may find the `done` that block 0
+// leaves here, and ends as all others do.
+__device__ bool cg_alpha(CgState* st, const double* p, int blocks, double* alpha) {
+  const double pap = sum_partials(p, blocks), a = st->rz / pap;
+  const bool bad = fabs(pap) < 1e-30 || !isfinite(pap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->pap = pap;
+    if (!isfinite(pap)) st->status |= MGPBD_STATUS_NAN;
+    if (bad) {
+      st->done = 1;
+    } else {
+      if (pap <= 0.0) st->status |= MGPBD_STATUS_PAP_NONPOS;
+      st->alpha = a;
+    }
+  }
+  *alpha = a;
+  return !bad;
+}
+
+__device__ bool cg_check(CgState* st, const double* p, int blocks) {
+  const double rr = sum_partials(p, blocks);
+  const bool nan = !isfinite(rr), stop = nan || rr < st->tol2;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->rr = rr;
+    if (stop) {
+      if (nan) st->status |= MGPBD_STATUS_NAN;
+      else st->iters += 1;
+      st->done = 1;
+    }
+  }
+  return !stop;
+}
+
+// rz of the next iteration is left in rz_new (the others still read rz), and
+// moved by the next iteration's SpMV
+__device__ bool cg_beta(CgState* st, const double* p, int blocks, double* beta) {
+  const double rzn = sum_partials(p, blocks), rz = st->rz;
+  const bool bad = fabs(rz) < 1e-30;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->rz_new = rzn;
+    st->iters += 1;
+    if (bad) {
+      st->done = 1;
+    } else {
+      st->beta = rzn / rz;
+      if (st->iters >= st->maxiter) {
+        st->done = 1;
+        st->status |= MGPBD_STATUS_CG_MAXITER;
+      }
+    }
+  }
+  *beta = rzn / rz;
+  return !bad;
+}
+
 // ---------------------------------------------------------------------------
 // Row operators on CSR: G lanes per row, rows strided over a fixed grid.
-enum RowOp { kSpmv = 0, kJacobi = 1, kResidual = 2, kSpmvDot = 3, kJacobiZero = 4 };
+// kSpmvDot: y = A x and partials of x.y; kJacobiDot: a sweep and those of b.y.
+// check: the partials of CG's r.r, when its stopping test is still to be made.
+enum RowOp { kSpmv = 0, kJacobi = 1, kResidual = 2, kSpmvDot = 3, kJacobiZero = 4, kJacobiDot = 5 };
 
 template <int G, int OP>
 __global__ void __launch_bounds__(kThreads)
@@ -575,8 +657,10 @@ __global__ void __launch_bounds__(kThreads)
                const float* __restrict__ data, const float* __restrict__ x,
                const float* __restrict__ b, const float* __restrict__ dinv, float* __restrict__ y,
                float w, const float* __restrict__ wp, double* __restrict__ partials,
-               const CgState* __restrict__ st) {
+               CgState* st, const double* __restrict__ check, int check_blocks) {
   if (st && st->done) return;
+  if (check && !cg_check(st, check, check_blocks)) return;
+  if (OP == kSpmvDot && blockIdx.x == 0 && threadIdx.x == 0) st->rz = st->rz_new;
   if (wp) w = *wp;
   // The loop bound is uniform per warp (all 32/G rows of a warp advance
   // together), so every lane reaches the shuffles.
@@ -607,12 +691,16 @@ __global__ void __launch_bounds__(kThreads)
         y[row] = b[row] - sum;
       } else if (OP == kJacobi) {
         y[row] = x[row] + w * dinv[row] * (b[row] - sum);
+      } else if (OP == kJacobiDot) {
+        const float v = x[row] + w * dinv[row] * (b[row] - sum);
+        y[row] = v;
+        dacc += (double)b[row] * (double)v;
       } else {  // x = 0: A x = 0 exactly for finite A
         y[row] = w * dinv[row] * b[row];
       }
     }
   }
-  if (OP == kSpmvDot) {
+  if (OP == kSpmvDot || OP == kJacobiDot) {
     dacc = block_sum(dacc);
     if (threadIdx.x == 0) partials[blockIdx.x] = dacc;
   }
@@ -632,8 +720,10 @@ __global__ void __launch_bounds__(kThreads)
                    const float* __restrict__ x, const float* __restrict__ b,
                    const float* __restrict__ dinv, float* __restrict__ y, float w,
                    const float* __restrict__ wp, double* __restrict__ partials,
-                   const CgState* __restrict__ st) {
+                   CgState* st, const double* __restrict__ check, int check_blocks) {
   if (st && st->done) return;
+  if (check && !cg_check(st, check, check_blocks)) return;
+  if (OP == kSpmvDot && blockIdx.x == 0 && threadIdx.x == 0) st->rz = st->rz_new;
   if (wp) w = *wp;
   const int lane = threadIdx.x % G;
   constexpr int kRowsPerWarp = 32 / G;
@@ -681,11 +771,13 @@ __global__ void __launch_bounds__(kThreads)
       } else if (OP == kResidual) {
         y[row] = b[row] - sum;
       } else {
-        y[row] = x[row] + w * dinv[row] * (b[row] - sum);
+        const float v = x[row] + w * dinv[row] * (b[row] - sum);
+        y[row] = v;
+        if (OP == kJacobiDot) dacc += (double)b[row] * (double)v;
       }
     }
   }
-  if (OP == kSpmvDot) {
+  if (OP == kSpmvDot || OP == kJacobiDot) {
     dacc = block_sum(dacc);
     if (threadIdx.x == 0) partials[blockIdx.x] = dacc;
   }
@@ -700,18 +792,19 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kRowShapeG[kNumRowShapes] = {4, 4, 4, 2, 2, 4, 8, 8};
 constexpr int kRowShapeU[kNumRowShapes] = {6, 4, 8, 4, 8, 2, 2, 4};
 
-// (kSpmvDot writes one partial per block of its grid; the launches return it)
+// (the launches return their blocks: the partials of the dot operators)
 template <int OP>
 int launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b, float* y,
-                      float w, double* partials, const CgState* st, cudaStream_t s,
-                      const float* wp) {
+                      float w, double* partials, CgState* st, cudaStream_t s, const float* wp = nullptr,
+                     const CgCheck& check = {}) {
   const int G = kRowShapeG[idx];
   const int grid = grid_for(a.n, kThreads / G);
   switch (idx) {
 #define MGPBD_VEC_CASE(I, GG, UU)                                                            \
   case I:                                                                                    \
     k_csr_rows_vec<GG, UU, OP><<<grid, kThreads, 0, s>>>(a.n, a.indptr, a.indices, a.data, x, \
-                                                         b, a.diag_inv, y, w, wp, partials, st); \
+                                                         b, a.diag_inv, y, w, wp, partials, st, \
+                                                         check.partials, check.blocks); \
     break;
     MGPBD_VEC_CASE(0, 4, 6)
     MGPBD_VEC_CASE(1, 4, 4)
@@ -731,12 +824,13 @@ int launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b, 
 
 template <int OP>
 int rows_dispatch(const CsrView& a, const float* x, const float* b, float* y, float w,
-                   double* partials, const CgState* st, cudaStream_t s, const float* wp = nullptr) {
+                  double* partials, CgState* st, cudaStream_t s, const float* wp = nullptr,
+                  const CgCheck& check = {}) {
   if (a.n <= 0) return 0;
   double avg = a.n ? (double)a.nnz / a.n : 0.0;
   if (a.padded && OP != kJacobiZero) {
     const int idx = a.shape >= 0 ? a.shape : (avg >= 40 ? 0 : 1);
-    return launch_vec_shape<OP>(idx, a, x, b, y, w, partials, st, s, wp);
+    return launch_vec_shape<OP>(idx, a, x, b, y, w, partials, st, s, wp, check);
   }
   int G = avg >= 48 ? 32 : (avg >= 20 ? 16 : (avg >= 8 ? 8 : 4));
   if (OP == kJacobiZero) G = 1;
@@ -746,7 +840,8 @@ int rows_dispatch(const CsrView& a, const float* x, const float* b, float* y, fl
 #define MGPBD_ROWS_CASE(GG)                                                                  \
   case GG:                                                                                   \
     k_csr_rows<GG, OP><<<grid, kThreads, 0, s>>>(a.n, a.indptr, a.indices, a.data, x, b,     \
-                                                 a.diag_inv, y, w, wp, partials, st);        \
+                                                 a.diag_inv, y, w, wp, partials, st,         \
+                                                 check.partials, check.blocks);              \
     break;
     MGPBD_ROWS_CASE(1)
     MGPBD_ROWS_CASE(4)
@@ -812,12 +907,6 @@ __global__ void k_xpay(float alpha, const float* __restrict__ x, float* __restri
     y[i] = x[i] + alpha * y[i];
 }
 
-__device__ double sum_partials(const double* __restrict__ p, int blocks) {
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < blocks; i += blockDim.x) acc += p[i];
-  return block_sum(acc);
-}
-
 __global__ void k_finalize(const double* __restrict__ partials, int blocks, int count,
                            double* __restrict__ out) {
   for (int g = 0; g < count; ++g) {
@@ -843,76 +932,41 @@ __global__ void k_cg_init(CgState* st, const double* __restrict__ p, int blocks,
     st->status = isfinite(rz) ? 0 : MGPBD_STATUS_NAN;
     st->maxiter = maxiter;
     st->body_runs = 0;
-    st->alpha = st->beta = st->pap = st->rr = st->rz_new = 0.0;
+    st->alpha = st->beta = st->pap = st->rr = 0.0;
+    st->rz_new = rz;
   }
 }
 
-__global__ void k_cg_alpha(CgState* st, const double* __restrict__ p, int blocks) {
+// alpha; x += alpha p; r -= alpha Ap; partials of r.r.  z (not null): the first
+// smoothing sweep of the V-cycle that follows, z = w D^-1 r, is made here,
+// where r is at hand.
+__global__ void k_cg_update_xr(CgState* st, const double* __restrict__ pap, int blocks,
+                               const float* __restrict__ p, const float* __restrict__ ap,
+                               float* __restrict__ x, float* __restrict__ r, int64_t n,
+                               double* __restrict__ partials, const float* __restrict__ dinv,
+                               const float* __restrict__ wp, float* __restrict__ z) {
   if (st->done) return;
-  double pap = sum_partials(p, blocks);
-  if (threadIdx.x == 0) {
-    st->pap = pap;
-    if (!isfinite(pap)) st->status |= MGPBD_STATUS_NAN;
-    if (fabs(pap) < 1e-30 || !isfinite(pap)) {
-      st->done = 1;
-    } else {
-      if (pap <= 0.0) st->status |= MGPBD_STATUS_PAP_NONPOS;
-      st->alpha = st->rz / pap;
-    }
-  }
-}
-
-__global__ void k_cg_update_xr(const CgState* __restrict__ st, const float* __restrict__ p,
-                               const float* __restrict__ ap, float* __restrict__ x,
-                               float* __restrict__ r, int64_t n, double* __restrict__ partials) {
-  if (st->done) return;
-  float a = (float)st->alpha;
-  float na = (float)(-st->alpha);
+  double alpha;
+  if (!cg_alpha(st, pap, blocks, &alpha)) return;
+  float a = (float)alpha;
+  float na = (float)(-alpha);
+  const float w = z ? *wp : 0.0f;
   double acc = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     x[i] += a * p[i];
     float ri = r[i] + na * ap[i];
     r[i] = ri;
+    if (z) z[i] = w * dinv[i] * ri;
     acc += (double)ri * (double)ri;
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
 }
 
+// the stopping test where no row operator follows
 __global__ void k_cg_check(CgState* st, const double* __restrict__ p, int blocks) {
-  if (st->done) return;
-  double rr = sum_partials(p, blocks);
-  if (threadIdx.x == 0) {
-    st->rr = rr;
-    if (!isfinite(rr)) {
-      st->status |= MGPBD_STATUS_NAN;
-      st->done = 1;
-    } else if (rr < st->tol2) {
-      st->iters += 1;
-      st->done = 1;
-    }
-  }
-}
-
-__global__ void k_cg_beta(CgState* st, const double* __restrict__ p, int blocks) {
-  if (st->done) return;
-  double rzn = sum_partials(p, blocks);
-  if (threadIdx.x == 0) {
-    st->rz_new = rzn;
-    if (fabs(st->rz) < 1e-30) {
-      st->iters += 1;
-      st->done = 1;
-      return;
-    }
-    st->beta = rzn / st->rz;
-    st->rz = rzn;
-    st->iters += 1;
-    if (st->iters >= st->maxiter) {
-      st->done = 1;
-      st->status |= MGPBD_STATUS_CG_MAXITER;
-    }
-  }
+  if (!st->done) cg_check(st, p, blocks);
 }
 
 // Restart of a CG solve from its current iterate: rz from the partials,
@@ -921,17 +975,26 @@ __global__ void k_cg_restart(CgState* st, const double* __restrict__ p, int bloc
                              int32_t clear_mask) {
   double rz = sum_partials(p, blocks);
   if (threadIdx.x == 0) {
-    st->rz = rz;
+    st->rz = st->rz_new = rz;
     st->status &= ~clear_mask;
     if (!isfinite(rz)) st->status |= MGPBD_STATUS_NAN;
     st->done = (st->iters >= st->maxiter || !isfinite(rz)) ? 1 : 0;
   }
 }
 
-__global__ void k_cg_update_p(const CgState* __restrict__ st, const float* __restrict__ z,
-                              float* __restrict__ p, int64_t n) {
-  if (st->done) return;
-  float bt = (float)st->beta;
+// beta; p = z + beta p; loop: the captured iteration's end, its condition is
+// set here
+__global__ void k_cg_update_p(CgState* st, const double* __restrict__ rz, int blocks,
+                              const float* __restrict__ z, float* __restrict__ p, int64_t n,
+                              cudaGraphConditionalHandle handle, int loop) {
+  double beta = 0.0;
+  const bool go = !st->done && cg_beta(st, rz, blocks, &beta);
+  if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
+    st->body_runs += 1;
+    cudaGraphSetConditional(handle, st->done ? 0u : 1u);
+  }
+  if (!go) return;
+  float bt = (float)beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     p[i] = z[i] + bt * p[i];
@@ -1174,19 +1237,14 @@ void launch_prolong_add(const int32_t* agg, const float* xc, int32_t n, float* x
   launch_prolong_add_g(nullptr, agg, xc, n, x, s);
 }
 
-void launch_jacobi_g(const CgState* st, const CsrView& a, const float* b, const float* x, float* x_new,
-                     float w, cudaStream_t s) {
-  if (x) rows_dispatch<kJacobi>(a, x, b, x_new, w, nullptr, st, s);
-  else rows_dispatch<kJacobiZero>(a, nullptr, b, x_new, w, nullptr, st, s);
+void launch_jacobi_gw(CgState* st, const CsrView& a, const float* b, const float* x, float* x_new,
+                      float w, const float* w_dev, const CgCheck& check, cudaStream_t s) {
+  if (x) rows_dispatch<kJacobi>(a, x, b, x_new, w, nullptr, st, s, w_dev, check);
+  else rows_dispatch<kJacobiZero>(a, nullptr, b, x_new, w, nullptr, st, s, w_dev, check);
 }
-void launch_jacobi_gw(const CgState* st, const CsrView& a, const float* b, const float* x,
-                      float* x_new, float w, const float* w_dev, cudaStream_t s) {
-  if (x) rows_dispatch<kJacobi>(a, x, b, x_new, w, nullptr, st, s, w_dev);
-  else rows_dispatch<kJacobiZero>(a, nullptr, b, x_new, w, nullptr, st, s, w_dev);
-}
-void launch_residual_g(const CgState* st, const CsrView& a, const float* b, const float* x, float* r,
-                       cudaStream_t s) {
-  rows_dispatch<kResidual>(a, x, b, r, 0.0f, nullptr, st, s);
+void launch_residual_g(CgState* st, const CsrView& a, const float* b, const float* x, float* r,
+                       const CgCheck& check, cudaStream_t s) {
+  rows_dispatch<kResidual>(a, x, b, r, 0.0f, nullptr, st, s, nullptr, check);
 }
 void launch_restrict_g(const CgState* st, const int32_t* mem_ptr, const int32_t* mem_rows,
                        const float* r, int32_t nc, float* bc, cudaStream_t s) {
@@ -1200,18 +1258,25 @@ void launch_prolong_add_g(const CgState* st, const int32_t* agg, const float* xc
   k_prolong_add<<<grid_for(n, kThreads), kThreads, 0, s>>>(agg, xc, n, x, st);
   MGPBD_CHECK_LAUNCH();
 }
-int launch_spmv_dot_g(const CgState* st, const CsrView& a, const float* x, float* y, double* partials,
-                      cudaStream_t s) {
+int launch_cg_spmv_dot(CgState* st, const CsrView& a, const float* x, float* y, double* partials,
+                       cudaStream_t s) {
   return rows_dispatch<kSpmvDot>(a, x, nullptr, y, 0.0f, partials, st, s);
 }
-void launch_dot_partials_g(const CgState* st, const float* a, const float* b, int64_t n,
-                           double* partials, cudaStream_t s) {
+int launch_cg_jacobi_dot(CgState* st, const CsrView& a, const float* b, const float* x, float* x_new,
+                         float w, const float* w_dev, double* partials, const CgCheck& check,
+                         cudaStream_t s) {
+  return rows_dispatch<kJacobiDot>(a, x, b, x_new, w, partials, st, s, w_dev, check);
+}
+int launch_cg_dot(CgState* st, const float* a, const float* b, int64_t n, double* partials,
+                  cudaStream_t s) {
   k_dot<<<reduce_blocks(n), kThreads, 0, s>>>(a, b, n, partials, st);
   MGPBD_CHECK_LAUNCH();
+  return reduce_blocks(n);
 }
 
 void launch_dot_partials(const float* a, const float* b, int64_t n, double* partials, cudaStream_t s) {
-  launch_dot_partials_g(nullptr, a, b, n, partials, s);
+  k_dot<<<reduce_blocks(n), kThreads, 0, s>>>(a, b, n, partials, nullptr);
+  MGPBD_CHECK_LAUNCH();
 }
 void launch_axpy(float alpha, const float* x, float* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
@@ -1238,21 +1303,16 @@ void launch_cg_init(CgState* st, const double* partials_rz, int blocks, double t
   k_cg_init<<<1, kThreads, 0, s>>>(st, partials_rz, blocks, tol_abs, tol_rel, maxiter);
   MGPBD_CHECK_LAUNCH();
 }
-void launch_cg_alpha(CgState* st, const double* p, int blocks, cudaStream_t s) {
-  k_cg_alpha<<<1, kThreads, 0, s>>>(st, p, blocks);
+int launch_cg_update_xr(CgState* st, const double* pap, int blocks, const float* p, const float* ap,
+                        float* x, float* r, int64_t n, double* partials, const float* dinv,
+                        const float* w_dev, float* z, cudaStream_t s) {
+  k_cg_update_xr<<<reduce_blocks(n), kThreads, 0, s>>>(st, pap, blocks, p, ap, x, r, n, partials,
+                                                       dinv, w_dev, z);
   MGPBD_CHECK_LAUNCH();
+  return reduce_blocks(n);
 }
-void launch_cg_update_xr(const CgState* st, const float* p, const float* ap, float* x, float* r,
-                         int64_t n, double* partials, cudaStream_t s) {
-  k_cg_update_xr<<<reduce_blocks(n), kThreads, 0, s>>>(st, p, ap, x, r, n, partials);
-  MGPBD_CHECK_LAUNCH();
-}
-void launch_cg_check(CgState* st, const double* p, int blocks, cudaStream_t s) {
-  k_cg_check<<<1, kThreads, 0, s>>>(st, p, blocks);
-  MGPBD_CHECK_LAUNCH();
-}
-void launch_cg_beta(CgState* st, const double* p, int blocks, cudaStream_t s) {
-  k_cg_beta<<<1, kThreads, 0, s>>>(st, p, blocks);
+void launch_cg_check(CgState* st, const CgCheck& check, cudaStream_t s) {
+  k_cg_check<<<1, kThreads, 0, s>>>(st, check.partials, check.blocks);
   MGPBD_CHECK_LAUNCH();
 }
 void launch_cg_restart(CgState* st, const double* p, int blocks, int32_t clear_mask,
@@ -1260,8 +1320,10 @@ void launch_cg_restart(CgState* st, const double* p, int blocks, int32_t clear_m
   k_cg_restart<<<1, kThreads, 0, s>>>(st, p, blocks, clear_mask);
   MGPBD_CHECK_LAUNCH();
 }
-void launch_cg_update_p(const CgState* st, const float* z, float* p, int64_t n, cudaStream_t s) {
-  k_cg_update_p<<<grid_for(n, kThreads), kThreads, 0, s>>>(st, z, p, n);
+void launch_cg_update_p(CgState* st, const double* rz, int blocks, const float* z, float* p, int64_t n,
+                        const cudaGraphConditionalHandle* loop, cudaStream_t s) {
+  k_cg_update_p<<<grid_for(n, kThreads), kThreads, 0, s>>>(st, rz, blocks, z, p, n, loop ? *loop : 0,
+                                                           loop != nullptr);
   MGPBD_CHECK_LAUNCH();
 }
 

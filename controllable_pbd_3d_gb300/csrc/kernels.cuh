@@ -110,7 +110,6 @@ int tune_row_shape(const CsrView& a, const float* x, const float* b, float* y, i
 constexpr int64_t kCsrPad = 8;
 // y = A x
 void launch_spmv(const CsrView& a, const float* x, float* y, cudaStream_t s);
-// y = A x and partials of x.y (float64)  -- for CG's p.Ap
 // x_new = x + w * dinv * (b - A x); x == nullptr means x = 0
 void launch_jacobi(const CsrView& a, const float* b, const float* x, float* x_new, float w,
                    cudaStream_t s);
@@ -141,38 +140,45 @@ struct CgState {
 // the fused vector kernels read the device state; all return early once done
 void launch_cg_init(CgState* st, const double* partials_rz, int blocks, double tol_abs,
                     double tol_rel, int maxiter, cudaStream_t s);
-void launch_cg_alpha(CgState* st, const double* partials_pap, int blocks, cudaStream_t s);
-// x += alpha p ; r -= alpha Ap ; partials of r.r
-void launch_cg_update_xr(const CgState* st, const float* p, const float* ap, float* x, float* r,
-                         int64_t n, double* partials, cudaStream_t s);
-void launch_cg_check(CgState* st, const double* partials_rr, int blocks, cudaStream_t s);
-void launch_cg_beta(CgState* st, const double* partials_rz, int blocks, cudaStream_t s);
+// The steps of an iteration.  Those that return a count leave that many
+// partials of a dot product for the step that needs it: x.y of y = A x
+int launch_cg_spmv_dot(CgState* st, const CsrView& a, const float* x, float* y, double* partials,
+                       cudaStream_t s);
+// alpha from p.Ap; x += alpha p ; r -= alpha Ap ; z (if given) = w D^-1 r ; r.r
+int launch_cg_update_xr(CgState* st, const double* pap, int blocks, const float* p, const float* ap,
+                        float* x, float* r, int64_t n, double* partials, const float* dinv,
+                        const float* w_dev, float* z, cudaStream_t s);
+// the stopping test from r.r: given to the row operator that comes next, or
+// made by a kernel of its own
+struct CgCheck {
+  const double* partials = nullptr;
+  int blocks = 0;
+};
+void launch_cg_check(CgState* st, const CgCheck& check, cudaStream_t s);
+// a.b, or b.x_new of a Jacobi sweep
+int launch_cg_dot(CgState* st, const float* a, const float* b, int64_t n, double* partials,
+                  cudaStream_t s);
+int launch_cg_jacobi_dot(CgState* st, const CsrView& a, const float* b, const float* x, float* x_new,
+                         float w, const float* w_dev, double* partials, const CgCheck& check,
+                         cudaStream_t s);
 // restart from the current iterate: rz from partials, drops status bits
 void launch_cg_restart(CgState* st, const double* partials_rz, int blocks, int32_t clear_mask,
                        cudaStream_t s);
-// p = z + beta p
-void launch_cg_update_p(const CgState* st, const float* z, float* p, int64_t n, cudaStream_t s);
+// beta from r.z; p = z + beta p; loop (if given): the condition of the captured
+// loop whose iteration ends here
+void launch_cg_update_p(CgState* st, const double* rz, int blocks, const float* z, float* p, int64_t n,
+                        const cudaGraphConditionalHandle* loop, cudaStream_t s);
 
-// guarded variants of the V-cycle pieces (no-ops once st->done)
-void launch_jacobi_g(const CgState* st, const CsrView& a, const float* b, const float* x,
-                     float* x_new, float w, cudaStream_t s);
-// same with the weight read from device memory (w_dev) when not null
-void launch_jacobi_gw(const CgState* st, const CsrView& a, const float* b, const float* x,
-                      float* x_new, float w, const float* w_dev, cudaStream_t s);
-void launch_residual_g(const CgState* st, const CsrView& a, const float* b, const float* x,
-                       float* r, cudaStream_t s);
+// guarded variants of the V-cycle pieces (no-ops once st->done); w_dev: the
+// weight in device memory when not null
+void launch_jacobi_gw(CgState* st, const CsrView& a, const float* b, const float* x, float* x_new,
+                      float w, const float* w_dev, const CgCheck& check, cudaStream_t s);
+void launch_residual_g(CgState* st, const CsrView& a, const float* b, const float* x, float* r,
+                       const CgCheck& check, cudaStream_t s);
 void launch_restrict_g(const CgState* st, const int32_t* mem_ptr, const int32_t* mem_rows,
                        const float* r, int32_t n_coarse, float* bc, cudaStream_t s);
 void launch_prolong_add_g(const CgState* st, const int32_t* agg, const float* xc, int32_t n,
                           float* x, cudaStream_t s);
-// y = A x and the partials of x.y, one per block of its grid: returns how many
-// (the grid of the other row kernels; on one block per 1024 rows, 32 for
-// 32,000 rows and 3.0e6 nonzeros, it took 55 us more: 263 -> 208 us of a CG
-// iteration)
-int launch_spmv_dot_g(const CgState* st, const CsrView& a, const float* x, float* y,
-                       double* partials, cudaStream_t s);
-void launch_dot_partials_g(const CgState* st, const float* a, const float* b, int64_t n,
-                           double* partials, cudaStream_t s);
 // dense float64 Cholesky solve on the coarsest level: x = L^-T L^-1 b
 void launch_dense_chol_solve(const CgState* st, const double* L, int32_t n, const float* b,
                              float* x, cudaStream_t s);

@@ -1140,14 +1140,25 @@ double Solver::compute_rhs() {
 // Jacobi sweeps on level l (cons/sparse_gpu.py:134-144 + gpu_copy); cur holds
 // the iterate, nxt the scratch, and they swap after each sweep.
 void Solver::smooth_level(int32_t l, const float* b, float*& cur, float*& nxt, int sweeps,
-                          bool from_zero, const CgState* guard) {
+                          bool from_zero, CgState* guard, CgSweeps& c) {
   Level& L = levels_[l];
   CsrView A = L.view();
   for (int it = 0; it < sweeps; ++it) {
+    if (from_zero && it == 0 && c.first) {  // (made already)
+      std::swap(cur, nxt);
+      continue;
+    }
+    if (!from_zero && it == sweeps - 1 && c.last) {
+      c.n_rz = launch_cg_jacobi_dot(guard, A, b, cur, nxt, p_.omega_jacobi, L.omega.p, c.rz,
+                                    std::exchange(c.check, {}), stream_);
+      std::swap(cur, nxt);
+      continue;
+    }
     bool zero = from_zero && it == 0 && p_.mode == MGPBD_MODE_FAST;
     if (from_zero && it == 0 && !zero)
       MGPBD_CUDA(cudaMemsetAsync(cur, 0, sizeof(float) * L.n, stream_));
-    launch_jacobi_gw(guard, A, b, zero ? nullptr : cur, nxt, p_.omega_jacobi, L.omega.p, stream_);
+    launch_jacobi_gw(guard, A, b, zero ? nullptr : cur, nxt, p_.omega_jacobi, L.omega.p,
+                     std::exchange(c.check, {}), stream_);
     std::swap(cur, nxt);
   }
   if (sweeps == 0 && from_zero) MGPBD_CUDA(cudaMemsetAsync(cur, 0, sizeof(float) * L.n, stream_));
@@ -1173,7 +1184,7 @@ void Solver::coarse_sweeps(const float* b, const SweepTransfer& t, const CgState
 
 // GPUMultigridSolver.vcycle (cons/mgpcg_gpu.py:214-259) with a zero initial
 // guess; the result ends in levels_[l].xa.
-void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
+void Solver::vcycle(int32_t l, const float* b, CgState* guard, CgSweeps& c) {
   Level& L = levels_[l];
   float* cur = L.xa.p;
   float* nxt = L.xb.p;
@@ -1186,14 +1197,14 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
       coarse_sweeps(b, SweepTransfer(), guard);
       return;
     }
-    smooth_level(l, b, cur, nxt, n_coarse_sweeps(), true, guard);
+    smooth_level(l, b, cur, nxt, n_coarse_sweeps(), true, guard, c);
   } else {
-    smooth_level(l, b, cur, nxt, p_.n_smooth, true, guard);
+    smooth_level(l, b, cur, nxt, p_.n_smooth, true, guard, c);
     Level& C = levels_[l + 1];
     // with cg_alias the level-0 residual lands in the CG residual vector, as
     // in the reference (cons/mgpcg_gpu.py:239-240 with :275)
     float* res = (l == 0 && p_.cg_alias) ? cg_r_.p : L.r.p;
-    launch_residual_g(guard, L.view(), b, cur, res, stream_);
+    launch_residual_g(guard, L.view(), b, cur, res, std::exchange(c.check, {}), stream_);
     // (a level-0 correction that is judged, learned or recorded is not only
     // the sweeps)
     const bool plain = l > 0 || !(judge_pending_ || net_active_ || rec_count_ < rec_cap_);
@@ -1213,7 +1224,7 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
         vcycle(l + 1, C.b.p, guard);
       launch_prolong_add_g(guard, L.agg.p, C.xa.p, L.n, cur, stream_);
     }
-    smooth_level(l, b, cur, nxt, p_.n_smooth, false, guard);
+    smooth_level(l, b, cur, nxt, p_.n_smooth, false, guard, c);
   }
   if (cur != L.xa.p)
     MGPBD_CUDA(cudaMemcpyAsync(L.xa.p, cur, sizeof(float) * L.n, cudaMemcpyDeviceToDevice, stream_));
@@ -1222,7 +1233,7 @@ void Solver::vcycle(int32_t l, const float* b, const CgState* guard) {
 // The coarse correction of the level-0 V-cycle: the recursion (the
 // reference's), the learned weights, or -- on the first V-cycle of a learned
 // solve -- both, the plain one judging the learned one by coarse energy.
-void Solver::coarse_correction(const CgState* guard) {
+void Solver::coarse_correction(CgState* guard) {
   Level& C = levels_[1];
   cudaStream_t s = stream_;
   if (judge_pending_) {
@@ -1331,7 +1342,7 @@ void Solver::record_coarse(float* rc, float* ec, int32_t capacity, int32_t every
   rec_calls_ = 0;
 }
 
-void Solver::precondition(const CgState* guard) {
+void Solver::precondition(CgState* guard, CgSweeps& c) {
   const float* b0 = cg_r_.p;
   if (p_.cg_alias && n_levels() > 1) {
     // the reference copies r into _b[0] before vcycle(0) (cons/mgpcg_gpu.py:278,311)
@@ -1339,7 +1350,7 @@ void Solver::precondition(const CgState* guard) {
                                cudaMemcpyDeviceToDevice, stream_));
     b0 = levels_[0].b.p;
   }
-  vcycle(0, b0, guard);
+  vcycle(0, b0, guard, c);
 }
 
 void Solver::vcycle_into(const float* r, float* z) {
@@ -1351,20 +1362,27 @@ void Solver::vcycle_into(const float* r, float* z) {
 }
 
 // One CG iteration (cons/mgpcg_gpu.py:289-327) on device scalars.
-void Solver::cg_body(const float* b, float* x) {
-  (void)b;
+// Loop: the condition of the captured loop that this is the body of.
+void Solver::cg_body(float* x, const cudaGraphConditionalHandle* loop) {
   cudaStream_t s = stream_;
   CgState* st = cg_state_.p;
   int64_t n = nt_;
-  int blocks = reduce_blocks(n);
-  const int dot_blocks = launch_spmv_dot_g(st, levels_[0].view(), cg_p_.p, cg_ap_.p, partials_.p, s);
-  launch_cg_alpha(st, partials_.p, dot_blocks, s);
-  launch_cg_update_xr(st, cg_p_.p, cg_ap_.p, x, cg_r_.p, n, partials_.p, s);
-  launch_cg_check(st, partials_.p, blocks, s);
-  precondition(st);
-  launch_dot_partials_g(st, cg_r_.p, levels_[0].xa.p, n, partials_.p, s);
-  launch_cg_beta(st, partials_.p, blocks, s);
-  launch_cg_update_p(st, levels_[0].xa.p, cg_p_.p, n, s);
+  Level& L = levels_[0];
+  double *pap = partials_.p, *rr = pap + kMaxReduceBlocks, *rz = rr + kMaxReduceBlocks;
+  const int n_pap = launch_cg_spmv_dot(st, L.view(), cg_p_.p, cg_ap_.p, pap, s);
+  // the V-cycle's first sweep (from zero) and last one take part in the
+  // vector update before it and the dot product after it
+  CgSweeps c;
+  c.first = n_levels() > 1 && p_.n_smooth > 0 && p_.mode == MGPBD_MODE_FAST && !p_.cg_alias;
+  c.last = n_levels() > 1 && p_.n_smooth > 0 && !p_.cg_alias;
+  c.check.partials = rr;
+  c.check.blocks = launch_cg_update_xr(st, pap, n_pap, cg_p_.p, cg_ap_.p, x, cg_r_.p, n, rr,
+                                       L.diag_inv.p, L.omega.p, c.first ? L.xb.p : nullptr, s);
+  if (n_levels() == 1) launch_cg_check(st, std::exchange(c.check, {}), s);
+  c.rz = rz;
+  precondition(st, c);
+  const int n_rz = c.last ? c.n_rz : launch_cg_dot(st, cg_r_.p, L.xa.p, n, rz, s);
+  launch_cg_update_p(st, rz, n_rz, L.xa.p, cg_p_.p, n, loop, s);
 }
 
 // PCG with the learned coarse correction (MGPBD_PRECOND_LEARNED): the
@@ -1404,7 +1422,7 @@ int32_t Solver::pcg_learned(const float* b, float* x) {
   int32_t best_at = 0;
   const uint32_t broken = MGPBD_STATUS_NAN | MGPBD_STATUS_PAP_NONPOS;
   for (int32_t k = 0; k < p_.maxiter_cg; ++k) {
-    cg_body(b, x);
+    cg_body(x);
     sync_read(h_state_, cg_state_.p, sizeof(CgState));
     const bool bad = net_active_ && (static_cast<uint32_t>(h_state_->status) & broken);
     if (h_state_->done && !bad) break;
@@ -1459,7 +1477,7 @@ int32_t Solver::pcg(const float* b, float* x) {
   launch_dot_partials(b, b, n, partials_.p + blocks, s);
   launch_cg_init(cg_state_.p, partials_.p, blocks, p_.tol_cg, p_.rel_tol_cg, p_.maxiter_cg, s);
   for (int32_t k = 0; k < p_.maxiter_cg; ++k) {
-    cg_body(b, x);
+    cg_body(x);
     sync_read(h_state_, cg_state_.p, sizeof(CgState));
     if (h_state_->done) break;
   }
@@ -1512,9 +1530,7 @@ int32_t Solver::pcg_graph(const float* b, float* x) {
       MGPBD_CUDA(cudaStreamUpdateCaptureDependencies(cs, &cond, nullptr, 1, cudaStreamSetCaptureDependencies));
       MGPBD_CUDA(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
       stream_ = bs;
-      cg_body(b, x);
-      k_set_cond<<<1, 1, 0, bs>>>(handle, cg_state_.p);
-      MGPBD_CHECK_LAUNCH();
+      cg_body(x, &handle);
       long long c2 = g_launches.load();
       // captured launches run later, when the graph does
       g_launches.fetch_sub(c2 - c0);

@@ -52,6 +52,15 @@ struct Level {
   }
 };
 
+// What the V-cycle around whose level 0 a CG iteration runs makes for it
+struct CgSweeps {
+  bool first = false;  // the first sweep from zero is made already, in xb
+  bool last = false;   // the last sweep also leaves n_rz partials of r.z in rz
+  double* rz = nullptr;
+  int n_rz = 0;
+  CgCheck check;       // the stopping test, for the first row operator
+};
+
 class Solver {
  public:
   explicit Solver(const mgpbd_params& p);
@@ -166,21 +175,29 @@ class Solver {
   int n_coarse_sweeps() const;
   bool fused_sweeps() const;
   void coarse_sweeps(const float* b, const SweepTransfer& t, const CgState* guard);
-  void vcycle(int32_t l, const float* b, const CgState* guard);
+  void vcycle(int32_t l, const float* b, CgState* guard, CgSweeps& c);
+  void vcycle(int32_t l, const float* b, CgState* guard) {
+    CgSweeps none;
+    vcycle(l, b, guard, none);
+  }
   void smooth_level(int32_t l, const float* b, float*& cur, float*& nxt, int sweeps,
-                    bool from_zero, const CgState* guard);
+                    bool from_zero, CgState* guard, CgSweeps& c);
   void update_smoother_weights();
   void factor_coarsest();
-  void cg_body(const float* b, float* x);
+  void cg_body(float* x, const cudaGraphConditionalHandle* loop = nullptr);
   // z = V-cycle(r) for the CG residual r (level-0 result left in xa)
-  void precondition(const CgState* guard);
+  void precondition(CgState* guard, CgSweeps& c);
+  void precondition(CgState* guard) {
+    CgSweeps none;
+    precondition(guard, none);
+  }
   int32_t pcg_graph(const float* b, float* x);
   // PCG with the learned coarse correction, judged and backed up by the
   // plain V-cycle
   bool learned() const { return p_.precond == MGPBD_PRECOND_LEARNED; }
   int32_t pcg_learned(const float* b, float* x);
   // coarse correction of the level-0 V-cycle into levels_[1].xa
-  void coarse_correction(const CgState* guard);
+  void coarse_correction(CgState* guard);
   NetGraph net_graph() const;
   // 1/2 e^T A_1 e - e^T r on level 1 (host sync)
   double coarse_energy(const float* e, const float* r);

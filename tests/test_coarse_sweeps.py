@@ -91,3 +91,56 @@ def test_two_levels(cuda, n, nc, per_row):
   ref = s(A, b64, x, 2)
   got = m.vcycle_apply(cuda.tensor(b, device='cuda')).cpu().numpy()
   assert np.abs(got - ref).max() <= s.err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('mode', ['fast', 'parity'])
+@pytest.mark.parametrize('n_smooth', [0, 1, 2, 3])
+@pytest.mark.parametrize('kw', [{}, {'smoother': 'safe'}, {'use_graph': False}, {'cg_alias': True}])
+def test_iterations_of_the_cg_around(cuda, mode, n_smooth, kw):
+  """The CG iteration shares its vector update and dot product with the
+  V-cycle's first and last sweep: the same iterates as a float64 CG around the
+  library's own V-cycle, to the accuracy float32 vectors leave it."""
+  if kw.get('cg_alias') and n_smooth == 0:
+    pytest.skip('no smoothing and an overwritten residual do not converge')
+  from controllable_pbd_3d_gb300 import MGPBDSolverGPU, meshgen
+  xr, t = meshgen.hex_grid_tets(4, 5, 3)
+  x0, _ = meshgen.hex_grid_tets(4, 5, 3, jitter=0.02, seed=3)
+  invm = np.ones(len(xr), np.float32)
+  s = MGPBDSolverGPU(cuda.tensor(x0, device='cuda'), cuda.tensor(xr, device='cuda'),
+                     cuda.tensor(invm, device='cuda'), cuda.tensor(t, device='cuda'), None,
+                     [0.0, -9.8, 0.0], 1.0 / 300, mu=1e5, mode=mode, n_smooth=n_smooth,
+                     maxiter_cg=6, tol_cg=1e-30, **kw)
+  s.init()
+  s._compute_C_and_gradC()
+  s._compute_rhs_gpu()
+  s._fill_A_and_update_gpu()
+  gm = s._gpu_solver
+  its = gm.solve(s._b_gpu, s._dlam_gpu)
+  assert 1 <= its <= 6
+  if kw.get('cg_alias'):
+    assert bool(cuda.isfinite(s._dlam_gpu).all())
+    return
+  L0 = gm._gpu_As[0]
+  nt = s.n_tets
+  A = sp.csr_matrix((L0.data.cpu().numpy()[:L0.nnz], L0.indices.cpu().numpy()[:L0.nnz],
+                     L0.indptr.cpu().numpy()), shape=(nt, nt)).astype(np.float64)
+  b = s._b_gpu.cpu().numpy().astype(np.float64)
+
+  def m(r):
+    return gm.vcycle_apply(cuda.tensor(r.astype(np.float32), device='cuda')).cpu().numpy().astype(np.float64)
+
+  x, r = np.zeros(nt), b.copy()
+  z = m(r)
+  p, rz = z, r @ z
+  for _ in range(its):
+    q = A @ p
+    a = rz / (p @ q)
+    x, r = x + a * p, r - a * q
+    z = m(r)
+    rz, old = r @ z, rz
+    p = z + rz / old * p
+  # a few roundings of every vector an iteration, grown by CG's own
+  # sensitivity: the square root of the condition number of M A, < 1e3 here
+  got = s._dlam_gpu.cpu().numpy()
+  assert np.abs(got - x).max() <= 1e3 * 8 * its * EPS * np.abs(x).max()
