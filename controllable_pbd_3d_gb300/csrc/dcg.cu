@@ -119,29 +119,6 @@ __device__ __forceinline__ void bar_sync1() {
   asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory");
 }
 
-// 16 bytes written and read in one access, data and generation tag together:
-// a reader that finds the tag it waits for has the data too, so the blocks of
-// a grid need neither fences nor a counter
-__device__ __forceinline__ void put_tagged(void* p, uint32_t x, uint32_t y, uint32_t z, uint32_t tag) {
-  asm volatile(
-      "{\n\t.reg .b128 v;\n\t.reg .b64 a, b;\n\t"
-      "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b128 v, {a, b};\n\t"
-      "st.relaxed.gpu.global.b128 [%0], v;\n\t}"
-      ::"l"(p), "r"(x), "r"(y), "r"(z), "r"(tag)
-      : "memory");
-}
-__device__ __forceinline__ uint4 get_tagged(const void* p) {
-  uint4 v;
-  asm volatile(
-      "{\n\t.reg .b128 v;\n\t.reg .b64 a, b;\n\t"
-      "ld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {a, b}, v;\n\t"
-      "mov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
-      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-      : "l"(p)
-      : "memory");
-  return v;
-}
-
 // Tensor memory as a second register file: a thread's lane and the columns
 // of its warp's window hold what it needs of its constraints.  Every access
 // is by the whole warp, converged, with one column address.

@@ -26,6 +26,7 @@ namespace mgpbd {
 namespace {
 
 constexpr int kLT = 256;  // threads per block
+constexpr int kFlowWarps = 8;  // most of a block of the colour kernels that wait for vertices
 constexpr int kVL = 4;    // lanes per vertex in the VBD colour kernel
 constexpr unsigned long long kSpinNs = 4000000000ull;  // grid barrier limit
 
@@ -127,27 +128,27 @@ struct XArgs {
   float dt, ha, da;
 };
 
-// ATOMIC: positions read through L2 and updated with atomic adds (the
-// parallel default method); otherwise plain read-modify-write in the
-// reference's order (all hydrostatic updates, then all deviatoric ones)
-template <bool ATOMIC>
-__device__ __forceinline__ void xpbd_tet(const XArgs& a, int64_t k) {
-  const int4 q = a.t_i[k];
-  const int64_t vid[4] = {q.x, q.y, q.z, q.w};
+// The update of the tet t: t.x(l, c) is coordinate c of its vertex l, t.B(m)
+// entry m of its rest matrix.  (The values come through memory in each kernel
+// that makes it: the compiler then orders, and rounds, them alike.)  ATOMIC: positions updated with atomic adds (the parallel
+// default method); otherwise plain read-modify-write in the reference's order
+// (all hydrostatic updates, then all deviatoric ones).
+template <bool ATOMIC, class T>
+__device__ __forceinline__ void xpbd_update(const XArgs& a, const T& t) {
   float p[4][3], w[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) p[l][c] = ATOMIC ? __ldcg(a.x + 3 * vid[l] + c) : a.x[3 * vid[l] + c];
-    w[l] = a.invm[vid[l]];
+    for (int c = 0; c < 3; ++c) p[l][c] = ATOMIC ? __ldcg(&t.x(l, c)) : t.x(l, c);
+    w[l] = t.w(l);
   }
-  float B[3][3];
+  float Bm[3][3];
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) B[r][c] = a.B[9 * k + 3 * r + c];
+    for (int c = 0; c < 3; ++c) Bm[r][c] = t.B(3 * r + c);
   float f[3][3];
-  deformation(p, B, f);
+  deformation(p, Bm, f);
 
   const float CH = det_cols(f) - 1.0f;
   float cof[3][3];  // columns f2 x f3, f3 x f1, f1 x f2
@@ -159,9 +160,9 @@ __device__ __forceinline__ void xpbd_tet(const XArgs& a, int64_t k) {
   for (int j = 0; j < 3; ++j)
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      gH[j][i] = cof[0][i] * B[j][0] + cof[1][i] * B[j][1] + cof[2][i] * B[j][2];
-      gD[j][i] = (2.0f * f[0][i]) * B[j][0] + (2.0f * f[1][i]) * B[j][1] +
-                 (2.0f * f[2][i]) * B[j][2];
+      gH[j][i] = cof[0][i] * Bm[j][0] + cof[1][i] * Bm[j][1] + cof[2][i] * Bm[j][2];
+      gD[j][i] = (2.0f * f[0][i]) * Bm[j][0] + (2.0f * f[1][i]) * Bm[j][1] +
+                 (2.0f * f[2][i]) * Bm[j][2];
     }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -169,7 +170,7 @@ __device__ __forceinline__ void xpbd_tet(const XArgs& a, int64_t k) {
     gD[3][i] = -gD[0][i] - gD[1][i] - gD[2][i];
   }
   const float SH = w[0] * nsq3(gH[0]) + w[1] * nsq3(gH[1]) + w[2] * nsq3(gH[2]) + w[3] * nsq3(gH[3]);
-  const float tm = a.t_m[k];
+  const float tm = t.tm();
   const float aH = a.ha / (a.dt * a.dt * tm);
   float FF = 0.0f;
 #pragma unroll
@@ -181,7 +182,7 @@ __device__ __forceinline__ void xpbd_tet(const XArgs& a, int64_t k) {
   const float aD = a.da / (a.dt * a.dt * tm);
   const float SDH = w[0] * dot3(gD[0], gH[0]) + w[1] * dot3(gD[1], gH[1]) +
                     w[2] * dot3(gD[2], gH[2]) + w[3] * dot3(gD[3], gH[3]);
-  const float lH = a.lh[k], lD = a.ld[k];
+  const float lH = t.lh(), lD = t.ld();
   const float dH = (SDH * (CD + aD * lD) - (CH + aH * lH) * (aD + SD)) /
                    ((aH + SH) * (aD + SD) - SDH * SDH);
   const float dD = -(CD + aD * lD + SDH * dH) / (aD + SD);
@@ -190,35 +191,195 @@ __device__ __forceinline__ void xpbd_tet(const XArgs& a, int64_t k) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float u = w[l] * gH[l][c] * dH;
-      if (ATOMIC) atomicAdd(a.x + 3 * vid[l] + c, u);
-      else a.x[3 * vid[l] + c] = a.x[3 * vid[l] + c] + u;
+      if (ATOMIC) atomicAdd(&t.x(l, c), u);
+      else t.x(l, c) = t.x(l, c) + u;
     }
-  a.lh[k] = lH + dH;
+  t.lh() = lH + dH;
 #pragma unroll
   for (int l = 0; l < 4; ++l)
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float u = w[l] * gD[l][c] * dD;
-      if (ATOMIC) atomicAdd(a.x + 3 * vid[l] + c, u);
-      else a.x[3 * vid[l] + c] = a.x[3 * vid[l] + c] + u;
+      if (ATOMIC) atomicAdd(&t.x(l, c), u);
+      else t.x(l, c) = t.x(l, c) + u;
     }
-  a.ld[k] = lD + dD;
+  t.ld() = lD + dD;
 }
+
+// a tet in global memory
+struct XTet {
+  const XArgs& a;
+  int64_t k, vid[4];
+  __device__ XTet(const XArgs& args, int64_t tet) : a(args), k(tet) {
+    const int4 q = a.t_i[k];
+    vid[0] = q.x;
+    vid[1] = q.y;
+    vid[2] = q.z;
+    vid[3] = q.w;
+  }
+  __device__ float& x(int l, int c) const { return a.x[3 * vid[l] + c]; }
+  __device__ float w(int l) const { return a.invm[vid[l]]; }
+  __device__ float B(int m) const { return a.B[9 * k + m]; }
+  __device__ float tm() const { return a.t_m[k]; }
+  __device__ float& lh() const { return a.lh[k]; }
+  __device__ float& ld() const { return a.ld[k]; }
+};
 
 // solve_cons (cons/deform3d.py:55-127): every tet at once
 __global__ void __launch_bounds__(kLT) k_xpbd_all(XArgs a) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.nt;
        k += (int64_t)gridDim.x * blockDim.x)
-    xpbd_tet<true>(a, k);
+    xpbd_update<true>(a, XTet(a, k));
 }
 
 // solve_cons_gauss_seidel (:128-200): one tet at a time, in index order
 __global__ void k_xpbd_serial(XArgs a, int32_t passes) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   for (int32_t s = 0; s < passes; ++s)
-    for (int64_t k = 0; k < a.nt; ++k) xpbd_tet<false>(a, k);
+    for (int64_t k = 0; k < a.nt; ++k) xpbd_update<false>(a, XTet(a, k));
 }
 
+// The tets of one colour share no vertex, so a colour's order does not matter
+// but each vertex's does: it is updated by its tets in the order of their
+// colours.  Each vertex carries, beside its position and in the same 16 bytes,
+// the number of updates it has had; a tet waits until its four vertices have
+// had those before it, which it knows from the mesh, and no more.  That chain
+// through L2 is the bound: 2.1 us a colour (24^3 hexes, 38 colours; 10 passes
+// 814 us).  With a grid barrier between the colours, behind which four
+// dependent loads began, and a colour's tets on the first few blocks, it was
+// 8 us (3,230).
+struct FlowArgs {
+  const int4* vid;   // vertices of each tet in chunk order (x < 0: padding)
+  const int4* rank;  // updates of each vertex before this tet's, in a pass
+  const int4* deg;   // and in a whole pass
+  const int32_t* tet;
+  const float* B;    // [9][32 n_chunks]
+  float4* xt;        // position and count of updates of each vertex
+  int32_t n_chunks;  // 32 tets of one colour each
+  int32_t passes;
+  GridSync* gs;
+  int32_t* status;
+};
+
+// Waits until each of K vertices has had the update it is wanted with (all are
+// polled at once: one after the other, each would add its own round trip);
+// false once a wait of the grid gave up
+template <int K>
+__device__ __forceinline__ bool wait_vertices(const float4* const (&p)[K], const uint32_t (&want)[K],
+                                              uint4 (&v)[K], GridSync* gs, int32_t* status) {
+#pragma unroll
+  for (int l = 0; l < K; ++l) v[l] = pdev::get_tagged(p[l]);
+  unsigned long long t0 = 0;
+  for (uint32_t n = 1;; ++n) {
+    bool ready = true;
+#pragma unroll
+    for (int l = 0; l < K; ++l) ready = ready && v[l].w == want[l];
+    if (ready) return true;
+#pragma unroll
+    for (int l = 0; l < K; ++l)
+      if (v[l].w != want[l]) v[l] = pdev::get_tagged(p[l]);
+    if ((n & 1023u) == 0) {
+      if (pdev::ld_relaxed(&gs->err) != 0u) return false;
+      const unsigned long long t = pdev::global_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kSpinNs) {
+        atomicExch(&gs->err, 1u);
+        atomicOr(reinterpret_cast<unsigned int*>(status), MGPBD_STATUS_SYNC_TIMEOUT);
+        return false;
+      }
+    }
+  }
+}
+
+// B in chunk order, one row of the arrays an entry
+__global__ void k_flow_rest(const float* __restrict__ B, const int32_t* __restrict__ tet, int64_t n,
+                            float* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    for (int m = 0; m < 9; ++m) out[m * n + i] = tet[i] >= 0 ? B[9LL * tet[i] + m] : 0.0f;
+}
+
+__global__ void k_flow_start(const float* __restrict__ x, float4* __restrict__ xt, int32_t nv) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nv;
+       v += (int64_t)gridDim.x * blockDim.x)
+    xt[v] = make_float4(x[3 * v], x[3 * v + 1], x[3 * v + 2], __uint_as_float(0u));
+}
+
+// a thread's tet in shared memory: positions, B, inverse masses, volume,
+// multipliers
+struct XFlowTet {
+  float* s;  // the lane's column of its warp's 32
+  __device__ float& at(int m) const { return s[32 * m]; }
+  __device__ float& x(int l, int c) const { return at(3 * l + c); }
+  __device__ float B(int m) const { return at(12 + m); }
+  __device__ float w(int l) const { return at(21 + l); }
+  __device__ float tm() const { return at(25); }
+  __device__ float& lh() const { return at(26); }
+  __device__ float& ld() const { return at(27); }
+};
+
+// solve_cons_graph_coloring / solve_range (:210-288).  A warp takes its chunks
+// in the order of the passes and colours, every wait is for an earlier chunk,
+// and all warps are resident: the waits end.
+__global__ void __launch_bounds__(32 * kFlowWarps) k_xpbd_flow(XArgs a, FlowArgs c) {
+  extern __shared__ float sm[];
+  const int lane = threadIdx.x & 31;
+  const int warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);  // neighbours on other SMs
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  const int64_t n = 32LL * c.n_chunks;
+  for (int32_t s = 0; s < c.passes; ++s)
+    for (int32_t j = warp; j < c.n_chunks; j += warps) {
+      const int64_t i = 32LL * j + lane;
+      const int4 q = __ldg(c.vid + i);
+      bool ok = true;
+      if (q.x >= 0) {
+        const int64_t vid[4] = {q.x, q.y, q.z, q.w};
+        const int4 rk = __ldg(c.rank + i), dg = __ldg(c.deg + i);
+        const uint32_t deg[4] = {(uint32_t)dg.x, (uint32_t)dg.y, (uint32_t)dg.z, (uint32_t)dg.w};
+        uint32_t ver[4] = {(uint32_t)rk.x, (uint32_t)rk.y, (uint32_t)rk.z, (uint32_t)rk.w};
+        const float4* const at[4] = {c.xt + vid[0], c.xt + vid[1], c.xt + vid[2], c.xt + vid[3]};
+        const int64_t k = __ldg(c.tet + i);
+        // all that does not wait
+        const XFlowTet t = {sm + 28 * 32 * (threadIdx.x >> 5) + lane};
+#pragma unroll
+        for (int m = 0; m < 9; ++m) t.at(12 + m) = __ldg(c.B + m * n + i);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) t.at(21 + l) = __ldg(a.invm + vid[l]);
+        t.at(25) = __ldg(a.t_m + k);
+        t.lh() = a.lh[k];
+        t.ld() = a.ld[k];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) ver[l] += (uint32_t)s * deg[l];
+        uint4 v[4];
+        ok = wait_vertices(at, ver, v, c.gs, c.status);
+        if (ok) {
+#pragma unroll
+          for (int l = 0; l < 4; ++l) {
+            t.x(l, 0) = __uint_as_float(v[l].x);
+            t.x(l, 1) = __uint_as_float(v[l].y);
+            t.x(l, 2) = __uint_as_float(v[l].z);
+          }
+          xpbd_update<false>(a, t);
+          a.lh[k] = t.lh();
+          a.ld[k] = t.ld();
+#pragma unroll
+          for (int l = 0; l < 4; ++l) {
+            const float y[3] = {t.x(l, 0), t.x(l, 1), t.x(l, 2)};
+            pdev::put_tagged(const_cast<float4*>(at[l]), __float_as_uint(y[0]), __float_as_uint(y[1]),
+                             __float_as_uint(y[2]), ver[l] + 1);
+            if (ver[l] + 1 == (uint32_t)c.passes * deg[l]) {
+#pragma unroll
+              for (int d = 0; d < 3; ++d) a.x[3 * vid[l] + d] = y[d];
+            }
+          }
+        }
+      }
+      if (!__all_sync(0xffffffffu, ok)) return;
+    }
+}
+
+// The order with a grid barrier between the colours, for meshes in which a tet
+// lists a vertex twice (its update is then two)
 struct ColorArgs {
   const int32_t* order;
   const int32_t* off;
@@ -228,8 +389,6 @@ struct ColorArgs {
   int32_t* status;
 };
 
-// solve_cons_graph_coloring / solve_range (:210-288): the tets of one colour
-// share no vertex; a grid barrier separates the colours
 __global__ void __launch_bounds__(kLT) k_xpbd_color(XArgs a, ColorArgs c) {
   unsigned long long gen = 0;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -237,7 +396,7 @@ __global__ void __launch_bounds__(kLT) k_xpbd_color(XArgs a, ColorArgs c) {
   for (int32_t s = 0; s < c.passes; ++s)
     for (int32_t col = 0; col < c.n_colors; ++col) {
       const int32_t b = c.off[col], e = c.off[col + 1];
-      for (int64_t i = b + tid; i < e; i += stride) xpbd_tet<false>(a, c.order[i]);
+      for (int64_t i = b + tid; i < e; i += stride) xpbd_update<false>(a, XTet(a, c.order[i]));
       const bool last = s == c.passes - 1 && col == c.n_colors - 1;
       if (!last && !pdev::grid_sync(c.gs, c.status, kSpinNs, gen)) return;
     }
@@ -482,13 +641,32 @@ int blocks_for(int64_t n) {
 
 // one block per SM (cooperative launches; fewer blocks keep the barrier
 // cheap, and a colour rarely has more elements than 152 x 256 threads)
-int coop_grid(const void* fn) {
+int coop_grid(const void* fn, int threads) {
   int dev = 0, sms = 0, occ = 0;
   MGPBD_CUDA(cudaGetDevice(&dev));
   MGPBD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kLT, 0));
+  MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, 0));
   require(occ >= 1, MGPBD_ECUDA, "local solver kernel cannot be resident");
   return sms;
+}
+
+constexpr int kFlowSmem = 28 * sizeof(float);  // bytes a thread (XFlowTet)
+
+// Warps of a colour kernel that waits for vertices: the chunks of a colour and
+// a quarter more, which have loaded what does not wait when their turn comes;
+// others only poll, in the way of those that can go on (10 passes over 24^3
+// hexes, 57 chunks a colour: 76 warps 814 us, 304 warps 916; 32^3, 137 chunks:
+// 76 warps 1232 us, 152 886, 304 942).
+void flow_shape(const void* fn, int smem, int64_t chunks, int32_t colors, int* grid, int* threads) {
+  int dev = 0, sms = 0, occ = 0;
+  MGPBD_CUDA(cudaGetDevice(&dev));
+  MGPBD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t warps = std::max<int64_t>(16, 5 * chunks / (4 * std::max(colors, 1)));
+  const int per = static_cast<int>(std::min<int64_t>(kFlowWarps, ceil_div(warps, sms)));
+  *grid = static_cast<int>(std::min<int64_t>(sms, ceil_div(warps, per)));
+  *threads = 32 * per;
+  MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, *threads, smem * *threads));
+  require(occ >= 1, MGPBD_ECUDA, "local solver kernel cannot be resident");
 }
 
 // host copy of t_i with ids validated
@@ -497,6 +675,16 @@ std::vector<int32_t> host_tets(const int32_t* t_i, int32_t nt, int32_t nv) {
   MGPBD_CUDA(cudaMemcpy(h.data(), t_i, sizeof(int32_t) * h.size(), cudaMemcpyDeviceToHost));
   for (int32_t v : h) require(v >= 0 && v < nv, MGPBD_EINVAL, "tet vertex id out of range");
   return h;
+}
+
+// whether no tet lists a vertex twice
+bool distinct_vertices(const std::vector<int32_t>& ht) {
+  for (size_t k = 0; k < ht.size(); k += 4) {
+    const int32_t *q = &ht[k];
+    if (q[0] == q[1] || q[0] == q[2] || q[0] == q[3] || q[1] == q[2] || q[1] == q[3] || q[2] == q[3])
+      return false;
+  }
+  return true;
 }
 
 void upload(DevBuf<int32_t>& d, const std::vector<int32_t>& h, cudaStream_t s) {
@@ -576,12 +764,48 @@ void Xpbd::set_mesh(float* x, const float* x_ref, const float* invm, const int32
   if (p_.method == MGPBD_XPBD_GRAPH_COLORING) {
     const Coloring col = color_elements(ht.data(), nt, 4, nv);
     n_colors_ = col.n_colors;
-    upload(order_, col.ordered, s);
-    upload(offsets_, col.offsets, s);
     gs_.alloc(1);
-    grid_ = coop_grid(reinterpret_cast<const void*>(k_xpbd_color));
+    n_chunks_ = 0;
+    if (distinct_vertices(ht)) {
+      build_flow(col, ht);
+      flow_shape(reinterpret_cast<const void*>(k_xpbd_flow), kFlowSmem, n_chunks_, n_colors_, &grid_, &threads_);
+    } else {
+      upload(order_, col.ordered, s);
+      upload(offsets_, col.offsets, s);
+      grid_ = coop_grid(reinterpret_cast<const void*>(k_xpbd_color), kLT);
+    }
   }
   MGPBD_CUDA(cudaStreamSynchronize(s));
+}
+
+// The tets in chunks of 32 of one colour, and each vertex's order of updates
+void Xpbd::build_flow(const Coloring& col, const std::vector<int32_t>& ht) {
+  std::vector<int32_t> deg(nv_, 0), tet;
+  for (int32_t c = 0; c < col.n_colors; ++c) {
+    for (int32_t i = col.offsets[c]; i < col.offsets[c + 1]; ++i) tet.push_back(col.ordered[i]);
+    while (tet.size() % 32) tet.push_back(-1);
+  }
+  const size_t n = tet.size();
+  std::vector<int32_t> vid(4 * n, -1), rank(4 * n, 0), total(4 * n, 0);
+  for (size_t i = 0; i < n; ++i)
+    for (int l = 0; l < 4 && tet[i] >= 0; ++l) {
+      const int32_t v = ht[4 * static_cast<size_t>(tet[i]) + l];
+      vid[4 * i + l] = v;
+      rank[4 * i + l] = deg[v]++;
+    }
+  for (size_t i = 0; i < 4 * n; ++i)
+    if (vid[i] >= 0) total[i] = deg[vid[i]];
+  cudaStream_t s = stream_;
+  upload(f_vid_, vid, s);
+  upload(f_rank_, rank, s);
+  upload(f_deg_, total, s);
+  upload(order_, tet, s);
+  f_B_.alloc(9 * static_cast<int64_t>(n));
+  xt_.alloc(nv_);
+  k_flow_rest<<<blocks_for(static_cast<int64_t>(n)), kLT, 0, s>>>(B_.p, order_.p, static_cast<int64_t>(n),
+                                                                  f_B_.p);
+  MGPBD_CHECK_LAUNCH();
+  n_chunks_ = static_cast<int32_t>(n / 32);
 }
 
 void Xpbd::preupdate() {
@@ -620,17 +844,36 @@ void Xpbd::update(int32_t passes) {
     MGPBD_CHECK_LAUNCH();
     return;
   }
-  ColorArgs c;
-  c.order = order_.p;
-  c.off = offsets_.p;
-  c.n_colors = n_colors_;
-  c.passes = passes;
-  c.gs = gs_.p;
-  c.status = status_.p;
   MGPBD_CUDA(cudaMemsetAsync(gs_.p, 0, sizeof(GridSync), s));
-  void* args[] = {&a, &c};
-  MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_xpbd_color), dim3(grid_),
-                                         dim3(kLT), args, 0, s));
+  if (n_chunks_ > 0) {
+    FlowArgs f;
+    f.vid = reinterpret_cast<const int4*>(f_vid_.p);
+    f.rank = reinterpret_cast<const int4*>(f_rank_.p);
+    f.deg = reinterpret_cast<const int4*>(f_deg_.p);
+    f.tet = order_.p;
+    f.B = f_B_.p;
+    f.xt = xt_.p;
+    f.n_chunks = n_chunks_;
+    f.passes = passes;
+    f.gs = gs_.p;
+    f.status = status_.p;
+    k_flow_start<<<blocks_for(nv_), kLT, 0, s>>>(x_, xt_.p, nv_);
+    MGPBD_CHECK_LAUNCH();
+    void* args[] = {&a, &f};
+    MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_xpbd_flow), dim3(grid_),
+                                           dim3(threads_), args, kFlowSmem * threads_, s));
+  } else {
+    ColorArgs c;
+    c.order = order_.p;
+    c.off = offsets_.p;
+    c.n_colors = n_colors_;
+    c.passes = passes;
+    c.gs = gs_.p;
+    c.status = status_.p;
+    void* args[] = {&a, &c};
+    MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_xpbd_color), dim3(grid_),
+                                           dim3(kLT), args, 0, s));
+  }
   MGPBD_CHECK_LAUNCH();
   lazy_.record(status_.p, s);
 }
@@ -706,7 +949,7 @@ void Vbd::set_mesh(float* x, const float* x_ref, const float* invm, const int32_
     upload(order_, col.ordered, s);
     upload(offsets_, col.offsets, s);
     gs_.alloc(1);
-    grid_ = coop_grid(reinterpret_cast<const void*>(k_vbd_color));
+    grid_ = coop_grid(reinterpret_cast<const void*>(k_vbd_color), kLT);
   }
   MGPBD_CUDA(cudaStreamSynchronize(s));
 }

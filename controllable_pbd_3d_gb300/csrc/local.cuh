@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/mgpbd_local.h"
+#include "coloring.h"
 #include "common.h"
 #include "jform.cuh"
 
@@ -57,8 +58,12 @@ class Xpbd {
   const float* t_m_ = nullptr;
   const int32_t* t_i_ = nullptr;
   int32_t nv_ = 0, nt_ = 0;
-  DevBuf<float> B_, lam_h_, lam_d_;
-  DevBuf<int32_t> order_, offsets_, status_;
+  void build_flow(const Coloring& col, const std::vector<int32_t>& ht);
+  DevBuf<float> B_, lam_h_, lam_d_, f_B_;
+  DevBuf<float4> xt_;
+  DevBuf<int32_t> order_, offsets_, status_, f_vid_, f_rank_, f_deg_;
+  int32_t n_chunks_ = 0;
+  int threads_ = 0;
   DevBuf<GridSync> gs_;
   int32_t n_colors_ = 0;
   int grid_ = 0;
