@@ -26,8 +26,13 @@ namespace mgpbd {
 namespace {
 
 constexpr int kLT = 256;  // threads per block
-constexpr int kFlowWarps = 8;  // most of a block of the colour kernels that wait for vertices
-constexpr int kVL = 4;    // lanes per vertex in the VBD colour kernel
+// most warps of a block of the colour kernels that wait for vertices
+constexpr int kXpbdWarps = 8;
+constexpr int kVbdWarps = 16;  // (8: 313 us over 32^3 hexes, 16: 232)
+// lanes per vertex in the VBD colour kernels: at most three tets in a row of the
+// 24 (with four lanes 10 iterations over 24^3 hexes take 244 us, with eight 196,
+// with sixteen 207, and 302, 313, 463 over 32^3)
+constexpr int kVL = 8;
 constexpr unsigned long long kSpinNs = 4000000000ull;  // grid barrier limit
 
 // 3x3 helpers (row-major m[r][c]); determinant by the first column's
@@ -264,11 +269,15 @@ struct FlowArgs {
 // Waits until each of K vertices has had the update it is wanted with (all are
 // polled at once: one after the other, each would add its own round trip);
 // false once a wait of the grid gave up
+// (a null vertex is one that is not waited for)
 template <int K>
 __device__ __forceinline__ bool wait_vertices(const float4* const (&p)[K], const uint32_t (&want)[K],
                                               uint4 (&v)[K], GridSync* gs, int32_t* status) {
 #pragma unroll
-  for (int l = 0; l < K; ++l) v[l] = pdev::get_tagged(p[l]);
+  for (int l = 0; l < K; ++l) {
+    v[l].w = want[l];
+    if (p[l]) v[l] = pdev::get_tagged(p[l]);
+  }
   unsigned long long t0 = 0;
   for (uint32_t n = 1;; ++n) {
     bool ready = true;
@@ -321,7 +330,7 @@ struct XFlowTet {
 // solve_cons_graph_coloring / solve_range (:210-288).  A warp takes its chunks
 // in the order of the passes and colours, every wait is for an earlier chunk,
 // and all warps are resident: the waits end.
-__global__ void __launch_bounds__(32 * kFlowWarps) k_xpbd_flow(XArgs a, FlowArgs c) {
+__global__ void __launch_bounds__(32 * kXpbdWarps) k_xpbd_flow(XArgs a, FlowArgs c) {
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);  // neighbours on other SMs
@@ -423,22 +432,10 @@ struct VArgs {
 };
 
 // force and Gauss-Newton Hessian (upper triangle 00 11 22 01 02 12) of one
-// incident tet, added to f / H
-__device__ __forceinline__ void vbd_entry(const VArgs& a, int32_t ent, float fo[3], float H[6]) {
-  const int64_t tet = ent >> 2;
-  const int l = ent & 3;
-  const int4 q = a.t_i[tet];
-  const int64_t vid[4] = {q.x, q.y, q.z, q.w};
-  float p[4][3];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) p[k][c] = a.x[3 * vid[k] + c];
-  float B[3][3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) B[r][c] = a.dm[9 * tet + 3 * r + c];
+// incident tet (its positions, rest matrix and volume; l: the vertex's place in
+// it), added to fo / H
+__device__ __forceinline__ void vbd_term(const VArgs& a, const float p[4][3], const float B[3][3],
+                                         float V0, int l, float fo[3], float H[6]) {
   float f[3][3];
   deformation(p, B, f);
   const float J = det_cols(f);
@@ -448,15 +445,9 @@ __device__ __forceinline__ void vbd_entry(const VArgs& a, int32_t ent, float fo[
   cross3(f[0], f[1], cof[2]);
   const float s = a.lam * (J - 1.0f);
   float b[3];
-  if (l < 3) {
-    b[0] = B[l][0];
-    b[1] = B[l][1];
-    b[2] = B[l][2];
-  } else {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) b[c] = -(B[0][c] + B[1][c] + B[2][c]);
-  }
-  const float V0 = a.vol[tet];
+  for (int c = 0; c < 3; ++c)
+    b[c] = l == 0 ? B[0][c] : l == 1 ? B[1][c] : l == 2 ? B[2][c] : -(B[0][c] + B[1][c] + B[2][c]);
   float qv[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -475,28 +466,58 @@ __device__ __forceinline__ void vbd_entry(const VArgs& a, int32_t ent, float fo[
   H[5] += V0 * (a.lam * (qv[1] * qv[2]));
 }
 
-// inertia, damping and the 3x3 solve of vertex vi from the summed tet
-// terms; skipped (as the reference) when |det H| <= 1e-10
-__device__ __forceinline__ void vbd_finish(const VArgs& a, int64_t vi, float w, const float fs[3],
-                                           const float Hs[6]) {
+__device__ __forceinline__ void vbd_entry(const VArgs& a, int32_t ent, float fo[3], float H[6]) {
+  const int64_t tet = ent >> 2;
+  const int l = ent & 3;
+  const int4 q = a.t_i[tet];
+  const int64_t vid[4] = {q.x, q.y, q.z, q.w};
+  float p[4][3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) p[k][c] = a.x[3 * vid[k] + c];
+  float B[3][3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) B[r][c] = a.dm[9 * tet + 3 * r + c];
+  vbd_term(a, p, B, a.vol[tet], l, fo, H);
+}
+
+// What a vertex's solve reads beside its tets: mass / h^2, the inertial and the
+// old position
+struct VInertia {
+  float mh, xt[3], xo[3];
+};
+__device__ __forceinline__ VInertia vbd_inertia(const VArgs& a, int64_t vi, float w) {
+  VInertia m;
   const float mi = 1.0f / w;
-  const float mh = mi / a.h2;
-  float x[3], f[3];
+  m.mh = mi / a.h2;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    x[c] = a.x[3 * vi + c];
-    f[c] = mh * (a.xt[3 * vi + c] - x[c]) + fs[c];
+    m.xt[c] = a.xt[3 * vi + c];
+    m.xo[c] = a.kd > 0.0f ? a.xo[3 * vi + c] : 0.0f;
   }
-  if (a.keep_prev) {
+  return m;
+}
+
+// inertia, damping and the 3x3 solve of a vertex at x from the summed tet
+// terms: its new position in y (x, as the reference, when |det H| <= 1e-10)
+__device__ __forceinline__ void vbd_solve(const VArgs& a, const VInertia& m, const float x[3],
+                                          const float fs[3], const float Hs[6], float y[3]) {
+  const float mh = m.mh;
+  float f[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) a.xp[3 * vi + c] = x[c];
+  for (int c = 0; c < 3; ++c) {
+    f[c] = mh * (m.xt[c] - x[c]) + fs[c];
+    y[c] = x[c];
   }
   float H[3][3] = {{mh + Hs[0], Hs[3], Hs[4]}, {Hs[3], mh + Hs[1], Hs[5]}, {Hs[4], Hs[5], mh + Hs[2]}};
   if (a.kd > 0.0f) {
     const float kdt = a.kd / a.dt;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      f[c] -= kdt * (x[c] - a.xo[3 * vi + c]);
+      f[c] -= kdt * (x[c] - m.xo[c]);
       H[c][c] += kdt;
     }
   }
@@ -504,9 +525,22 @@ __device__ __forceinline__ void vbd_finish(const VArgs& a, int64_t vi, float w, 
     float inv[3][3];
     inv3(H, inv);
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-      a.x[3 * vi + i] = x[i] + (inv[i][0] * f[0] + inv[i][1] * f[1] + inv[i][2] * f[2]);
+    for (int i = 0; i < 3; ++i) y[i] = x[i] + (inv[i][0] * f[0] + inv[i][1] * f[1] + inv[i][2] * f[2]);
   }
+}
+
+__device__ __forceinline__ void vbd_finish(const VArgs& a, int64_t vi, float w, const float fs[3],
+                                           const float Hs[6]) {
+  float x[3], y[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) x[c] = a.x[3 * vi + c];
+  if (a.keep_prev) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a.xp[3 * vi + c] = x[c];
+  }
+  vbd_solve(a, vbd_inertia(a, vi, w), x, fs, Hs, y);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) a.x[3 * vi + c] = y[c];
 }
 
 // sum of 9 values over groups of W lanes (fixed xor tree; all 32 lanes call)
@@ -559,6 +593,135 @@ __global__ void k_vbd_serial(VArgs a, const float* __restrict__ om, int32_t n_it
   }
 }
 
+// As for the tets of XPBD, without a barrier: a vertex of iteration n waits for
+// its neighbours' positions, those of earlier colours of iteration n and those
+// of later colours of iteration n - 1 (with Chebyshev: accelerated).  Each
+// vertex publishes both with the count of its iterations; it cannot overwrite
+// one that a neighbour still needs, because it waits for that neighbour.  What a
+// vertex reads of its tets is laid out in the order of the lanes at each solve,
+// so a warp streams it from L1, and what does not wait is loaded before.  10
+// iterations over 24^3 hexes: 461 us with a grid barrier between the colours, 9
+// scattered words a tet and four dependent loads before them; 180 here, 3.6 us a
+// colour: the exchange through L2, then the tets and the solve in a row.
+struct VFlowArgs {
+  const int32_t* vert;    // the vertices of a warp, of one colour, a chunk (-1: padding)
+  const int32_t* nb_off;  // first round of neighbours of each chunk
+  const uint32_t* nb;     // [round][32]: neighbour * 2 + (1: of an earlier colour)
+  const int32_t* rec_off; // first step of each chunk
+  float4* rec;            // [step][3][32]: B, V0, the tet's vertices as places in
+                          // the neighbours (bytes), the vertex's place in the tet
+  const int32_t* ent;     // [step][32]: tet * 4 + place, -1: none
+  const uint32_t* loc;    // [step][32]: those bytes
+  float4* xa;             // positions after an iteration, before Chebyshev
+  float4* xb;             // and after it (the same array without)
+  int32_t n_chunks, n_steps;
+  int32_t max_rounds;
+  int32_t n_iter;
+  float rho;
+  const float* om;
+  GridSync* gs;
+  int32_t* status;
+};
+constexpr uint32_t kNoVertex = 0xffffffffu;
+constexpr int kVblk = 32 / kVL;   // vertices of a warp
+constexpr int kVblkMost = 48;     // most neighbours (and itself) of one: 48 kB with 16 warps
+
+// rest matrices and volumes as they are now, in the order of VFlowArgs::rec
+__global__ void k_vbd_rest(const float* __restrict__ dm, const float* __restrict__ vol, VFlowArgs c) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 32LL * c.n_steps;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t ent = c.ent[i];
+    if (ent < 0) continue;
+    const float* B = dm + 9LL * (ent >> 2);
+    float4* r = c.rec + 3 * (i & ~31LL) + (i & 31);
+    r[0] = make_float4(B[0], B[1], B[2], B[3]);
+    r[32] = make_float4(B[4], B[5], B[6], B[7]);
+    r[64] = make_float4(B[8], vol[ent >> 2], __uint_as_float(c.loc[i]), __int_as_float(ent & 3));
+  }
+}
+
+__global__ void __launch_bounds__(32 * kVbdWarps) k_vbd_flow(VArgs a, VFlowArgs c) {
+  extern __shared__ float4 sv[];  // positions of the neighbours of a warp's vertices
+  const int lane = threadIdx.x & 31, gl = lane % kVL;
+  const int warp = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  float4* mine = sv + (threadIdx.x >> 5) * (32 * c.max_rounds) + (lane / kVL) * (kVL * c.max_rounds);
+  for (int32_t n = 0; n < c.n_iter; ++n) {
+    const bool cheb = c.rho > 0.0f && n >= 1;
+    const float om = cheb ? __ldg(c.om + n) : 0.0f;
+    for (int32_t j = warp; j < c.n_chunks; j += warps) {
+      const int32_t vi = __ldg(c.vert + kVblk * j + lane / kVL);
+      const float w = vi >= 0 ? __ldg(a.invm + vi) : 0.0f;
+      // this lane's tets (none of a fixed vertex)
+      const int32_t tets = w != 0.0f ? (__ldg(a.adj_ptr + vi + 1) - __ldg(a.adj_ptr + vi) + kVL - 1 - gl) / kVL : 0;
+      const int32_t r0 = __ldg(c.nb_off + j), r1 = __ldg(c.nb_off + j + 1);
+      const int32_t s0 = __ldg(c.rec_off + j), s1 = __ldg(c.rec_off + j + 1);
+      VInertia inertia;
+      if (gl == 0 && w != 0.0f) inertia = vbd_inertia(a, vi, w);
+      bool ok = true;
+      constexpr int K = 8;  // neighbours polled at once
+      for (int32_t r = r0; r < r1 && ok; r += K) {
+        const float4* at[K];
+        uint32_t want[K];
+        uint4 v[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const uint32_t u = r + k < r1 ? __ldg(c.nb + 32LL * (r + k) + lane) : kNoVertex;
+          const bool some = u != kNoVertex;
+          at[k] = some ? (u & 1 ? c.xa : c.xb) + (u >> 1) : nullptr;
+          want[k] = n + (some ? u & 1 : 0);
+        }
+        ok = wait_vertices(at, want, v, c.gs, c.status);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (at[k])
+            mine[kVL * (r - r0 + k) + gl] = make_float4(__uint_as_float(v[k].x), __uint_as_float(v[k].y),
+                                                        __uint_as_float(v[k].z), 0.0f);
+      }
+      if (!__all_sync(0xffffffffu, ok)) return;
+      __syncwarp();
+      float f[3] = {0.f, 0.f, 0.f}, H[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int32_t s = s0; s < s1; ++s) {
+        if (s - s0 >= tets) continue;
+        const float4* r = c.rec + 96LL * s + lane;
+        const float4 b0 = __ldg(r), b1 = __ldg(r + 32), b2 = __ldg(r + 64);
+        const float B[3][3] = {{b0.x, b0.y, b0.z}, {b0.w, b1.x, b1.y}, {b1.z, b1.w, b2.x}};
+        const uint32_t q = __float_as_uint(b2.z);
+        float p[4][3];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const float4 y = mine[q >> (8 * l) & 0xff];
+          p[l][0] = y.x;
+          p[l][1] = y.y;
+          p[l][2] = y.z;
+        }
+        vbd_term(a, p, B, b2.y, __float_as_int(b2.w), f, H);
+      }
+      group_sum<kVL>(f, H);
+      if (gl == 0 && vi >= 0) {
+        const float x[3] = {mine[0].x, mine[0].y, mine[0].z};  // (the vertex itself comes first)
+        float y[3] = {x[0], x[1], x[2]}, z[3];
+        if (w != 0.0f) vbd_solve(a, inertia, x, f, H, y);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) z[d] = cheb && w > 0.0f ? y[d] + om * (y[d] - x[d]) : y[d];
+        pdev::put_tagged(c.xa + vi, __float_as_uint(y[0]), __float_as_uint(y[1]), __float_as_uint(y[2]),
+                         n + 1);
+        if (c.xb != c.xa)
+          pdev::put_tagged(c.xb + vi, __float_as_uint(z[0]), __float_as_uint(z[1]),
+                           __float_as_uint(z[2]), n + 1);
+        if (n == c.n_iter - 1 && w != 0.0f) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) a.x[3LL * vi + d] = z[d];
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// With a grid barrier between the colours, for meshes with a vertex of more
+// neighbours than a warp of the above keeps
 struct VColorArgs {
   const int32_t* order;
   const int32_t* off;
@@ -652,17 +815,16 @@ int coop_grid(const void* fn, int threads) {
 
 constexpr int kFlowSmem = 28 * sizeof(float);  // bytes a thread (XFlowTet)
 
-// Warps of a colour kernel that waits for vertices: the chunks of a colour and
-// a quarter more, which have loaded what does not wait when their turn comes;
-// others only poll, in the way of those that can go on (10 passes over 24^3
-// hexes, 57 chunks a colour: 76 warps 814 us, 304 warps 916; 32^3, 137 chunks:
-// 76 warps 1232 us, 152 886, 304 942).
-void flow_shape(const void* fn, int smem, int64_t chunks, int32_t colors, int* grid, int* threads) {
+// Warps of a colour kernel that waits for vertices: `ahead` times the chunks of
+// a colour, which have loaded what does not wait when their turn comes; others
+// only poll, in the way of those that can go on.
+void flow_shape(const void* fn, int smem, int most, double ahead, int64_t chunks, int32_t colors,
+                int* grid, int* threads) {
   int dev = 0, sms = 0, occ = 0;
   MGPBD_CUDA(cudaGetDevice(&dev));
   MGPBD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int64_t warps = std::max<int64_t>(16, 5 * chunks / (4 * std::max(colors, 1)));
-  const int per = static_cast<int>(std::min<int64_t>(kFlowWarps, ceil_div(warps, sms)));
+  const int64_t warps = std::max<int64_t>(16, std::llround(ahead * chunks / std::max(colors, 1)));
+  const int per = static_cast<int>(std::min<int64_t>(most, ceil_div(warps, sms)));
   *grid = static_cast<int>(std::min<int64_t>(sms, ceil_div(warps, per)));
   *threads = 32 * per;
   MGPBD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, *threads, smem * *threads));
@@ -768,7 +930,10 @@ void Xpbd::set_mesh(float* x, const float* x_ref, const float* invm, const int32
     n_chunks_ = 0;
     if (distinct_vertices(ht)) {
       build_flow(col, ht);
-      flow_shape(reinterpret_cast<const void*>(k_xpbd_flow), kFlowSmem, n_chunks_, n_colors_, &grid_, &threads_);
+      // (57 chunks a colour, 10 passes: 76 warps 814 us, 304 warps 916; 137
+      // chunks: 76 warps 1232 us, 152 886, 304 942)
+      flow_shape(reinterpret_cast<const void*>(k_xpbd_flow), kFlowSmem, kXpbdWarps, 1.25, n_chunks_,
+                 n_colors_, &grid_, &threads_);
     } else {
       upload(order_, col.ordered, s);
       upload(offsets_, col.offsets, s);
@@ -946,12 +1111,100 @@ void Vbd::set_mesh(float* x, const float* x_ref, const float* invm, const int32_
   if (p_.method == MGPBD_VBD_COLOR) {
     const Coloring col = color_vertices(ht.data(), nt, 4, nv);
     n_colors_ = col.n_colors;
-    upload(order_, col.ordered, s);
-    upload(offsets_, col.offsets, s);
     gs_.alloc(1);
-    grid_ = coop_grid(reinterpret_cast<const void*>(k_vbd_color), kLT);
+    if (!build_flow(col, ht, ptr, ent)) {
+      upload(order_, col.ordered, s);
+      upload(offsets_, col.offsets, s);
+      grid_ = coop_grid(reinterpret_cast<const void*>(k_vbd_color), kLT);
+    }
   }
   MGPBD_CUDA(cudaStreamSynchronize(s));
+}
+
+// The vertices in chunks of a warp's, of one colour, their neighbours and tets in the
+// order of a warp's lanes.  False: a vertex has too many neighbours.
+bool Vbd::build_flow(const Coloring& col, const std::vector<int32_t>& ht,
+                     const std::vector<int32_t>& ptr, const std::vector<int32_t>& ent) {
+  n_chunks_ = 0;
+  std::vector<int32_t> color(nv_), vert;
+  for (int32_t c = 0; c < col.n_colors; ++c) {
+    for (int32_t i = col.offsets[c]; i < col.offsets[c + 1]; ++i) {
+      color[col.ordered[i]] = c;
+      vert.push_back(col.ordered[i]);
+    }
+    while (vert.size() % kVblk) vert.push_back(-1);
+  }
+  const size_t chunks = vert.size() / kVblk;
+  std::vector<int32_t> nb_off(chunks + 1, 0), rec_off(chunks + 1, 0), entries;
+  std::vector<uint32_t> nb, loc;
+  std::vector<int32_t> place(nv_, -1);
+  int32_t most = 0;
+  std::vector<int32_t> list[kVblk];
+  nb.reserve(8 * vert.size());
+  loc.reserve(2 * ent.size());
+  entries.reserve(2 * ent.size());
+  for (size_t j = 0; j < chunks; ++j) {
+    size_t rounds = 0, steps = 0;
+    for (int b = 0; b < kVblk; ++b) {
+      const int32_t v = vert[kVblk * j + b];
+      list[b].clear();
+      if (v < 0) continue;
+      list[b].push_back(v);
+      for (int32_t e = ptr[v]; e < ptr[v + 1]; ++e)
+        for (int l = 0; l < 4; ++l) {
+          const int32_t u = ht[4 * static_cast<size_t>(ent[e] >> 2) + l];
+          if (u != v && place[u] < 0) {
+            place[u] = 1;
+            list[b].push_back(u);
+          }
+        }
+      for (int32_t u : list[b]) place[u] = -1;
+      if (list[b].size() > static_cast<size_t>(kVblkMost)) return false;
+      rounds = std::max(rounds, (list[b].size() + kVL - 1) / kVL);
+      steps = std::max<size_t>(steps, (ptr[v + 1] - ptr[v] + kVL - 1) / kVL);
+    }
+    most = std::max(most, static_cast<int32_t>(rounds));
+    const size_t n0 = nb.size(), e0 = entries.size();
+    nb.resize(n0 + 32 * rounds, kNoVertex);
+    entries.resize(e0 + 32 * steps, -1);
+    loc.resize(e0 + 32 * steps, 0);
+    for (int b = 0; b < kVblk; ++b) {
+      const int32_t v = vert[kVblk * j + b];
+      if (v < 0) continue;
+      for (size_t m = 0; m < list[b].size(); ++m) {
+        const int32_t u = list[b][m];
+        place[u] = static_cast<int32_t>(m);
+        nb[n0 + 32 * (m / kVL) + kVL * b + m % kVL] = 2u * u + (color[u] < color[v] ? 1u : 0u);
+      }
+      for (int32_t e = ptr[v]; e < ptr[v + 1]; ++e) {
+        const size_t k = e - ptr[v], at = e0 + 32 * (k / kVL) + kVL * b + k % kVL;
+        entries[at] = ent[e];
+        for (int l = 0; l < 4; ++l)
+          loc[at] |= static_cast<uint32_t>(place[ht[4 * static_cast<size_t>(ent[e] >> 2) + l]]) << (8 * l);
+      }
+      for (int32_t u : list[b]) place[u] = -1;
+    }
+    nb_off[j + 1] = static_cast<int32_t>(nb.size() / 32);
+    rec_off[j + 1] = static_cast<int32_t>(entries.size() / 32);
+  }
+  cudaStream_t s = stream_;
+  upload(order_, vert, s);
+  upload(f_nb_off_, nb_off, s);
+  upload(f_rec_off_, rec_off, s);
+  upload(f_ent_, entries, s);
+  upload(f_nb_, std::vector<int32_t>(nb.begin(), nb.end()), s);
+  upload(f_loc_, std::vector<int32_t>(loc.begin(), loc.end()), s);
+  f_rec_.alloc(std::max<int64_t>(1, 3 * static_cast<int64_t>(entries.size())));
+  xa_.alloc(nv_);
+  if (p_.rho > 0.0f) xb_.alloc(nv_);
+  max_rounds_ = most;
+  n_steps_ = rec_off[chunks];
+  n_chunks_ = static_cast<int32_t>(chunks);
+  // (five colours, half of the vertices in the first; 781 chunks a colour, 10
+  // iterations: 1172 warps 197 us, 1953 180)
+  flow_shape(reinterpret_cast<const void*>(k_vbd_flow), flow_smem(), kVbdWarps, 2.5, n_chunks_,
+             n_colors_, &grid_, &threads_);
+  return true;
 }
 
 void Vbd::init() {
@@ -1005,19 +1258,53 @@ void Vbd::solve() {
     MGPBD_CHECK_LAUNCH();
     return;
   }
-  VColorArgs c;
-  c.order = order_.p;
-  c.off = offsets_.p;
-  c.n_colors = n_colors_;
-  c.n_iter = p_.n_iterations;
-  c.rho = p_.rho;
-  c.om = om_.p;
-  c.gs = gs_.p;
-  c.status = status_.p;
   MGPBD_CUDA(cudaMemsetAsync(gs_.p, 0, sizeof(GridSync), s));
-  void* args[] = {&a, &c};
-  MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_vbd_color), dim3(grid_),
-                                         dim3(kLT), args, 0, s));
+  if (n_chunks_ > 0) {
+    VFlowArgs f;
+    f.vert = order_.p;
+    f.nb_off = f_nb_off_.p;
+    f.nb = reinterpret_cast<const uint32_t*>(f_nb_.p);
+    f.rec_off = f_rec_off_.p;
+    f.rec = f_rec_.p;
+    f.ent = f_ent_.p;
+    f.loc = reinterpret_cast<const uint32_t*>(f_loc_.p);
+    f.xa = xa_.p;
+    f.xb = p_.rho > 0.0f ? xb_.p : xa_.p;
+    f.n_chunks = n_chunks_;
+    f.n_steps = n_steps_;
+    f.max_rounds = max_rounds_;
+    f.n_iter = p_.n_iterations;
+    f.rho = p_.rho;
+    f.om = om_.p;
+    f.gs = gs_.p;
+    f.status = status_.p;
+    if (n_steps_ > 0) {
+      k_vbd_rest<<<blocks_for(32LL * n_steps_), kLT, 0, s>>>(dm_inv_.p, vol_.p, f);
+      MGPBD_CHECK_LAUNCH();
+    }
+    k_flow_start<<<blocks_for(nv_), kLT, 0, s>>>(x_, xa_.p, nv_);
+    MGPBD_CHECK_LAUNCH();
+    if (f.xb != f.xa) {
+      k_flow_start<<<blocks_for(nv_), kLT, 0, s>>>(x_, xb_.p, nv_);
+      MGPBD_CHECK_LAUNCH();
+    }
+    void* args[] = {&a, &f};
+    MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_vbd_flow), dim3(grid_),
+                                           dim3(threads_), args, flow_smem() * threads_, s));
+  } else {
+    VColorArgs c;
+    c.order = order_.p;
+    c.off = offsets_.p;
+    c.n_colors = n_colors_;
+    c.n_iter = p_.n_iterations;
+    c.rho = p_.rho;
+    c.om = om_.p;
+    c.gs = gs_.p;
+    c.status = status_.p;
+    void* args[] = {&a, &c};
+    MGPBD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_vbd_color), dim3(grid_),
+                                           dim3(kLT), args, 0, s));
+  }
   MGPBD_CHECK_LAUNCH();
   lazy_.record(status_.p, s);
 }

@@ -1,7 +1,7 @@
 // Comparison solvers of the MGPBD convergence experiments: local XPBD
 // (cons/deform3d.py) and Vertex Block Descent (cons/vbd.py).  The colour
-// methods run as one cooperative kernel per pass / solve with a bounded grid
-// barrier between colours; the serial methods keep the reference's order
+// methods run as one cooperative kernel per pass / solve whose warps wait
+// (bounded) for the vertices they read; the serial methods keep the reference's order
 // (one tet, or one vertex, at a time).
 #pragma once
 
@@ -103,7 +103,14 @@ class Vbd {
   const int32_t* t_i_ = nullptr;
   int32_t nv_ = 0, nt_ = 0;
   bool inited_ = false;
+  bool build_flow(const Coloring& col, const std::vector<int32_t>& ht,
+                  const std::vector<int32_t>& ptr, const std::vector<int32_t>& ent);
+  int flow_smem() const { return 16 * max_rounds_; }  // bytes a thread
   DevBuf<float> v_, x_old_, x_tilde_, x_prev_, dm_inv_, vol_, om_;
+  DevBuf<float4> xa_, xb_, f_rec_;
+  DevBuf<int32_t> f_nb_off_, f_nb_, f_rec_off_, f_ent_, f_loc_;
+  int32_t n_chunks_ = 0, n_steps_ = 0, max_rounds_ = 0;
+  int threads_ = 0;
   DevBuf<int32_t> adj_ptr_, adj_, order_, offsets_, status_;
   DevBuf<GridSync> gs_;
   int32_t n_colors_ = 0;
