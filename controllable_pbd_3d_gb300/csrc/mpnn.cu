@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kT = 256;           // threads of the row-parallel kernels
 constexpr int kLayerRows = 64;    // aggregates per layer CTA
-constexpr int kLayerThreads = 128;
+constexpr int kLayerThreads = 512;
 constexpr int kXS = 136;          // padded bf16 row stride of the shared tiles
 constexpr int kWgradBlocks = 304; // 2 x 152 SMs
 constexpr int kBigPart = 2 * kNetF * kNetF + kNetF;  // W (128 x 64) + b
@@ -51,16 +51,17 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// float64 block sum in a fixed pattern; valid in thread 0
+// float64 block sum in a fixed pattern; valid in thread 0.  One warp adds:
+// float64 additions are slow.
 __device__ __forceinline__ double block_sum_d(double v) {
-  __shared__ double sh[32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  v = warp_sum_d(v);
-  if (lane == 0) sh[wid] = v;
+  __shared__ double sh[kT];
+  sh[threadIdx.x] = v;
   __syncthreads();
-  int nw = (blockDim.x + 31) >> 5;
-  v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
-  if (wid == 0) v = warp_sum_d(v);
+  v = 0.0;
+  if (threadIdx.x < 32) {
+    for (int i = threadIdx.x; i < blockDim.x; i += 32) v += sh[i];
+    v = warp_sum_d(v);
+  }
   __syncthreads();
   return v;
 }
@@ -84,9 +85,19 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 
 // ---- forward ---------------------------------------------------------------
 
-// partials of sum_i (s_i r_i)^2
-__global__ void k_net_sumsq(int32_t n, const float* __restrict__ r,
-                            const float* __restrict__ dinv, double* __restrict__ part) {
+// The fields of a batch: field k is samples + ((first + k) % count) n
+struct NetFields {
+  const float* samples;
+  int32_t first, count;
+  __device__ const float* at(int k, int32_t n) const {
+    return samples + (int64_t)((first + (int64_t)k) % count) * n;
+  }
+};
+
+// partials of sum_i (s_i r_i)^2, fields along grid.y
+__global__ void k_net_sumsq(int32_t n, NetFields f, const float* __restrict__ dinv,
+                            double* __restrict__ part) {
+  const float* r = f.at(blockIdx.y, n);
   double acc = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -94,7 +105,7 @@ __global__ void k_net_sumsq(int32_t n, const float* __restrict__ r,
     acc += (double)v * (double)v;
   }
   acc = block_sum_d(acc);
-  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+  if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = acc;
 }
 
 __global__ void k_net_sum(const double* __restrict__ part, int blocks, double* __restrict__ out,
@@ -105,14 +116,24 @@ __global__ void k_net_sum(const double* __restrict__ part, int blocks, double* _
   if (threadIdx.x == 0) out[0] = accumulate ? out[0] + acc : acc;
 }
 
-__device__ __forceinline__ float inv_sigma(const double* sumsq, int32_t n) {
-  double ss = *sumsq;
-  return ss > 0.0 ? (float)(1.0 / sqrt(ss / (double)n)) : 0.f;
+// sigma = sqrt(|S r|^2 / n) and its inverse, of each block's field.  Made here
+// once: in each thread of the kernels that use it, the float64 root and
+// quotients were most of their time (layer 1 25 -> 8 us for 13,800 rows).
+__global__ void k_net_sigma(const double* __restrict__ part, int blocks, int32_t n,
+                            NetSigma* __restrict__ out) {
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < blocks; i += blockDim.x) acc += part[blockIdx.x * blocks + i];
+  acc = block_sum_d(acc);
+  if (threadIdx.x == 0) {
+    const bool some = acc > 0.0;
+    out[blockIdx.x].inv = some ? (float)(1.0 / sqrt(acc / (double)n)) : 0.f;
+    out[blockIdx.x].sigma = some ? (float)sqrt(acc / (double)n) : 0.f;
+  }
 }
 
 // layer 1: warp per aggregate; H1 = relu(u w1s + (Ah u) w1n + b1)
 __global__ void __launch_bounds__(kT) k_net_l1(NetGraph g, const float* __restrict__ r,
-                                               const double* __restrict__ sumsq,
+                                               const NetSigma* __restrict__ sg,
                                                const float* __restrict__ P,
                                                __nv_bfloat16* __restrict__ H1,
                                                float* __restrict__ ah,
@@ -122,7 +143,7 @@ __global__ void __launch_bounds__(kT) k_net_l1(NetGraph g, const float* __restri
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (kT / 32) + (threadIdx.x >> 5);
   if (row >= g.n) return;
-  const float inv = inv_sigma(sumsq, g.n);
+  const float inv = sg->inv;
   const float si = scale_of(g.diag_inv, row);
   const float ui = si * r[row] * inv;
   float acc = 0.f;  // sum_j Ah_ij u_j; Ah_ij = s_i A_ij s_j kept for the layers
@@ -160,7 +181,7 @@ __global__ void __launch_bounds__(kLayerThreads) k_net_layer(
     NetGraph g, const float* __restrict__ ah, const __nv_bfloat16* __restrict__ H,
     const __nv_bfloat16* __restrict__ Wt, const float* __restrict__ P, int bias_off,
     __nv_bfloat16* __restrict__ Hn,
-    __nv_bfloat16* __restrict__ Gout, const double* __restrict__ sumsq, float* __restrict__ y_out,
+    __nv_bfloat16* __restrict__ Gout, const NetSigma* __restrict__ sg, float* __restrict__ y_out,
     float* __restrict__ e_out, float* __restrict__ h3_out) {
   __shared__ __align__(16) __nv_bfloat16 Xs[kLayerRows * kXS];
   __shared__ __align__(16) __nv_bfloat16 Ws[kNetF * kXS];
@@ -180,13 +201,16 @@ __global__ void __launch_bounds__(kLayerThreads) k_net_layer(
     *reinterpret_cast<uint4*>(Xs + r * kXS + k8 * 8) = v;
   }
 
-  // G = Ah H for this CTA's rows: warp w takes rows 16w..16w+15.  The warp
+  // G = Ah H for this CTA's rows: warp w takes rows 4w..4w+3 (with
+  // four warps of 16 rows each, one after the other, a layer of 13,800 rows
+  // took 36 us; here 13).  The warp
   // loads up to 32 (column, Ah) pairs of a row at once; each quarter warp
   // then gathers four neighbours' 64 features (16 bytes a lane) before
   // using any, so 16 neighbour rows are in flight per warp.
   const int grp = lane >> 3, sub = lane & 7;
-  for (int rr = 0; rr < 16; ++rr) {
-    const int r = warp * 16 + rr;
+  constexpr int kAggRows = kLayerRows / (kLayerThreads / 32);
+  for (int rr = 0; rr < kAggRows; ++rr) {
+    const int r = warp * kAggRows + rr;
     const int row = row0 + r;
     float acc[8];
 #pragma unroll
@@ -249,7 +273,8 @@ __global__ void __launch_bounds__(kLayerThreads) k_net_layer(
   }
   __syncthreads();
 
-  // X (rows 16w..16w+15) . W on the tensor cores
+  // X (rows 16w..16w+15) . W on the tensor cores, by four of the warps
+  if (warp >= kLayerRows / 16) return;
   float acc[8][4];
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
@@ -314,8 +339,7 @@ __global__ void __launch_bounds__(kLayerThreads) k_net_layer(
     yb += __shfl_xor_sync(0xffffffffu, yb, 2);
     if (tq == 0) {
       const float bo = P[kNetOffBo];
-      const double ss = *sumsq;
-      const float sigma = ss > 0.0 ? (float)sqrt(ss / (double)g.n) : 0.f;
+      const float sigma = sg->sigma;
       ya += bo;
       yb += bo;
       if (rowA < g.n) {
@@ -366,33 +390,70 @@ __global__ void __launch_bounds__(kT) k_net_out_bwd(NetGraph g, const float* __r
   if (threadIdx.x == 0) loss_part[blockIdx.x] = lacc;
 }
 
-// Weights form, per sample: u = S r / sigma_r, v = w * u (w the squashed
-// weights, dw = dw/dy), gy += (Ah v - u) * u * dw * scale, loss partials of
-// (1/2 v^T Ah v - v^T u) * scale.  Warp per row over a fixed grid.
+// Weights form: per sample u = S r / sigma_r, v = w u (w the squashed weights,
+// dw = dw/dy), gy += (Ah v - u) u dw scale, loss partials of (1/2 v^T Ah v -
+// v^T u) scale.  kNetSamples samples at once, so that a row's matrix entries
+// are read once for them, with v and u of a row side by side (a launch each,
+// with the roots and quotients in every thread, took 28 us a sample).
+constexpr int kNetSamples = 8;
+
+// u and v of samples s0 .. of a row: uv[row][0..7] = v, uv2[row][0..7] = u
+__global__ void k_net_uv(NetGraph g, NetFields f, int s0, int ns, const NetSigma* __restrict__ sg,
+                         const float* __restrict__ w, float* __restrict__ vs,
+                         float* __restrict__ us) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= g.n) return;
+  const float si = scale_of(g.diag_inv, (int)i), wi = w[i];
+#pragma unroll
+  for (int k = 0; k < kNetSamples; ++k) {
+    const float u = k < ns ? si * f.at(s0 + k, g.n)[i] * sg[s0 + k].inv : 0.f;
+    us[kNetSamples * i + k] = u;
+    vs[kNetSamples * i + k] = wi * u;
+  }
+}
+
+// Warp per row over a fixed grid
 __global__ void __launch_bounds__(kT) k_net_wloss(NetGraph g, const float* __restrict__ ah,
-                                                  const float* __restrict__ w,
-                                                  const float* __restrict__ dw,
-                                                  const float* __restrict__ r,
-                                                  const double* __restrict__ sumsq, float scale,
+                                                  const float* __restrict__ dw, int ns,
+                                                  const float* __restrict__ vs,
+                                                  const float* __restrict__ us, float scale,
                                                   float* __restrict__ gy,
                                                   double* __restrict__ loss_part) {
   const int lane = threadIdx.x & 31;
   const int wpb = kT / 32;
-  const float inv = inv_sigma(sumsq, g.n);
-  double lacc = 0.0;
+  double lacc = 0.0;  // of the lane's sample
   for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < g.n; row += gridDim.x * wpb) {
-    float acc = 0.f;
+    float acc[kNetSamples];
+#pragma unroll
+    for (int s = 0; s < kNetSamples; ++s) acc[s] = 0.f;
     for (int k = g.indptr[row] + lane; k < g.indptr[row + 1]; k += 32) {
-      const int j = g.indices[k];
-      acc += ah[k] * (w[j] * (scale_of(g.diag_inv, j) * r[j] * inv));
+      const float a = ah[k];
+      const float4* v = reinterpret_cast<const float4*>(vs + (int64_t)kNetSamples * g.indices[k]);
+      const float4 x = v[0], y = v[1];
+      acc[0] += a * x.x;
+      acc[1] += a * x.y;
+      acc[2] += a * x.z;
+      acc[3] += a * x.w;
+      acc[4] += a * y.x;
+      acc[5] += a * y.y;
+      acc[6] += a * y.z;
+      acc[7] += a * y.w;
     }
-    const float av = warp_sum_f(acc);
-    if (lane == 0) {
-      const float ui = scale_of(g.diag_inv, row) * r[row] * inv;
-      const float vi = w[row] * ui;
-      gy[row] += (av - ui) * ui * dw[row] * scale;
+    float av = 0.f;
+#pragma unroll
+    for (int s = 0; s < kNetSamples; ++s) {
+      const float t = warp_sum_f(acc[s]);
+      if (lane == s) av = t;
+    }
+    float term = 0.f;
+    if (lane < ns) {
+      const float ui = us[(int64_t)kNetSamples * row + lane], vi = vs[(int64_t)kNetSamples * row + lane];
+      term = (av - ui) * ui * dw[row] * scale;
       lacc += (0.5 * (double)vi * (double)av - (double)vi * (double)ui) * (double)scale;
     }
+    float sum = gy[row];
+    for (int s = 0; s < ns; ++s) sum += __shfl_sync(0xffffffffu, term, s);
+    if (lane == 0) gy[row] = sum;
   }
   lacc = block_sum_d(lacc);
   if (threadIdx.x == 0) loss_part[blockIdx.x] = lacc;
@@ -489,90 +550,151 @@ __global__ void __launch_bounds__(kT) k_net_wgrad_l1(int32_t n, const float* __r
 }
 
 // partials of [W | b] for X = [H, G] (bf16, n x 128) and gz (n x 64):
-// W[k][f] = sum_i X[i][k] gz[i][f], b[f] = sum_i gz[i][f].  Thread t owns
-// k = t / 2 and the features f = 2 j + (t & 1).
-__global__ void __launch_bounds__(kT) k_net_wgrad_big(int32_t n,
+// W[k][f] = sum_i X[i][k] gz[i][f], b[f] = sum_i gz[i][f].  A thread owns 8 k by
+// 4 f: three 16-byte reads of shared memory for 32 multiply-adds (with 32 f of
+// one k, 33 reads were the bound: 43 us a layer of 13,800 rows, here 14).
+__global__ void __launch_bounds__(kT, 2) k_net_wgrad_big(int32_t n,
                                                       const __nv_bfloat16* __restrict__ H,
                                                       const __nv_bfloat16* __restrict__ G,
                                                       const float* __restrict__ gz,
                                                       float* __restrict__ part) {
   constexpr int kTile = 32;
-  __shared__ float xs[kTile][2 * kNetF];
-  __shared__ float zs[kTile][kNetF];
-  const int t = threadIdx.x, k = t >> 1, par = t & 1;
+  __shared__ __align__(16) float xs[kTile][2 * kNetF];
+  __shared__ __align__(16) float zs[kTile][kNetF];
+  const int t = threadIdx.x, k0 = 8 * (t >> 4), f0 = 4 * (t & 15);
   int lo, hi;
   block_rows(n, lo, hi);
-  float acc[32];
+  float acc[8][4];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[j][c] = 0.f;
   float accb = 0.f;
   for (int base = lo; base < hi; base += kTile) {
     const int rows = min(kTile, hi - base);
     __syncthreads();
-    for (int c = t; c < kTile * 2 * kNetF; c += kT) {
-      const int r = c >> 7, kk = c & 127;
-      float v = 0.f;
-      if (r < rows) {
-        const int64_t i = base + r;
-        v = kk < kNetF ? __bfloat162float(H[i * kNetF + kk]) : __bfloat162float(G[i * kNetF + kk - kNetF]);
-      }
-      xs[r][kk] = v;
+    for (int c = t; c < kTile * 16; c += kT) {  // 16 bytes (8 features) of H or G each
+      const int r = c >> 4, kk = 8 * (c & 15);
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < rows)
+        v = *reinterpret_cast<const uint4*>((kk < kNetF ? H + kk : G + kk - kNetF) +
+                                            (int64_t)(base + r) * kNetF);
+      *reinterpret_cast<float4*>(&xs[r][kk]) = make_float4(bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y));
+      *reinterpret_cast<float4*>(&xs[r][kk + 4]) =
+          make_float4(bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w));
     }
-    for (int c = t; c < kTile * kNetF; c += kT) {
-      const int r = c >> 6, ff = c & 63;
-      zs[r][ff] = r < rows ? gz[(int64_t)(base + r) * kNetF + ff] : 0.f;
+    for (int c = t; c < kTile * (kNetF / 4); c += kT) {
+      const int r = c >> 4, ff = 4 * (c & 15);
+      *reinterpret_cast<float4*>(&zs[r][ff]) =
+          r < rows ? *reinterpret_cast<const float4*>(gz + (int64_t)(base + r) * kNetF + ff)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
+#pragma unroll 4
     for (int r = 0; r < rows; ++r) {
-      const float x = xs[r][k];
+      const float4 xa = *reinterpret_cast<const float4*>(&xs[r][k0]);
+      const float4 xb = *reinterpret_cast<const float4*>(&xs[r][k0 + 4]);
+      const float4 z = *reinterpret_cast<const float4*>(&zs[r][f0]);
+      const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] += x * zs[r][2 * j + par];
+      for (int j = 0; j < 8; ++j) {
+        acc[j][0] += x[j] * z.x;
+        acc[j][1] += x[j] * z.y;
+        acc[j][2] += x[j] * z.z;
+        acc[j][3] += x[j] * z.w;
+      }
       if (t < kNetF) accb += zs[r][t];
     }
   }
   float* out = part + (int64_t)blockIdx.x * kBigPart;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) out[k * kNetF + 2 * j + par] = acc[j];
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<float4*>(out + (k0 + j) * kNetF + f0) =
+        make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
   if (t < kNetF) out[2 * kNetF * kNetF + t] = accb;
 }
 
-// dst[c] += sum_b part[b * count + c], blocks in ascending order
-__global__ void k_net_wsum(const float* __restrict__ part, int blocks, int count,
-                           float* __restrict__ dst) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= count) return;
+// dst[c] += sum_b part[b * count + c]: kWsumGroups chains over the blocks, added
+// in a fixed order (one chain of 216 blocks took 17 us, here 8)
+constexpr int kWsumGroups = 16;
+__global__ void __launch_bounds__(16 * kWsumGroups) k_net_wsum(const float* __restrict__ part, int blocks,
+                                                               int count, float* __restrict__ dst) {
+  __shared__ float sh[kWsumGroups][16];
+  const int c = blockIdx.x * 16 + (threadIdx.x & 15), grp = threadIdx.x >> 4;
   float acc = 0.f;
-  for (int b = 0; b < blocks; ++b) acc += part[(int64_t)b * count + c];
-  dst[c] += acc;
+  if (c < count) {
+#pragma unroll 8
+    for (int b = grp; b < blocks; b += kWsumGroups) acc += part[(int64_t)b * count + c];
+  }
+  sh[grp][threadIdx.x & 15] = acc;
+  __syncthreads();
+  if (threadIdx.x < 16 && c < count) {
+    acc = 0.f;
+    for (int k = 0; k < kWsumGroups; ++k) acc += sh[k][threadIdx.x];
+    dst[c] += acc;
+  }
 }
 
-// gX = gz W^T (n x 128): gself = columns 0..63, q = columns 64..127.
-// Thread t of the 128 owns input feature k = t; rows in tiles of 32.
-__global__ void __launch_bounds__(2 * kNetF) k_net_xgrad(int32_t n, const float* __restrict__ gz,
-                                                         const __nv_bfloat16* __restrict__ Wt,
-                                                         float* __restrict__ gself,
-                                                         float* __restrict__ q) {
-  constexpr int kTile = 32;
-  __shared__ float wf[kNetF][2 * kNetF];
-  __shared__ float zs[kTile][kNetF];
-  const int t = threadIdx.x;
-  for (int c = t; c < kNetF * 2 * kNetF; c += blockDim.x)
-    wf[c >> 7][c & 127] = __bfloat162float(Wt[c]);
-  const int base = blockIdx.x * kTile;
-  for (int c = t; c < kTile * kNetF; c += blockDim.x) {
+// gX = gz W^T (n x 128): gself = columns 0..63, q = columns 64..127.  A block
+// takes kXgRows rows; a thread owns 4 rows by 4 columns of each, so a step over o reads
+// three times 16 bytes of shared memory for 32 multiply-adds (with one column a
+// thread, two reads a multiply-add: 30 us a layer of 13,800 rows, here 18).
+constexpr int kXgRows = 64;
+__global__ void __launch_bounds__(kT, 2) k_net_xgrad(int32_t n, const float* __restrict__ gz,
+                                                  const __nv_bfloat16* __restrict__ Wt,
+                                                  float* __restrict__ gself,
+                                                  float* __restrict__ q) {
+  __shared__ __align__(16) float wf[kNetF / 2][2 * kNetF];  // W^T, 32 of its rows at a time
+  __shared__ __align__(16) float zs[kNetF][kXgRows + 4];    // gz transposed
+  const int t = threadIdx.x, c0 = 4 * (t & 15), r0 = 4 * (t >> 4);
+  const int base = blockIdx.x * kXgRows;
+  for (int c = t; c < kXgRows * kNetF; c += kT) {
     const int r = c >> 6, f = c & 63;
-    zs[r][f] = base + r < n ? gz[(int64_t)(base + r) * kNetF + f] : 0.f;
+    zs[f][r] = base + r < n ? gz[(int64_t)(base + r) * kNetF + f] : 0.f;
   }
-  __syncthreads();
-  for (int r = 0; r < kTile && base + r < n; ++r) {
-    float acc = 0.f;
-#pragma unroll 16
-    for (int o = 0; o < kNetF; ++o) acc += zs[r][o] * wf[o][t];
-    const int64_t i = base + r;
-    if (t < kNetF)
-      gself[i * kNetF + t] = acc;
-    else
-      q[i * kNetF + t - kNetF] = acc;
+  float acc[4][8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[j][c] = 0.f;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    __syncthreads();
+    for (int c = t; c < kNetF / 2 * 16; c += kT) {
+      const int o = c >> 4, kk = 8 * (c & 15);
+      const uint4 v = *reinterpret_cast<const uint4*>(Wt + (h * (kNetF / 2) + o) * 2 * kNetF + kk);
+      *reinterpret_cast<float4*>(&wf[o][kk]) = make_float4(bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y));
+      *reinterpret_cast<float4*>(&wf[o][kk + 4]) =
+          make_float4(bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w));
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int o = 0; o < kNetF / 2; ++o) {
+      const float4 z = *reinterpret_cast<const float4*>(&zs[h * (kNetF / 2) + o][r0]);
+      const float4 wa = *reinterpret_cast<const float4*>(&wf[o][c0]);
+      const float4 wb = *reinterpret_cast<const float4*>(&wf[o][kNetF + c0]);
+      const float zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[j][0] += zz[j] * wa.x;
+        acc[j][1] += zz[j] * wa.y;
+        acc[j][2] += zz[j] * wa.z;
+        acc[j][3] += zz[j] * wa.w;
+        acc[j][4] += zz[j] * wb.x;
+        acc[j][5] += zz[j] * wb.y;
+        acc[j][6] += zz[j] * wb.z;
+        acc[j][7] += zz[j] * wb.w;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int64_t i = base + r0 + j;
+    if (i >= n) continue;
+    *reinterpret_cast<float4*>(gself + i * kNetF + c0) =
+        make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+    *reinterpret_cast<float4*>(q + i * kNetF + c0) =
+        make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
   }
 }
 
@@ -678,7 +800,7 @@ void CoarseNet::ensure(const NetGraph& g) {
   if (n <= cap_) return;
   const int64_t nf = (int64_t)n * kNetF;
   part_.alloc(kMaxReduceBlocks);
-  sumsq_.alloc(2);
+  sigma_.alloc(1);
   u_.alloc(n);
   a1_.alloc(n);
   y_.alloc(n);
@@ -696,6 +818,8 @@ void CoarseNet::ensure(const NetGraph& g) {
   wcap_.alloc(n);
   wv_.alloc(n);
   dw_.alloc(n);
+  vs_.alloc((int64_t)n * kNetSamples);
+  us_.alloc((int64_t)n * kNetSamples);
   wpart_.alloc((int64_t)kWgradBlocks * kBigPart);
   cap_ = n;
 }
@@ -703,22 +827,22 @@ void CoarseNet::ensure(const NetGraph& g) {
 void CoarseNet::run_forward(const NetGraph& g, const float* r, float* e, float* y_out, bool train,
                             float* cap_out, cudaStream_t s) {
   const int32_t n = g.n;
-  const int rb = std::min(kMaxReduceBlocks, std::max(1, ceil_div(n, kT * 4)));
-  k_net_sumsq<<<rb, kT, 0, s>>>(n, r, g.diag_inv, part_.p);
+  const int rb = std::min(kMaxReduceBlocks, std::max(1, ceil_div(n, kT)));
+  k_net_sumsq<<<rb, kT, 0, s>>>(n, NetFields{r, 0, 1}, g.diag_inv, part_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_sum<<<1, kT, 0, s>>>(part_.p, rb, sumsq_.p, 0);
+  k_net_sigma<<<1, kT, 0, s>>>(part_.p, rb, n, sigma_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_l1<<<ceil_div(n, kT / 32), kT, 0, s>>>(g, r, sumsq_.p, p_.p, h1_.p, ah_.p, cap_out,
+  k_net_l1<<<ceil_div(n, kT / 32), kT, 0, s>>>(g, r, sigma_.p, p_.p, h1_.p, ah_.p, cap_out,
                                                 train ? u_.p : nullptr, train ? a1_.p : nullptr);
   MGPBD_CHECK_LAUNCH();
   const int lb = ceil_div(n, kLayerRows);
   k_net_layer<false><<<lb, kLayerThreads, 0, s>>>(g, ah_.p, h1_.p, wt_.p, p_.p, kNetOffB2, h2_.p,
-                                                  train ? g1_.p : nullptr, sumsq_.p, nullptr,
+                                                  train ? g1_.p : nullptr, sigma_.p, nullptr,
                                                   nullptr, nullptr);
   MGPBD_CHECK_LAUNCH();
   k_net_layer<true><<<lb, kLayerThreads, 0, s>>>(g, ah_.p, h2_.p, wt_.p + 2 * kNetF * kNetF, p_.p,
                                                  kNetOffB3, nullptr, train ? g2_.p : nullptr,
-                                                 sumsq_.p, y_out ? y_out : (train ? y_.p : nullptr),
+                                                 sigma_.p, y_out ? y_out : (train ? y_.p : nullptr),
                                                  e, train ? h3_.p : nullptr);
   MGPBD_CHECK_LAUNCH();
 }
@@ -753,14 +877,14 @@ void CoarseNet::backward_layers(const NetGraph& g, cudaStream_t s) {
   const int rowb = ceil_div(n, kT / 32);
   k_net_wgrad_out<<<wb, kT, 0, s>>>(n, h3_.p, gy_.p, wpart_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_wsum<<<1, kT, 0, s>>>(wpart_.p, wb, kNetF + 1, g_.p + kNetOffWo);
+  k_net_wsum<<<ceil_div(kNetF + 1, 16), 16 * kWsumGroups, 0, s>>>(wpart_.p, wb, kNetF + 1, g_.p + kNetOffWo);
   MGPBD_CHECK_LAUNCH();
   // layer 3
   k_net_wgrad_big<<<wb, kT, 0, s>>>(n, h2_.p, g2_.p, gz_.p, wpart_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_wsum<<<ceil_div(kBigPart, kT), kT, 0, s>>>(wpart_.p, wb, kBigPart, g_.p + kNetOffW3);
+  k_net_wsum<<<ceil_div(kBigPart, 16), 16 * kWsumGroups, 0, s>>>(wpart_.p, wb, kBigPart, g_.p + kNetOffW3);
   MGPBD_CHECK_LAUNCH();
-  k_net_xgrad<<<ceil_div(n, 32), 2 * kNetF, 0, s>>>(n, gz_.p, wt_.p + 2 * kNetF * kNetF,
+  k_net_xgrad<<<ceil_div(n, kXgRows), kT, 0, s>>>(n, gz_.p, wt_.p + 2 * kNetF * kNetF,
                                                      gself_.p, q_.p);
   MGPBD_CHECK_LAUNCH();
   k_net_hgrad<<<rowb, kT, 0, s>>>(g, ah_.p, gself_.p, q_.p, h2_.p, gz_.p);
@@ -768,16 +892,16 @@ void CoarseNet::backward_layers(const NetGraph& g, cudaStream_t s) {
   // layer 2
   k_net_wgrad_big<<<wb, kT, 0, s>>>(n, h1_.p, g1_.p, gz_.p, wpart_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_wsum<<<ceil_div(kBigPart, kT), kT, 0, s>>>(wpart_.p, wb, kBigPart, g_.p + kNetOffW2);
+  k_net_wsum<<<ceil_div(kBigPart, 16), 16 * kWsumGroups, 0, s>>>(wpart_.p, wb, kBigPart, g_.p + kNetOffW2);
   MGPBD_CHECK_LAUNCH();
-  k_net_xgrad<<<ceil_div(n, 32), 2 * kNetF, 0, s>>>(n, gz_.p, wt_.p, gself_.p, q_.p);
+  k_net_xgrad<<<ceil_div(n, kXgRows), kT, 0, s>>>(n, gz_.p, wt_.p, gself_.p, q_.p);
   MGPBD_CHECK_LAUNCH();
   k_net_hgrad<<<rowb, kT, 0, s>>>(g, ah_.p, gself_.p, q_.p, h1_.p, gz_.p);
   MGPBD_CHECK_LAUNCH();
   // layer 1
   k_net_wgrad_l1<<<wb, kT, 0, s>>>(n, u_.p, a1_.p, gz_.p, wpart_.p);
   MGPBD_CHECK_LAUNCH();
-  k_net_wsum<<<1, kT, 0, s>>>(wpart_.p, wb, 3 * kNetF, g_.p + kNetOffW1s);
+  k_net_wsum<<<ceil_div(3 * kNetF, 16), 16 * kWsumGroups, 0, s>>>(wpart_.p, wb, 3 * kNetF, g_.p + kNetOffW1s);
   MGPBD_CHECK_LAUNCH();
 }
 
@@ -795,7 +919,6 @@ void CoarseNet::loss_grad(const NetGraph& g, const float* samples, int32_t n_sam
   MGPBD_CUDA(cudaMemsetAsync(loss_dev, 0, sizeof(double), s));
   const float scale = (float)(1.0 / ((double)n * (double)S));
   const int ob = std::min(kMaxReduceBlocks, ceil_div(n, kT / 32));
-  const int rb = std::min(kMaxReduceBlocks, std::max(1, ceil_div(n, kT * 4)));
   auto sample = [&](int32_t k) {
     return samples + (int64_t)((first + (int64_t)k) % n_samples) * n;
   };
@@ -806,13 +929,22 @@ void CoarseNet::loss_grad(const NetGraph& g, const float* samples, int32_t n_sam
     k_net_squash<<<ceil_div(n, kT), kT, 0, s>>>(n, y_.p, wcap_.p, wv_.p, dw_.p);
     MGPBD_CHECK_LAUNCH();
     MGPBD_CUDA(cudaMemsetAsync(gy_.p, 0, sizeof(float) * n, s));
-    for (int32_t k = 0; k < S; ++k) {
-      k_net_sumsq<<<rb, kT, 0, s>>>(n, sample(k), g.diag_inv, part_.p);
+    const int sb = std::min(64, std::max(1, ceil_div(n, kT)));
+    const NetFields fields{samples, first % n_samples, n_samples};
+    if (S > sig_cap_) {
+      sigs_.alloc(S);
+      spart_.alloc((int64_t)S * 64);
+      sig_cap_ = S;
+    }
+    k_net_sumsq<<<dim3(sb, S), kT, 0, s>>>(n, fields, g.diag_inv, spart_.p);
+    MGPBD_CHECK_LAUNCH();
+    k_net_sigma<<<S, kT, 0, s>>>(spart_.p, sb, n, sigs_.p);
+    MGPBD_CHECK_LAUNCH();
+    for (int32_t k = 0; k < S; k += kNetSamples) {
+      const int ns = std::min(kNetSamples, S - k);
+      k_net_uv<<<ceil_div(n, kT), kT, 0, s>>>(g, fields, k, ns, sigs_.p, wv_.p, vs_.p, us_.p);
       MGPBD_CHECK_LAUNCH();
-      k_net_sum<<<1, kT, 0, s>>>(part_.p, rb, sumsq_.p + 1, 0);
-      MGPBD_CHECK_LAUNCH();
-      k_net_wloss<<<ob, kT, 0, s>>>(g, ah_.p, wv_.p, dw_.p, sample(k), sumsq_.p + 1, scale,
-                                    gy_.p, part_.p);
+      k_net_wloss<<<ob, kT, 0, s>>>(g, ah_.p, dw_.p, ns, vs_.p, us_.p, scale, gy_.p, part_.p);
       MGPBD_CHECK_LAUNCH();
       k_net_sum<<<1, kT, 0, s>>>(part_.p, ob, loss_dev, 1);
       MGPBD_CHECK_LAUNCH();

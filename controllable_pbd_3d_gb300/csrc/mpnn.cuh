@@ -56,6 +56,11 @@ struct NetGraph {
   const float* diag_inv = nullptr;
 };
 
+// scale of a field: sigma = sqrt(mean (S r)^2) and its inverse (0: r = 0)
+struct NetSigma {
+  float inv, sigma;
+};
+
 class CoarseNet {
  public:
   // Glorot-uniform weights from `seed`, zero biases.
@@ -95,7 +100,10 @@ class CoarseNet {
   DevBuf<__nv_bfloat16> wt_;  // W2^T then W3^T, each [64 out][128 in]
   int32_t cap_ = -1;
   // workspace (cap_ rows)
-  DevBuf<double> part_, sumsq_;
+  DevBuf<double> part_, spart_;
+  DevBuf<NetSigma> sigma_, sigs_;  // of the forward field, of a batch
+  int32_t sig_cap_ = 0;
+  DevBuf<float> vs_, us_;  // w u and u of eight samples side by side
   DevBuf<float> u_, a1_, y_, e_, h3_, gy_, gz_, gself_, q_, wpart_;
   DevBuf<float> ah_;    // Ah = S A S per nonzero, written by layer 1
   DevBuf<float> feat_;  // the feature field sqrt(diag A)
