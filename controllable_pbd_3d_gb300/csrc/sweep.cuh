@@ -15,13 +15,13 @@ namespace mgpbd {
 // How a matrix is spread over the cluster.  blocks == 0: it is not (it does
 // not fit into the blocks' shared memory).
 struct SweepPlan {
-  int32_t blocks = 0, lanes = 0;       // blocks of the cluster, lanes of a row
-  int32_t rows = 0, groups = 0, nx = 0;  // the most rows, 4-element groups and x of a block
+  int32_t blocks = 0, threads = 0, lanes = 0;  // of the cluster, a block, a row
+  int32_t rows = 0, steps = 0, nx = 0;  // the most rows, steps and x of a block
   int32_t smem = 0;
-  // first row of each block and the end, quads of x that a block receives,
-  // first group of each block; first group of each row in its block
-  DevBuf<int32_t> dev;
-  DevBuf<uint16_t> cols;  // columns of the groups, as positions in the block's x
+  DevBuf<int32_t> dev;    // first row of each block and the end; quads of x it receives
+  DevBuf<int32_t> step;   // first step of each task (a warp's rows)
+  DevBuf<int32_t> src;    // [step][lane][4]: element of the matrix, -1: padding
+  DevBuf<uint16_t> cols;  // and its column, as a byte offset in the block's x
   DevBuf<uint16_t> pos;   // where each block keeps a quad of rows (kSweepNone: nowhere)
 };
 constexpr uint16_t kSweepNone = 0xffff;
