@@ -98,6 +98,7 @@ class BodyBatch:
     self.per_body = fast_cheb if per_body is None else bool(per_body)
     if self.per_body:
       self.solver.set_bodies(self.vert_off, self.segments())
+      self.solver.set_body_compliance([b.compliance for b in self.bodies])
 
   def constraint_body(self) -> np.ndarray:
     """Body id of every constraint: one per tet (ARAP), or the volume

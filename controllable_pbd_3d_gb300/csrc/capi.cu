@@ -186,6 +186,11 @@ int mgpbd_set_bodies(mgpbd_handle h, int32_t n_bodies, const int32_t* vert_off, 
   return guarded([&] { h->impl.set_bodies(n_bodies, vert_off, n_segs, segs); });
 }
 
+int mgpbd_set_body_compliance(mgpbd_handle h, int32_t n_bodies, const float* compliance) {
+  if (!h) return MGPBD_EINVAL;
+  return guarded([&] { h->impl.set_body_compliance(n_bodies, compliance); });
+}
+
 int mgpbd_body_stats(mgpbd_handle h, int32_t n, int32_t* newton_iters, double* residual0,
                      double* residual, double* omega) {
   if (!h) return MGPBD_EINVAL;
@@ -702,15 +707,21 @@ int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32
                                int32_t n_blocks, int32_t cluster, int32_t threads,
                                int32_t smem_limit, const float* gradC, const float* invm,
                                const float* alpha, const float* x, double* y, int32_t* info) {
-  if (!t_i || nt <= 0 || n4 < 0 || n4 > nt || nv <= 0 || !x_ref || n_prob <= 0 || n_blocks <= 0 ||
+  if (!t_i || nt <= 0 || n4 < 0 || n4 > nt || nv <= 0 || !x_ref || n_prob <= 0 || n_blocks < 0 || (n_blocks == 0 && (!cluster || !prob)) ||
       n_blocks > (cluster ? mgpbd::kDMaxCluster : 255) || threads < 128 ||
       threads > mgpbd::kDMaxThreads || threads % 128 != 0 || !gradC || !invm || !alpha || !x || !y ||
       !info)
     return MGPBD_EINVAL;
   return guarded([&] {
     mgpbd::DcgPlan p;
-    mgpbd::require(mgpbd::build_dcg_plan(t_i, nt, n4, nv, x_ref, prob, n_prob, n_blocks, cluster != 0,
-                                         threads, smem_limit, p),
+    mgpbd::DcgPlaces places = mgpbd::dcg_places(n_prob, std::max(n_blocks, 1));
+    if (n_blocks == 0) {
+      std::vector<double> size(n_prob, 0.0);
+      for (int32_t c = 0; c < nt; ++c) size[prob[c]] += c < n4 ? 4.0 : 2.0;
+      places = mgpbd::dcg_place_bodies(size, {}, 2, 0, 0)[0];
+    }
+    mgpbd::require(mgpbd::build_dcg_plan(t_i, nt, n4, nv, x_ref, prob, places, cluster != 0, threads,
+                                         smem_limit, p),
                    MGPBD_ERANGE, "a block's vectors do not fit");
     mgpbd::dcg_plan_apply(p, gradC, invm, alpha, x, y);
     int32_t least = nt, most = 0;

@@ -280,13 +280,20 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   const int nthr = blockDim.x, nw = nthr / 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const bool syncw = wid == nw - 1;
-  const int prob = blockIdx.x / a.nblk, rank = blockIdx.x % a.nblk, G = a.nblk;
   if (tid < static_cast<int>(sizeof(DBlock) / 4))
     reinterpret_cast<int32_t*>(&s_B)[tid] = reinterpret_cast<const int32_t*>(a.d.blocks + blockIdx.x)[tid];
   const DWarp W = a.d.warps[blockIdx.x * nw + wid];
   __syncthreads();
   const DBlock& B = s_B;
   const int64_t NC = a.d.nc;
+  const int prob = CLUSTER ? B.prob : blockIdx.x / a.nblk, rank = CLUSTER ? B.rank : blockIdx.x % a.nblk;
+  const int G = CLUSTER ? B.size : a.nblk;
+  // the cluster's block that is the first of this problem
+  uint32_t base = 0;
+  if (CLUSTER) {
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(base));
+    base -= rank;
+  }
 
   // all of the SM's tensor memory: the block takes more than half of the
   // shared memory, so no second block of this kernel waits here for it
@@ -519,7 +526,8 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         for (int k = sub; k < others; k += 1 << vshift) {
           const uint32_t t = sm_i(a.o.tgt, (f.x >> 16) + k);
           const uint32_t to = smem_u32(s_dyn) + a.o.rbuf + 16 * ((gen & 1) * a.rmax + (t & 0xffff));
-          send_f4(map_rank(to, t >> 16), map_rank(smem_u32(&s_bar[gen & 1]), t >> 16), ax, ay, az);
+          send_f4(map_rank(to, base + (t >> 16)), map_rank(smem_u32(&s_bar[gen & 1]), base + (t >> 16)),
+                  ax, ay, az);
         }
       }
       if (sub == 0 && others > 0) {
@@ -592,7 +600,7 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         const double v = warp_sum_d(lane < nw ? s_red[k][lane] : 0.0);
         if (CLUSTER) {
           if (lane < G)
-            send_f64(map_rank(smem_u32(&s_sum[nsum & 1][k][rank]), lane), map_rank(sbar, lane), v);
+            send_f64(map_rank(smem_u32(&s_sum[nsum & 1][k][rank]), base + lane), map_rank(sbar, base + lane), v);
         } else if (lane == 0) {
           const unsigned long long u = __double_as_longlong(v);
           put_tagged(a.d.partials + ((nsum & 1) * 3 + k) * G + rank, static_cast<uint32_t>(u),
@@ -808,7 +816,7 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         const bool ok = cheb_interval(lmax, deg, a.lo_ratio, s_c1, s_c2, &theta, &it);
         if (!ok) status |= MGPBD_STATUS_NAN;
         s_it = it;
-        if (blockIdx.x == 0) {
+        if (prob == 0 && rank == 0) {
           ChebCoef& f = a.js->cf;
           for (int i = 0; i < kMaxCheb; ++i) {
             f.c1[i] = s_c1[i];
@@ -1106,7 +1114,7 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
     st->done = 1;
     st->maxiter = maxiter;
     st->body_runs = 1;
-    if (a.iters) a.iters[prob] = iters;
+    if (a.iters && prob >= 0) a.iters[prob] = iters;
     atomicMax(&st->iters, iters);
     if (status) atomicOr(reinterpret_cast<unsigned int*>(&st->status), status);
   }
@@ -1260,34 +1268,6 @@ int dcg_max_clusters(int size, int threads, int smem) {
   return n;
 }
 
-// A body's CG takes about side x (23 us + 1.9 us per 1000 entries a block,
-// twice that beyond the 12k entries that stay on the chip) on its cluster
-// (measured: cubes of 10 to 20 hexes on 8 and 16 blocks; the iterations grow
-// with the side).  The clusters that are resident at once take the bodies
-// largest first; the size with the shortest schedule is tried first.  16
-// bodies of 6..18 hexes a side: 144 / 109 / 204 ms a substep on clusters of
-// 16 / 8 / 4, 279 ms in lockstep over the whole pack.
-std::vector<std::pair<int32_t, bool>> dcg_body_shapes(const std::vector<double>& entries) {
-  std::vector<std::pair<double, int32_t>> cost;
-  for (int32_t size : {16, 8, 4}) {
-    const int n = dcg_max_clusters(size, kDMaxThreads, dcg_smem_limit());
-    if (n < 1) continue;
-    std::vector<double> t;
-    for (double e : entries) {
-      const double per = e / size / 1000.0;
-      t.push_back(std::cbrt(e) * (23.0 + 1.9 * per + 1.9 * std::max(0.0, per - 12.0)));
-    }
-    std::sort(t.rbegin(), t.rend());
-    std::vector<double> busy(n, 0.0);
-    for (double v : t) *std::min_element(busy.begin(), busy.end()) += v;
-    cost.push_back({*std::max_element(busy.begin(), busy.end()), size});
-  }
-  std::sort(cost.begin(), cost.end());
-  std::vector<std::pair<int32_t, bool>> r;
-  for (const auto& c : cost) r.push_back({c.second, true});
-  return r;
-}
-
 void launch_dcg_pack(const JView& j, const DcgDev& d, int64_t n_rows, cudaStream_t s) {
   const int64_t n = std::max<int64_t>(32 * n_rows, d.nc);
   MGPBD_CUDA(cudaMemsetAsync(d.gflag, 0, sizeof(uint32_t), s));
@@ -1344,14 +1324,14 @@ void launch_dcg(const JView& j, const JcgVecs& v, const DcgPlan& plan, const Dcg
     MGPBD_CUDA(cudaMemsetAsync(d.exch, 0, sizeof(float4) * (2 * d.n_slots + 6 * plan.nblk), s));
   const void* fn = kernel_of(plan.cluster);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(plan.nprob * plan.nblk);
+  cfg.gridDim = dim3(plan.nblk);
   cfg.blockDim = dim3(plan.threads);
   cfg.dynamicSmemBytes = plan.smem;
   cfg.stream = s;
   cudaLaunchAttribute at;
   if (plan.cluster) {
     at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = plan.nblk;
+    at.val.clusterDim.x = plan.csize;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
   } else {
     at.id = cudaLaunchAttributeCooperative;

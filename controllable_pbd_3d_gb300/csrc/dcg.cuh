@@ -73,9 +73,6 @@ constexpr double kDClusterEntries = 120e3;
 // besides the constraints.  us per CG iteration at 512 / 768 threads, 600
 // constraints a block 39.4 / 41.7, 1600: 45.0 / 46.2, 4700: 70.8 / 67.2.
 constexpr double kDWideConstraints = 3000.0;
-// Packed bodies: the cluster sizes to try, the best first, for bodies of the
-// given numbers of entries.
-std::vector<std::pair<int32_t, bool>> dcg_body_shapes(const std::vector<double>& entries);
 
 // Dynamic shared memory a block of the kernel may use on this device (and the
 // kernel's attributes set for it): before a plan is built or launched there.

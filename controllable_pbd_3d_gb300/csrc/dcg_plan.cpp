@@ -3,6 +3,9 @@
 #include "dcg_plan.h"
 
 #include <algorithm>
+#include <array>
+#include <cmath>
+#include <numeric>
 
 namespace mgpbd {
 
@@ -77,25 +80,165 @@ void bisect(Item* it, int64_t lo, int64_t hi, int n, int64_t* out, int32_t n4) {
 
 }  // namespace
 
+DcgPlaces dcg_places(int32_t nprob, int32_t nblk) {
+  DcgPlaces p;
+  p.cluster = nblk;
+  p.blocks = nprob * nblk;
+  p.size.assign(nprob, nblk);
+  for (int32_t k = 0; k < nprob; ++k) p.first.push_back(k * nblk);
+  return p;
+}
+
+// A body's CG takes its iterations x (23 us + 1.9 us per 1000 entries a block,
+// twice that beyond the 12k entries that stay on the chip) (measured: cubes of
+// 10 to 20 hexes on 8 and 16 blocks).  The iterations follow from the softness
+// (alpha~ by a unit's J W J^T) and, of stiff bodies, from the side: cubes of 6 /
+// 12 / 17 hexes need 1682 / 2812 / 3309 in two solves at 0.009, 915 / 1177 / 1152
+// at 0.09, 364 / 390 / 391 at 0.9.  Where the softness is not known the sides
+// have to do.  An arrangement is judged by its mean over kHardness draws of a
+// factor for each body: up to 1.2 for what the formula misses, 2 for an unknown
+// softness.  The clusters that are resident at once take the bodies longest
+// first.  A cluster of 16 holds one body, two of 8 blocks or four of 4, so that
+// the bodies that everything else waits for can have more SMs than the others:
+// 16 bodies of 6..18 hexes a side, compliances 1e-7..1e-5, three draws: 102 / 85
+// / 111 ms a substep, on clusters of 8 each 132 / 111 / 169; 24 bodies of 8..17:
+// 123 / 116 / 110 and 149 / 167 / 161.
+std::vector<DcgPlaces> dcg_place_bodies(const std::vector<double>& entries,
+                                        const std::vector<double>& softness, int n16, int n8, int n4) {
+  constexpr int kHardness = 16;
+  const int32_t nb = static_cast<int32_t>(entries.size());
+  const bool known = !softness.empty();
+  std::vector<double> its(nb);
+  for (int32_t k = 0; k < nb; ++k) {
+    const double side = std::cbrt(entries[k] / 36.0);  // hexes, length + volume
+    its[k] = known ? 1.0 / (std::pow(std::max(softness[k], 1e-12), 0.46) / 372.0 + 1.0 / (97.0 * side * side))
+                   : 100.0 * side;
+  }
+  // body k on 16, 8 and 4 blocks.  All blocks have the memory layout that the
+  // fullest one needs, so none is to be fuller than the largest body on 8.
+  const double fullest = std::max(12.0, *std::max_element(entries.begin(), entries.end()) / 8000.0);
+  auto time_of = [&](int32_t k, int q) {
+    const double per = entries[k] / (16 >> q) / 1000.0;
+    if (q > 0 && per > fullest) return 1e6 * its[k];
+    return its[k] * (23.0 + 1.9 * per + 1.9 * std::max(0.0, per - 12.0));
+  };
+  std::vector<int32_t> order(nb);  // longest first
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return time_of(a, 1) > time_of(b, 1); });
+  std::vector<std::array<double, kHardness>> hard(nb);
+  uint32_t seed = 1;
+  for (auto& h : hard)
+    for (double& v : h) {
+      seed = seed * 1664525u + 1013904223u;
+      v = std::exp2(((seed >> 8) * (2.0 / (1 << 24)) - 1.0) * (known ? 0.25 : 1.0));
+    }
+  std::vector<std::array<double, 3>> time(nb);
+  for (int32_t i = 0; i < nb; ++i)
+    for (int q = 0; q < 3; ++q) time[i][q] = time_of(order[i], q);
+  struct Job {  // a cluster's bodies: `n` from the at-th longest, on 16 >> q blocks each
+    double t;
+    int32_t at, n, q;
+  };
+  // clusters of 16 >> q0: the first `one` bodies have one each, the next `two`
+  // half a one, the rest a quarter
+  auto jobs_of = [&](int q0, int32_t one, int32_t two) {
+    std::vector<Job> jobs;
+    for (int32_t i = 0; i < nb;) {
+      const int half = i < one ? 0 : i < one + two ? 1 : 2;
+      const int32_t end = i < one ? one : i < one + two ? one + two : nb;
+      const Job j{time[i][q0 + half], i, std::min<int32_t>(1 << half, end - i), q0 + half};
+      jobs.push_back(j);
+      i += j.n;
+    }
+    std::stable_sort(jobs.begin(), jobs.end(), [](const Job& a, const Job& b) { return a.t > b.t; });
+    return jobs;
+  };
+  // the longest queue when `resident` clusters take the jobs in their order
+  auto cost = [&](const std::vector<Job>& jobs, int resident) {
+    double sum = 0.0;
+    std::vector<double> busy;
+    for (int h = 0; h < kHardness; ++h) {
+      busy.assign(resident, 0.0);
+      for (const Job& j : jobs) {
+        double t = 0.0;
+        for (int32_t k = 0; k < j.n; ++k) t = std::max(t, time[j.at + k][j.q] * hard[j.at + k][h]);
+        *std::min_element(busy.begin(), busy.end()) += t;
+      }
+      sum += *std::max_element(busy.begin(), busy.end());
+    }
+    return sum / kHardness;
+  };
+  auto place = [&](int q0, const std::vector<Job>& jobs) {
+    const int c = 16 >> q0;
+    DcgPlaces p;
+    p.cluster = c;
+    p.blocks = c * static_cast<int32_t>(jobs.size());
+    p.first.resize(nb);
+    p.size.resize(nb);
+    for (size_t b = 0; b < jobs.size(); ++b)
+      for (int32_t k = 0; k < jobs[b].n; ++k) {
+        const int32_t body = order[jobs[b].at + k], size = 16 >> jobs[b].q;
+        p.first[body] = c * static_cast<int32_t>(b) + k * size;
+        p.size[body] = size;
+      }
+    return p;
+  };
+  std::vector<std::pair<double, DcgPlaces>> all;
+  if (n16 > 0) {
+    double least = 1e300;
+    std::vector<Job> best;
+    for (int32_t a = 0; a <= std::min(nb, 48); ++a)
+      for (int32_t b = 0; b <= std::min(nb - a, 48); ++b) {
+        const std::vector<Job> jobs = jobs_of(0, a, b);
+        const double v = cost(jobs, n16);
+        if (v < least) {
+          least = v;
+          best = jobs;
+        }
+      }
+    all.push_back({least, place(0, best)});
+  }
+  for (int q = 1; q < 3; ++q)
+    if (const int n = q == 1 ? n8 : n4; n > 0) {
+      std::vector<Job> jobs;
+      for (int32_t i = 0; i < nb; ++i) jobs.push_back({time[i][q], i, 1, q});
+      all.push_back({cost(jobs, n), place(q, jobs)});
+    }
+  std::stable_sort(all.begin(), all.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+  std::vector<DcgPlaces> r;
+  for (auto& a : all) r.push_back(std::move(a.second));
+  if (n16 > 0) r.push_back(place(0, jobs_of(0, nb, 0)));  // (the most memory a body)
+  return r;
+}
+
 bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, const float* x_ref,
-                    const int32_t* prob, int32_t nprob, int32_t nblk, bool cluster,
-                    int threads, int32_t smem_limit, DcgPlan& plan) {
+                    const int32_t* prob, const DcgPlaces& places, bool cluster, int threads,
+                    int32_t smem_limit, DcgPlan& plan) {
   plan = DcgPlan();
   plan.threads = threads;
+  const int32_t nprob = static_cast<int32_t>(places.first.size());
   plan.nprob = nprob;
-  plan.nblk = nblk;
+  plan.nblk = places.blocks;
+  plan.csize = places.cluster;
   plan.cluster = cluster;
-  const int64_t nb = static_cast<int64_t>(nprob) * nblk;
+  const int64_t nb = places.blocks;
   const int warps = threads / 32;
   auto slots = [n4](int32_t c) { return c < n4 ? 4 : 2; };
 
-  // centroids, grouped by problem
-  std::vector<int64_t> pbeg(nprob + 1, 0);
-  for (int32_t c = 0; c < nt; ++c) pbeg[(prob ? prob[c] : 0) + 1]++;
-  for (int32_t k = 0; k < nprob; ++k) pbeg[k + 1] += pbeg[k];
+  // centroids, grouped by problem in the order of their blocks
+  std::vector<int32_t> order(nprob);
+  std::iota(order.begin(), order.end(), 0);
+  std::sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return places.first[a] < places.first[b]; });
+  std::vector<int64_t> count(nprob, 0), pbeg(nprob), pend(nprob);
+  for (int32_t c = 0; c < nt; ++c) count[prob ? prob[c] : 0]++;
+  int64_t sum = 0;
+  for (int32_t k : order) {
+    pbeg[k] = sum;
+    pend[k] = sum += count[k];
+  }
   std::vector<Item> items(nt);
   {
-    std::vector<int64_t> cur(pbeg.begin(), pbeg.end() - 1);
+    std::vector<int64_t> cur(pbeg);
     std::vector<int64_t> at(nt);
     for (int32_t c = 0; c < nt; ++c) at[c] = cur[prob ? prob[c] : 0]++;
 #pragma omp parallel for schedule(static)
@@ -110,19 +253,31 @@ bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, cons
       }
     }
   }
+  plan.blocks.assign(nb, DBlock());
+  for (DBlock& B : plan.blocks) {
+    B.prob = -1;
+    B.size = 1;
+  }
+  for (int32_t k = 0; k < nprob; ++k)
+    for (int32_t r = 0; r < places.size[k]; ++r) {
+      DBlock& B = plan.blocks[places.first[k] + r];
+      B.prob = k;
+      B.rank = r;
+      B.size = places.size[k];
+    }
   std::vector<int64_t> part(nb + 1, nt);
 #pragma omp parallel
 #pragma omp single
   for (int32_t k = 0; k < nprob; ++k) {
 #pragma omp task
-    bisect(items.data(), pbeg[k], pbeg[k + 1], nblk, part.data() + static_cast<int64_t>(k) * nblk,
-           n4);
+    bisect(items.data(), pbeg[k], pend[k], places.size[k], part.data() + places.first[k], n4);
   }
   part[nb] = nt;
+  for (int64_t b = nb - 1; b >= 0; --b)
+    if (plan.blocks[b].prob < 0) part[b] = part[b + 1];
 
   // each block's constraints (4-slot ones first, ascending) and vertices
   plan.perm.resize(nt);
-  plan.blocks.resize(nb);
   std::vector<std::vector<int32_t>> verts(nb);
 #pragma omp parallel for schedule(dynamic, 1)
   for (int64_t b = 0; b < nb; ++b) {
@@ -131,7 +286,6 @@ bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, cons
     for (int32_t i = 0; i < n; ++i) pm[i] = items[part[b] + i].id;
     std::sort(pm, pm + n);
     DBlock& B = plan.blocks[b];
-    B = DBlock();
     B.c0 = static_cast<int32_t>(part[b]);
     B.nT = static_cast<int32_t>(std::lower_bound(pm, pm + n, n4) - pm);
     B.nE = n - B.nT;
@@ -363,7 +517,7 @@ bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, cons
               if (j == own[b][v]) continue;
               // the slots of block who[f + j] leave out its own place j
               const int32_t slot = recv[f + j] + (own[b][v] < j ? own[b][v] : own[b][v] - 1);
-              L.tgt.push_back(static_cast<uint32_t>(who[f + j] % nblk) << 16 | static_cast<uint32_t>(slot));
+              L.tgt.push_back(static_cast<uint32_t>(plan.blocks[who[f + j]].rank) << 16 | static_cast<uint32_t>(slot));
             }
           }
           L.pos_info[2LL * p] = at0;
@@ -522,7 +676,7 @@ void dcg_plan_apply(const DcgPlan& P, const float* gradC, const float* invm, con
           } else {
             for (uint32_t j = 0; j + 1 < n >> 8; ++j) {
               const uint32_t t = P.tgt[B.t0 + (to >> 16) + j];
-              rbuf[b / P.nblk * P.nblk + (t >> 16)][t & 0xffff] = a;
+              rbuf[b - B.rank + (t >> 16)][t & 0xffff] = a;
             }
           }
         }

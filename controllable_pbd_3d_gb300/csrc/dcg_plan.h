@@ -25,7 +25,23 @@ struct DBlock {
   int32_t s0, nsl;           // slices from s0
   int32_t r0, nrows;         // rows from r0
   int32_t t0, ntgt, nrecv;   // cluster: its sends from t0, partials it receives per exchange
+  int32_t prob, rank, size;  // its problem (-1: none), its place among that problem's blocks, how many
 };
+
+// Where the blocks of each problem are: size[k] of them from block first[k], of
+// `blocks` in clusters of `cluster`.  The blocks that no problem has only meet
+// the rest of their cluster.
+struct DcgPlaces {
+  int32_t cluster = 0, blocks = 0;
+  std::vector<int32_t> first, size;
+};
+
+// Arrangements of independent bodies, by the number of vertex entries of each
+// (and how soft it is, or nothing), on clusters of 16, 8 and 4 blocks, of which
+// n16, n8 and n4 are resident at once (0: none): the one whose schedule should
+// be shortest first.
+std::vector<DcgPlaces> dcg_place_bodies(const std::vector<double>& entries,
+                                        const std::vector<double>& softness, int n16, int n8, int n4);
 
 // The vertex sums of one warp: slices s .. p - 1 of shared vertices, p .. e - 1
 // of private ones (from the block's s0); its rows from row (from r0), the
@@ -34,10 +50,10 @@ struct DWarp {
   int32_t s, p, e, row, rows, srow, held;
 };
 
-// Host-built partition of one or several independent problems (bodies),
-// nblk blocks each.
+// Host-built partition of one or several independent problems (bodies).
 struct DcgPlan {
-  int32_t nprob = 0, nblk = 0;
+  int32_t nprob = 0, nblk = 0;  // blocks in all
+  int32_t csize = 0;            // blocks of a cluster
   bool cluster = false;  // blocks of a problem form one thread-block cluster
   bool onchip = false;   // every block's operator fits in tensor and shared memory
   int32_t threads = kDMaxThreads;  // per block, a multiple of 128
@@ -47,7 +63,7 @@ struct DcgPlan {
   int32_t cmax = 0, posmax = 0, possmax = 0, slmax = 0, tmax = 0, rmax = 0;  // largest counts of a block
   int64_t n_rows = 0;
   int64_t n_slots = 0;   // grid: exchange slots
-  std::vector<DBlock> blocks;     // nprob * nblk
+  std::vector<DBlock> blocks;     // nblk
   std::vector<DWarp> warps;       // threads / 32 per block
   std::vector<int32_t> perm;      // (nc) constraint of each plan position
   std::vector<uint16_t> ti;       // (nc, 4) byte offsets of its vertices' u in its block
@@ -85,8 +101,10 @@ inline DcgSmem dcg_smem_parts(const DcgPlan& p) {
 // constraint c (null: one problem).  Returns false when some block's vectors
 // do not fit (the plan is then unusable).
 bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, const float* x_ref,
-                    const int32_t* prob, int32_t nprob, int32_t nblk, bool cluster,
-                    int threads, int32_t smem_limit, DcgPlan& plan);
+                    const int32_t* prob, const DcgPlaces& places, bool cluster, int threads,
+                    int32_t smem_limit, DcgPlan& plan);
+// the places of one problem on nblk blocks, of nprob problems on nblk each
+DcgPlaces dcg_places(int32_t nprob, int32_t nblk);
 
 // y = (J W J^T + alpha~) x in float64 by way of the plan's arrays, as the
 // kernel goes (tests)

@@ -476,7 +476,7 @@ void Solver::init() {
   dcg_ready_ = false;
   if (cheb() && p_.persistent == 1) build_dcg(t_host);
   if (dcg_ready_) {
-    stats_.cg_grid = dplan_.nprob * dplan_.nblk;
+    stats_.cg_grid = dplan_.nblk;
   }
 }
 
@@ -494,8 +494,8 @@ void Solver::build_dcg(const std::vector<int32_t>& t_host) {
   std::vector<int32_t> body;
   const bool per_body = nb_ > 0 && p_.body_cg;
   const double entries = 4.0 * n4_ + 2.0 * (nt_ - n4_);
-  // candidates in order of preference: blocks per problem, cluster or grid
-  std::vector<std::pair<int32_t, bool>> shapes;
+  // candidates in order of preference: places, cluster or grid
+  std::vector<std::pair<DcgPlaces, bool>> shapes;
   if (per_body) {
     body.resize(nt_);
     std::vector<double> size(nb_, 0.0);
@@ -505,18 +505,32 @@ void Solver::build_dcg(const std::vector<int32_t>& t_host) {
         size[body[t]] += t < n4_ ? 4.0 : 2.0;
       }
     prob = body.data();
-    shapes = dcg_body_shapes(size);
+    auto resident = [&](int c) { return dcg_max_clusters(c, kDMaxThreads, limit); };
+    std::vector<double> softness;
+    if (!body_compliance_.empty()) {
+      std::vector<float> w(nv_);
+      MGPBD_CUDA(cudaMemcpyAsync(w.data(), invm_, sizeof(float) * w.size(), cudaMemcpyDeviceToHost, s));
+      MGPBD_CUDA(cudaStreamSynchronize(s));
+      for (int32_t b = 0; b < nb_; ++b) {
+        double sum = 0.0;
+        for (int32_t v = body_vert_off_[b]; v < body_vert_off_[b + 1]; ++v) sum += w[v];
+        const double mean = sum / (body_vert_off_[b + 1] - body_vert_off_[b]);
+        softness.push_back(body_compliance_[b] / (p_.dt * p_.dt) / std::max(mean, 1e-30));
+      }
+    }
+    for (DcgPlaces& p : dcg_place_bodies(size, softness, resident(16), resident(8), resident(4)))
+      shapes.push_back({std::move(p), true});
   } else {
-    if (entries <= kDClusterEntries) shapes.push_back({kDMaxCluster, true});
-    shapes.push_back({std::min(sms, 255), false});
+    if (entries <= kDClusterEntries) shapes.push_back({dcg_places(1, kDMaxCluster), true});
+    shapes.push_back({dcg_places(1, std::min(sms, 255)), false});
   }
   bool built = false;
   for (const auto& sh : shapes) {
-    const double per_block = static_cast<double>(nt_) / ((per_body ? nb_ : 1) * sh.first);
+    const double per_block = static_cast<double>(nt_) / sh.first.blocks;
     const int threads = per_body || per_block >= kDWideConstraints ? kDMaxThreads : 512;
-    if (build_dcg_plan(t_host.data(), nt_, n4_, nv_, xr.data(), prob, per_body ? nb_ : 1, sh.first,
-                       sh.second, threads, limit, dplan_) &&
-        (!sh.second || dcg_max_clusters(sh.first, threads, dplan_.smem) >= 1)) {
+    if (build_dcg_plan(t_host.data(), nt_, n4_, nv_, xr.data(), prob, sh.first, sh.second, threads,
+                       limit, dplan_) &&
+        (!sh.second || dcg_max_clusters(sh.first.cluster, threads, dplan_.smem) >= 1)) {
       built = true;
       break;
     }
@@ -1730,6 +1744,7 @@ constexpr int kBodyTrials = 10;       // line-search steps 1, 1/2, ..., 1/512
 void Solver::set_bodies(int32_t n_bodies, const int32_t* vert_off, int32_t n_segs,
                         const int32_t* segs) {
   require(x_ && t_i_ && !matrix_mode_, MGPBD_ESTATE, "mgpbd_set_mesh must come before mgpbd_set_bodies");
+  body_compliance_.clear();
   if (n_bodies == 0) {
     nb_ = 0;
     inited_ = false;
@@ -1756,6 +1771,15 @@ void Solver::set_bodies(int32_t n_bodies, const int32_t* vert_off, int32_t n_seg
   nb_ = n_bodies;
   body_vert_off_.assign(vert_off, vert_off + n_bodies + 1);
   body_segs_.assign(segs, segs + 3LL * n_segs);
+  inited_ = false;
+}
+
+void Solver::set_body_compliance(int32_t n_bodies, const float* compliance) {
+  require(nb_ > 0, MGPBD_ESTATE, "mgpbd_set_bodies must come before mgpbd_set_body_compliance");
+  require(n_bodies == nb_ && compliance, MGPBD_EINVAL, "body compliances: one per body");
+  for (int32_t b = 0; b < nb_; ++b)
+    require(compliance[b] >= 0.0f && std::isfinite(compliance[b]), MGPBD_EINVAL, "body compliances: negative or not finite");
+  body_compliance_.assign(compliance, compliance + nb_);
   inited_ = false;
 }
 

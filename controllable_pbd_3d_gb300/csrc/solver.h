@@ -84,6 +84,7 @@ class Solver {
   // segs[3k+2], covering [0, nt) in order): each body gets its own Newton
   // loop (residual, stopping test, line-search step) over one shared
   // block-diagonal CG solve per Newton iteration.  FAST Chebyshev only.
+  void set_body_compliance(int32_t n_bodies, const float* compliance);
   void set_bodies(int32_t n_bodies, const int32_t* vert_off, int32_t n_segs, const int32_t* segs);
   int32_t n_bodies() const { return nb_; }
   // per body: Newton iterations, first and last residual, last line-search
@@ -230,6 +231,7 @@ class Solver {
   bool warm_next_ = false;
   // packed bodies (set_bodies)
   int32_t nb_ = 0;
+  std::vector<float> body_compliance_;  // empty: not told
   std::vector<int32_t> body_vert_off_, body_segs_, chunk_body_;
   DevBuf<int32_t> chunks_, cons_body_, vert_body_, body_active_;
   DevBuf<float> body_omega_;

@@ -283,6 +283,14 @@ class MGPBDSolverGPU:
     self.n_bodies = len(vo) - 1
     self._inited = False
 
+  def set_body_compliance(self, compliance):
+    """The bodies' compliances, as a hint for how they share the SMs (a stiff
+    body's CG needs more iterations).  After set_bodies, before init()."""
+    c = np.ascontiguousarray(compliance, np.float32)
+    N.check(self._lib.mgpbd_set_body_compliance(self._h, len(c), c.ctypes.data),
+            'mgpbd_set_body_compliance')
+    self._inited = False
+
   def body_stats(self) -> dict:
     """Per body: Newton iterations, first / last residual, last step."""
     n = self.n_bodies

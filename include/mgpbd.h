@@ -331,6 +331,13 @@ int mgpbd_set_constraint_types(mgpbd_handle h, const int32_t* types);
  * No counterpart in the reference. */
 int mgpbd_set_bodies(mgpbd_handle h, int32_t n_bodies, const int32_t* vert_off, int32_t n_segs,
                      const int32_t* segs);
+
+/* How soft each body will be (its XPBD compliance), between mgpbd_set_bodies
+ * and mgpbd_init: a hint, from which the per-body CG arranges the bodies on
+ * the SMs (stiff bodies need more iterations).  Results do not depend on it
+ * but for the rounding of another partition; the compliances that count are
+ * those of the alpha~ view. */
+int mgpbd_set_body_compliance(mgpbd_handle h, int32_t n_bodies, const float* compliance);
 /* Per body (n = n_bodies entries each, NULL to skip): Newton iterations,
  * first and last residual norm, last line-search step of the last solve. */
 int mgpbd_body_stats(mgpbd_handle h, int32_t n, int32_t* newton_iters, double* residual0,
@@ -637,7 +644,8 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
  * the persistent dual CG runs on: nt constraints t_i (nt,4), the length
  * constraints from n4 on, rest positions x_ref (nv,3), prob (nt, or NULL) the
  * body of each of n_prob bodies, n_blocks blocks each (cluster: exchanging
- * within a cluster), `threads` a block, smem_limit bytes of shared memory.
+ * within a cluster; 0: bodies of several sizes share clusters of 16, two of
+ * which are resident), `threads` a block, smem_limit bytes of shared memory.
  * info (6): whether every block's operator stays on the chip, shared memory a
  * block, rows in it, rounds of 4-slot constraints in tensor memory, fewest
  * and most vertex entries of a block.  Host arrays; MGPBD_ERANGE when a

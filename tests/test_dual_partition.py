@@ -101,8 +101,8 @@ def test_plan_of_several_bodies_and_short_memory():
   alpha = rng.random(len(c)).astype(np.float32)
   x = rng.standard_normal(len(c)).astype(np.float32)
   ref, size = apply64(c, n4, g, w, alpha, x)
-  for smem, fits in ((SMEM, True), (20000, True), (3000, False)):
-    rc, y, info = run_plan(xr, c, n4, prob, 4, 4, True, 256, smem, g, w, alpha, x)
+  for smem, fits, blocks in ((SMEM, True, 4), (SMEM, True, 0), (20000, True, 4), (3000, False, 4)):
+    rc, y, info = run_plan(xr, c, n4, prob, 4, blocks, True, 256, smem, g, w, alpha, x)
     assert (rc == 0) == fits
     if not fits:
       assert rc == -6  # MGPBD_ERANGE
