@@ -78,7 +78,7 @@ int mgpbd_xpbd_set_mesh(mgpbd_xpbd_handle h, float* x, const float* x_ref, const
 /* preupdate_cons (:40-42): both multipliers to zero */
 int mgpbd_xpbd_preupdate(mgpbd_xpbd_handle h);
 /* update_cons (:44-52), n_passes times.  Asynchronous on the handle's
- * stream; a grid barrier of the colour kernel that gave up is reported by a
+ * stream; a wait of the colour kernel that gave up is reported by a
  * later call, or by mgpbd_xpbd_synchronize. */
 int mgpbd_xpbd_update(mgpbd_xpbd_handle h, int32_t n_passes);
 /* waits for the last update and reports its status */
