@@ -80,7 +80,7 @@ struct DArgs {
   double tol_abs, tol_rel, lo_ratio;
   int32_t estimate;  // 1: the Chebyshev interval is estimated first, 0: from js
   int32_t maxiter, degree, warm, per_problem, unit_dinv;
-  int32_t nblk, nprob, rmax, kT, kE;
+  int32_t nblk, nprob, rmax, kT, kE;  // kT, kE: of every block of a grid
   DcgSmem o;  // byte offsets of the shared-memory parts (u is at 0)
   unsigned long long spin_ns;
 };
@@ -346,14 +346,15 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   }
   general = __syncthreads_or(general);
   // (the barrier also orders the allocation's address before its use)
+  const int colT = CLUSTER ? B.kT : a.kT, colE = CLUSTER ? B.kE : a.kE;
   const uint32_t tm0 = s_tmem + (static_cast<uint32_t>(wid & 3) << 21) +
-                       static_cast<uint32_t>(wid >> 2) * (16 * a.kT + 8 * a.kE);
-  const uint32_t tme = tm0 + 16 * a.kT;
+                       static_cast<uint32_t>(wid >> 2) * (16 * colT + 8 * colE);
+  const uint32_t tme = tm0 + 16 * colT;
 
   // in tensor memory: constraints below nTr / nEr (no 4-slot one when some
   // slot-0 gradient is not minus the sum of the others), in kT / kE rounds
   const int nT = B.nT, nE = B.nE, nC = nT + nE;
-  const int nTr = *a.d.gflag ? 0 : min(nT, a.kT * nthr), nEr = min(nE, a.kE * nthr);
+  const int nTr = *a.d.gflag ? 0 : min(nT, colT * nthr), nEr = min(nE, colE * nthr);
   // rounds in which this warp has some
   const int kT = max(0, (nTr - 32 * wid + nthr - 1) / nthr);
   const int kE = max(0, (nEr - 32 * wid + nthr - 1) / nthr);

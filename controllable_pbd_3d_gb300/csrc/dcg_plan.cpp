@@ -100,9 +100,9 @@ DcgPlaces dcg_places(int32_t nprob, int32_t nblk) {
 // softness.  The clusters that are resident at once take the bodies longest
 // first.  A cluster of 16 holds one body, two of 8 blocks or four of 4, so that
 // the bodies that everything else waits for can have more SMs than the others:
-// 16 bodies of 6..18 hexes a side, compliances 1e-7..1e-5, three draws: 102 / 85
-// / 111 ms a substep, on clusters of 8 each 132 / 111 / 169; 24 bodies of 8..17:
-// 123 / 116 / 110 and 149 / 167 / 161.
+// 16 bodies of 6..18 hexes a side, compliances 1e-7..1e-5, three draws: 93 / 83
+// / 109 ms a substep, on clusters of 8 each 132 / 111 / 169; 24 bodies of 8..17:
+// 105 / 114 / 99 and 149 / 167 / 161.
 std::vector<DcgPlaces> dcg_place_bodies(const std::vector<double>& entries,
                                         const std::vector<double>& softness, int n16, int n8, int n4) {
   constexpr int kHardness = 16;
@@ -590,23 +590,34 @@ bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, cons
   plan.warps.resize(nb * warps);
   plan.row_ent.resize(32 * nr);
   plan.row_idx.resize(32 * nr);
-  // rounds of constraints in tensor memory: as many as the blocks need of
-  // both kinds, cut to the columns a warp gets (4-slot ones, which save
-  // more, first)
+  // rounds of constraints in tensor memory: as many as the block needs of both
+  // kinds, cut to the columns a warp gets (4-slot ones, which save more, first)
   const int cols = kDColumns / (threads / 128);
-  int32_t rmax = 0, needT = 0, needE = 0;
+  // A grid's blocks are alike and have the fullest one's rounds, which the
+  // kernel then reads from its arguments (from the block, 40^3 takes 67.7 ms
+  // instead of 64.0); packed bodies are not (16 of them 102 -> 93 ms, 24 123 ->
+  // 105).
+  int32_t rmax = 0, mostT = 0, mostE = 0;
   for (const DBlock& B : plan.blocks) {
     rmax = std::max(rmax, B.nrows);
-    needT = std::max(needT, (B.nT + threads - 1) / threads);
-    needE = std::max(needE, (B.nE + threads - 1) / threads);
+    mostT = std::max(mostT, (B.nT + threads - 1) / threads);
+    mostE = std::max(mostE, (B.nE + threads - 1) / threads);
   }
-  plan.kT = std::min(needT, cols / 16);
-  plan.kE = std::min(needE, (cols - 16 * plan.kT) / 8);
+  bool held = true;
+  for (DBlock& B : plan.blocks) {
+    const int32_t needT = cluster ? (B.nT + threads - 1) / threads : mostT;
+    const int32_t needE = cluster ? (B.nE + threads - 1) / threads : mostE;
+    B.kT = std::min(needT, cols / 16);
+    B.kE = std::min(needE, (cols - 16 * B.kT) / 8);
+    held = held && B.kT == needT && B.kE == needE;
+    plan.kT = std::max(plan.kT, B.kT);
+    plan.kE = std::max(plan.kE, B.kE);
+  }
   // shared memory: the vectors and tables, the rest holds rows
   const DcgSmem o = dcg_smem_parts(plan);
   if (o.rows > smem_limit) return false;
   plan.srows = std::min(rmax, (smem_limit - o.rows) / kDRow);
-  plan.onchip = plan.kT == needT && plan.kE == needE && plan.srows == rmax;
+  plan.onchip = held && plan.srows == rmax;
   plan.smem = std::max(o.rows + plan.srows * kDRow, kDMinSmem);
   // the same share of every warp's rows
   for (int64_t b = 0; b < nb; ++b) {

@@ -26,6 +26,7 @@ struct DBlock {
   int32_t r0, nrows;         // rows from r0
   int32_t t0, ntgt, nrecv;   // cluster: its sends from t0, partials it receives per exchange
   int32_t prob, rank, size;  // its problem (-1: none), its place among that problem's blocks, how many
+  int32_t kT, kE;            // 4-slot / length constraints a thread keeps in tensor memory
 };
 
 // Where the blocks of each problem are: size[k] of them from block first[k], of
@@ -57,7 +58,7 @@ struct DcgPlan {
   bool cluster = false;  // blocks of a problem form one thread-block cluster
   bool onchip = false;   // every block's operator fits in tensor and shared memory
   int32_t threads = kDMaxThreads;  // per block, a multiple of 128
-  int32_t kT = 0, kE = 0;  // 4-slot / length constraints a thread keeps in tensor memory
+  int32_t kT = 0, kE = 0;  // the most of DBlock::kT, kE
   int32_t srows = 0;     // rows a block keeps in shared memory
   int32_t smem = 0;      // dynamic shared memory per block
   int32_t cmax = 0, posmax = 0, possmax = 0, slmax = 0, tmax = 0, rmax = 0;  // largest counts of a block
