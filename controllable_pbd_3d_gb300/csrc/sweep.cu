@@ -117,8 +117,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_sweeps(SArgs a) {
   const uint32_t xs0 = smem_u32(xs);
   int to_slot = 0, slot = 0;  // of sweep s and s - 1: s % 3
   uint32_t parity = 0;        // of the barrier of sweep s - 1
+  // Only warps with rows take part.  A phase of a block's barrier completes
+  // with the rows of all of them, so none of them falls behind by more than one
+  // sweep; a warp without rows holds nothing back, and three sweeps behind
+  // it would find the parity that it waits for turned over.
 #pragma unroll 1
-  for (int s = 1; s <= a.sweeps; ++s) {
+  for (int s = 1; s <= a.sweeps && wid < tasks; ++s) {
     slot = to_slot;
     to_slot = slot == 2 ? 0 : slot + 1;
     const bool last = s == a.sweeps;
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_sweeps(SArgs a) {
   }
   __syncthreads();
   const bool fail = s_fail != 0;
-  const float* x = xs + to_slot * a.nx;
+  const float* x = xs + a.sweeps % 3 * a.nx;
   for (int row = tid; row < nr; row += nthr)
     if (r0 + row < a.n) a.x[r0 + row] = fail ? NAN : x[row];
   if (a.t.xf) {
