@@ -532,7 +532,10 @@ int mgpbd_level_sweep(mgpbd_handle h, int32_t level, int32_t op, const float* x,
 
 int mgpbd_synchronize(mgpbd_handle h) {
   if (!h) return MGPBD_EINVAL;
-  return guarded([&] { MGPBD_CUDA(cudaStreamSynchronize(h->impl.stream())); });
+  return guarded([&] {
+    MGPBD_CUDA(cudaStreamSynchronize(h->impl.stream()));
+    h->impl.check_sweeps();
+  });
 }
 
 // ---- standalone sparse kernels --------------------------------------------

@@ -135,6 +135,7 @@ Solver::~Solver() {
   if (h_body_loop_) cudaFreeHost(h_body_loop_);
   if (h_buf_) cudaFreeHost(h_buf_);
   if (h_state_) cudaFreeHost(h_state_);
+  if (h_sweep_) cudaFreeHost(h_sweep_);
   if (h_cf_) cudaFreeHost(h_cf_);
   for (cudaEvent_t e : ev_)
     if (e) cudaEventDestroy(e);
@@ -701,6 +702,8 @@ void Solver::alloc_work() {
   }
   // the coarsest level's rows on a cluster
   sweep_ = SweepPlan();
+  if (!h_sweep_) MGPBD_CUDA(cudaMallocHost(&h_sweep_, sizeof(int32_t)));
+  *h_sweep_ = 0;
   if (!cheb() && levels_.back().nnz <= kSweepMaxNnz) {
     const Level& L = levels_.back();
     std::vector<int32_t> ip(L.n + 1), ix(L.nnz);
@@ -1193,7 +1196,16 @@ bool Solver::fused_sweeps() const {
 void Solver::coarse_sweeps(const float* b, const SweepTransfer& t, const CgState* guard) {
   Level& L = levels_.back();
   launch_sweeps(guard, L.view(), sweep_, b, p_.omega_jacobi, L.omega.p, n_coarse_sweeps(),
-                p_.mode == MGPBD_MODE_FAST, L.xa.p, t, &cg_state_.p->status, stream_);
+                p_.mode == MGPBD_MODE_FAST, L.xa.p, t, barrier_limit_s_, h_sweep_, stream_);
+}
+
+// Reports a wait of the coarse sweeps that gave up, once
+void Solver::check_sweeps() {
+  if (!h_sweep_ || *const_cast<volatile int32_t*>(h_sweep_) == 0) return;
+  *h_sweep_ = 0;
+  status_ |= MGPBD_STATUS_SYNC_TIMEOUT;
+  net_active_ = judge_pending_ = false;
+  throw Error(MGPBD_ECUDA, "coarse sweeps: a wait timed out");
 }
 
 // GPUMultigridSolver.vcycle (cons/mgpcg_gpu.py:214-259) with a zero initial
@@ -1370,6 +1382,7 @@ void Solver::precondition(CgState* guard, CgSweeps& c) {
 void Solver::vcycle_into(const float* r, float* z) {
   require_init();
   require(!cheb(), MGPBD_ENOTSUP, "no V-cycle: the solver uses the Chebyshev preconditioner");
+  check_sweeps();
   vcycle(0, r, nullptr);
   MGPBD_CUDA(cudaMemcpyAsync(z, levels_[0].xa.p, sizeof(float) * nt_, cudaMemcpyDeviceToDevice,
                              stream_));
@@ -1438,6 +1451,7 @@ int32_t Solver::pcg_learned(const float* b, float* x) {
   for (int32_t k = 0; k < p_.maxiter_cg; ++k) {
     cg_body(x);
     sync_read(h_state_, cg_state_.p, sizeof(CgState));
+    check_sweeps();
     const bool bad = net_active_ && (static_cast<uint32_t>(h_state_->status) & broken);
     if (h_state_->done && !bad) break;
     if (!net_active_) continue;
@@ -1465,6 +1479,7 @@ int32_t Solver::pcg_learned(const float* b, float* x) {
     }
   }
   sync_read(h_state_, cg_state_.p, sizeof(CgState));
+  check_sweeps();
   if (net_active_) stats_.learned_solves += 1;
   net_active_ = false;
   status_ |= static_cast<uint32_t>(h_state_->status);
@@ -1476,6 +1491,7 @@ int32_t Solver::pcg(const float* b, float* x) {
   require_init();
   dual_x_ = nullptr;
   if (cheb()) return pcg_cheb(b, x);
+  check_sweeps();
   if (learned()) return pcg_learned(b, x);
   if (p_.mode == MGPBD_MODE_FAST && p_.use_graph && b == rhs_.p && x == dlam_.p &&
       rec_count_ >= rec_cap_)
@@ -1493,9 +1509,11 @@ int32_t Solver::pcg(const float* b, float* x) {
   for (int32_t k = 0; k < p_.maxiter_cg; ++k) {
     cg_body(x);
     sync_read(h_state_, cg_state_.p, sizeof(CgState));
+    check_sweeps();
     if (h_state_->done) break;
   }
   sync_read(h_state_, cg_state_.p, sizeof(CgState));
+  check_sweeps();
   status_ |= static_cast<uint32_t>(h_state_->status);
   return h_state_->iters;
 }
@@ -1505,7 +1523,7 @@ int32_t Solver::pcg(const float* b, float* x) {
 // is bounded on the device by maxiter_cg (k_cg_beta sets done).
 int32_t Solver::pcg_graph(const float* b, float* x) {
   cudaStream_t outer = stream_;
-  if (!cg_exec_ || cg_graph_b_ != b || cg_graph_x_ != x) {
+  if (!cg_exec_ || cg_graph_b_ != b || cg_graph_x_ != x || cg_graph_limit_ != barrier_limit_s_) {
     if (cg_exec_) {
       cudaGraphExecDestroy(cg_exec_);
       cg_exec_ = nullptr;
@@ -1576,9 +1594,11 @@ int32_t Solver::pcg_graph(const float* b, float* x) {
     cudaStreamDestroy(bs);
     cg_graph_b_ = b;
     cg_graph_x_ = x;
+    cg_graph_limit_ = barrier_limit_s_;
   }
   MGPBD_CUDA(cudaGraphLaunch(cg_exec_, outer));
   sync_read(h_state_, cg_state_.p, sizeof(CgState));
+  check_sweeps();
   g_launches.fetch_add(graph_init_launches_ + graph_body_launches_ * h_state_->body_runs);
   status_ |= static_cast<uint32_t>(h_state_->status);
   return h_state_->iters;

@@ -90,11 +90,12 @@ class Solver {
   // per body: Newton iterations, first and last residual, last line-search
   // step of the last solve
   void body_stats(int32_t n, int32_t* newton, double* r0, double* r, double* omega) const;
-  // wait limit of the persistent CG kernels' grid barriers (seconds)
+  // wait limit of the persistent CG kernels and of the coarse sweeps (seconds)
   void set_barrier_limit(double seconds) {
     require(seconds >= 0.0 && seconds <= 60.0, MGPBD_EINVAL, "barrier limit must be in [0, 60] s");
     barrier_limit_s_ = seconds;
   }
+  void check_sweeps();
   // per-constraint MGPBD_CONS_* types (host array of nt; nullptr: all ARAP)
   void set_constraint_types(const int32_t* types);
   void init();
@@ -276,6 +277,7 @@ class Solver {
   DevBuf<float> pw_a_, pw_b_;  // power-iteration vectors
   double* h_buf_ = nullptr;    // pinned host scratch
   CgState* h_state_ = nullptr;
+  int32_t* h_sweep_ = nullptr;  // pinned: 1 after a wait of the coarse sweeps gave up
   ChebCoef* h_cf_ = nullptr;   // pinned staging of the Chebyshev coefficients
   cudaEvent_t ev_[2] = {nullptr, nullptr};  // around each persistent CG launch
   static double event_ms(cudaEvent_t a, cudaEvent_t b);
@@ -284,6 +286,7 @@ class Solver {
   cudaGraphExec_t cg_exec_ = nullptr;
   const float* cg_graph_b_ = nullptr;
   float* cg_graph_x_ = nullptr;
+  double cg_graph_limit_ = 0.0;
   long long graph_init_launches_ = 0;
   long long graph_body_launches_ = 0;
 

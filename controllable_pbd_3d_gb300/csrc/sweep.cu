@@ -17,6 +17,7 @@
 #include <utility>
 
 #include "cluster_dev.cuh"
+#include "persist.cuh"
 
 namespace mgpbd {
 
@@ -28,7 +29,6 @@ constexpr int kSweepThreads = 1024;
 constexpr int kSweepWarps = kSweepThreads / 32;
 constexpr int kSweepBlocks = 16;
 constexpr int kCutRows = 16;  // rows are handed out in groups of 16
-constexpr uint32_t kPollLimit = 1 << 24;  // polls of a barrier before a wait gives up
 
 struct SArgs {
   const CgState* st;
@@ -43,11 +43,28 @@ struct SArgs {
   float w;
   const float* wp;
   SweepTransfer t;
-  int32_t* status;
+  int32_t* timed_out;
+  unsigned long long spin_ns;
   int32_t n, blocks, rows, steps, nx, sweeps, zero_first;
 };
 
 extern __shared__ __align__(16) unsigned char s_mem[];
+
+// Waits for a phase of a barrier; false when the limit is reached or another
+// warp of the block has given up.  A limit of 0 gives up at the first poll that
+// finds the phase incomplete.
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, unsigned long long limit,
+                                           volatile int* fail) {
+  if (limit == 0) return test_phase(bar, parity);
+  unsigned long long t0 = 0;
+  for (uint32_t n = 1; !try_phase(bar, parity); ++n) {
+    if (n % 64 != 0) continue;
+    const unsigned long long t = pdev::global_ns();
+    if (t0 == 0) t0 = t;
+    if (*fail != 0 || t - t0 > limit) return false;
+  }
+  return true;
+}
 
 // G lanes of a warp share a row (32 / G rows a warp, a task).  In each step a
 // lane multiplies four elements, in the order that the plan found: the 32 reads
@@ -113,7 +130,6 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_sweeps(SArgs a) {
   __syncthreads();
   cluster_meet();  // every block's barriers and copies are ready for stores
 
-  bool ok = true;
   const uint32_t xs0 = smem_u32(xs);
   int to_slot = 0, slot = 0;  // of sweep s and s - 1: s % 3
   uint32_t parity = 0;        // of the barrier of sweep s - 1
@@ -129,15 +145,10 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_sweeps(SArgs a) {
     const uint32_t bar = smem_u32(&s_bar[to_slot]);
     if (tid == 0 && !last) expect_bytes(bar, 16 * recv);
     if (s > 1) {
-      if (ok) {
-        const uint32_t from = smem_u32(&s_bar[slot]);
-        uint32_t n = 0;
-        while (!try_phase(from, parity))
-          if (++n == kPollLimit) {
-            ok = false;
-            s_fail = 1;
-            break;
-          }
+      const bool ok = wait_phase(smem_u32(&s_bar[slot]), parity, a.spin_ns, &s_fail);
+      if (!__all_sync(0xffffffffu, ok)) {  // no more arrivals, no more stores
+        s_fail = 1;
+        break;
       }
       if (slot == 0) parity ^= 1;  // (sweeps 1 to 3, 4 to 6, ...)
     }
@@ -203,13 +214,15 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_sweeps(SArgs a) {
       for (int k = a.t.mem_ptr[r0 + row] + i % kL; k < k1; k += kL) a.t.xf[a.t.mem_rows[k]] += v;
     }
   }
-  if (fail) {
-    if (tid == 0) atomicOr(reinterpret_cast<unsigned int*>(a.status), MGPBD_STATUS_SYNC_TIMEOUT);
-    // stores to this block may still be on their way
-    for (int k = 0; k < 50; ++k) __nanosleep(1000);
+  if (fail && tid == 0) {
+    *const_cast<volatile int32_t*>(a.timed_out) = 1;
+    __threadfence_system();
   }
   __syncthreads();
   cluster_meet();
+  // stores to a block that gave up may still be on their way
+  if (fail)
+    for (int k = 0; k < 50; ++k) __nanosleep(1000);
 }
 
 using SweepFn = void (*)(SArgs);
@@ -404,7 +417,7 @@ void build_sweep_plan(const std::vector<int32_t>& indptr, const std::vector<int3
 
 void launch_sweeps(const CgState* st, const CsrView& a, const SweepPlan& plan, const float* b, float w,
                    const float* w_dev, int32_t sweeps, bool zero_first, float* x,
-                   const SweepTransfer& t, int32_t* status, cudaStream_t s) {
+                   const SweepTransfer& t, double spin_limit_s, int32_t* timed_out, cudaStream_t s) {
   require(plan.blocks > 0 && sweeps >= 1, MGPBD_ESTATE, "no plan for the coarse sweeps");
   SArgs g = {};
   g.st = st;
@@ -420,7 +433,8 @@ void launch_sweeps(const CgState* st, const CsrView& a, const SweepPlan& plan, c
   g.w = w;
   g.wp = w_dev;
   g.t = t;
-  g.status = status;
+  g.timed_out = timed_out;
+  g.spin_ns = static_cast<unsigned long long>(spin_limit_s * 1e9);
   g.n = a.n;
   g.blocks = plan.blocks;
   g.rows = plan.rows;

@@ -43,10 +43,10 @@ struct SweepTransfer {
 
 // x = `sweeps` sweeps x += w D^-1 (b - A x) from x = 0, w from w_dev when not
 // null; zero_first: the first sweep is written down as w D^-1 b.  A no-op
-// once st->done.  A wait that gave up leaves NaN in x (and xf) and
-// MGPBD_STATUS_SYNC_TIMEOUT in *status.
+// once st->done.  A wait longer than spin_limit_s leaves NaN in the x (and xf)
+// of the blocks that gave up and 1 in *timed_out (pinned host memory).
 void launch_sweeps(const CgState* st, const CsrView& a, const SweepPlan& plan, const float* b, float w,
                    const float* w_dev, int32_t sweeps, bool zero_first, float* x,
-                   const SweepTransfer& t, int32_t* status, cudaStream_t s);
+                   const SweepTransfer& t, double spin_limit_s, int32_t* timed_out, cudaStream_t s);
 
 }  // namespace mgpbd

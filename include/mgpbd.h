@@ -343,11 +343,12 @@ int mgpbd_set_body_compliance(mgpbd_handle h, int32_t n_bodies, const float* com
 int mgpbd_body_stats(mgpbd_handle h, int32_t n, int32_t* newton_iters, double* residual0,
                      double* residual, double* omega);
 
-/* Wait limit, in seconds [0, 60], of every grid-barrier wait of the
- * persistent CG kernels (default 4).  A wait that reaches it ends the
+/* Wait limit, in seconds [0, 60], of every wait for another block in the
+ * persistent CG kernels and in the V-cycle's coarse sweeps (default 4).  A wait that reaches it ends the
  * kernel on every block, marks MGPBD_STATUS_SYNC_TIMEOUT and makes the call
  * return MGPBD_ECUDA; the next launch starts afresh, so the handle stays
- * usable.  0 gives up at the first wait that finds another block not yet
+ * usable.  (mgpbd_vcycle only queues its work: there a later mgpbd_vcycle,
+ * mgpbd_pcg or mgpbd_synchronize returns the error.)  0 gives up at the first wait that finds another block not yet
  * arrived, which makes a solve fail this way on purpose (how the tests
  * exercise the path).  No counterpart in the reference. */
 int mgpbd_set_barrier_limit(mgpbd_handle h, double seconds);

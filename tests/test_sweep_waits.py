@@ -2,7 +2,9 @@
 barriers.  A block has three, reused every three sweeps and tested by one bit
 of parity, so a warp that a phase does not need can miss it: on the CPU, a model
 of the barriers in which one warp at a time is kept from running; on the GPU,
-thousands of sweeps in blocks with fewer rows than warps, or none."""
+thousands of sweeps in blocks with fewer rows than warps, or none; and waits that
+run out (a limit of 0: a block gives up at the first poll that finds a phase
+incomplete, and all blocks end within their first sweeps)."""
 
 import numpy as np
 import pytest
@@ -119,3 +121,57 @@ def test_many_sweeps_of_few_rows(cuda, monkeypatch, n, per_row):
   for g in got[1:]:
     assert np.array_equal(got[0], g)
   assert np.abs(got[0] - ref).max() <= s.err
+
+
+@pytest.mark.gpu
+def test_a_wait_that_runs_out_is_reported_later_by_the_vcycle(cuda):
+  from controllable_pbd_3d_gb300.mgpcg_gpu import GPUMultigridSolver
+  m = GPUMultigridSolver().setup(matrix(3001, 30, 5), [])
+  b = cuda.tensor(np.random.default_rng(3).standard_normal(3001).astype(np.float32), device='cuda')
+  want = m.vcycle_apply(b).clone()
+  L = N.lib()
+  for again in (lambda: m.vcycle_apply(b), lambda: m.solve(b, cuda.zeros_like(b)),
+                lambda: N.check(L.mgpbd_synchronize(m._h), 'mgpbd_synchronize')):
+    assert L.mgpbd_set_barrier_limit(m._h, 0.0) == 0
+    got = m.vcycle_apply(b)
+    cuda.cuda.synchronize()
+    assert bool(cuda.isnan(got).any())
+    assert L.mgpbd_set_barrier_limit(m._h, 4.0) == 0
+    with pytest.raises(N.MGPBDError, match='timed out') as e:
+      again()
+    assert e.value.code == -2
+    assert cuda.equal(m.vcycle_apply(b), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('kw', [dict(mode='fast'), dict(mode='parity'), dict(mode='fast', use_graph=False)])
+def test_a_wait_that_runs_out_ends_the_solve(cuda, kw):
+  from controllable_pbd_3d_gb300 import MGPBDSolverGPU, meshgen
+  xr, t = meshgen.hex_grid_tets(7, 8, 6)
+  x0, _ = meshgen.hex_grid_tets(7, 8, 6, jitter=0.02, seed=3)
+
+  def solver():
+    x = cuda.tensor(x0, device='cuda')
+    s = MGPBDSolverGPU(x, cuda.tensor(xr, device='cuda'),
+                       cuda.tensor(np.ones(len(xr), np.float32), device='cuda'), cuda.tensor(t, device='cuda'),
+                       None, [0.0, -9.8, 0.0], 1.0 / 300, mu=1e5, maxiter=2, **kw)
+    s.init()
+    s.step(0)
+    return s, x
+
+  (s, x), (ref, x_ref) = solver(), solver()
+  L = N.lib()
+  assert L.mgpbd_set_barrier_limit(s._h, 0.0) == 0
+  s.make_prediction()
+  before = x.clone()
+  with pytest.raises(N.MGPBDError, match='timed out') as e:
+    s.solve(1)
+  assert e.value.code == -2
+  assert L.mgpbd_set_barrier_limit(s._h, 4.0) == 0
+  with cuda.no_grad():
+    x.copy_(before)
+  s.solve(1)
+  s.update_vel()
+  ref.step(1)
+  assert s.stats()['status'] == ref.stats()['status']
+  assert cuda.equal(x, x_ref)
