@@ -1123,14 +1123,14 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   if (syncw)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(s_tmem));
   if (CLUSTER) {
-    // after a wait that gave up, stores to this block may still be on their
-    // way: let them land before any block of the cluster leaves
+    __syncthreads();
+    cluster_meet();
+    // stores to a block that gave up may still be on their way: it stays until
+    // they have landed
     if (!s_ok) {
       const unsigned long long t0 = global_ns();
       while (global_ns() - t0 < 50000) __nanosleep(1000);
     }
-    __syncthreads();
-    cluster_meet();
   }
 }
 
