@@ -39,8 +39,7 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Block-wide float64 sum in a fixed pattern; result valid in thread 0.
-// Sum over the block (at most kThreads), in thread 0.  One warp adds: float64
+// Float64 sum over the block (at most kThreads) in a fixed order, in thread 0.  One warp adds: float64
 // additions are slow here (2 a clock and SM), and a tree in every warp takes
 // four times as many.
 __device__ __forceinline__ double block_sum(double v) {
@@ -590,59 +589,88 @@ __device__ double sum_partials(const double* __restrict__ p, int blocks) {
 // before it; block 0 leaves the result in the state.  (As one-block kernels of
 // their own these steps were three of the 16 launches of an iteration; made by
 // the last block of the launch before, the tickets and fences took 6 us each.)
-// True: go on.  A block that starts late may find the `done` that block 0
-// leaves here, and ends as all others do.
-__device__ bool cg_alpha(CgState* st, const double* p, int blocks, double* alpha) {
-  const double pap = sum_partials(p, blocks), a = st->rz / pap;
-  const bool bad = fabs(pap) < 1e-30 || !isfinite(pap);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->pap = pap;
-    if (!isfinite(pap)) st->status |= MGPBD_STATUS_NAN;
-    if (bad) {
-      st->done = 1;
-    } else {
-      if (pap <= 0.0) st->status |= MGPBD_STATUS_PAP_NONPOS;
-      st->alpha = a;
+//
+// Block 0 may store `done` while other blocks start.  One thread reads it for
+// its block and decides, and all threads follow: a block that finds it set ends
+// as the sum would have made it end.  step(sum, scalar) runs in that thread and
+// returns whether to go on.
+template <class F>
+__device__ bool cg_scalar(const CgState* st, const double* __restrict__ p, int blocks, double* scalar,
+                          F step) {
+  __shared__ double value;
+  __shared__ int go;
+  if (threadIdx.x < 32) {
+    const int32_t done = *const_cast<const volatile int32_t*>(&st->done);
+    double acc = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < blocks; i += 32) acc += p[i];
+    acc = warp_sum(acc);
+    if (threadIdx.x == 0) {
+      value = 0.0;
+      go = !done && step(acc, &value);
     }
   }
-  *alpha = a;
-  return !bad;
+  __syncthreads();
+  *scalar = value;
+  return go != 0;
+}
+
+__device__ bool cg_alpha(CgState* st, const double* p, int blocks, double* alpha) {
+  return cg_scalar(st, p, blocks, alpha, [&](double pap, double* a) {
+    const bool bad = fabs(pap) < 1e-30 || !isfinite(pap);
+    *a = st->rz / pap;
+    if (blockIdx.x == 0) {
+      st->pap = pap;
+      if (!isfinite(pap)) st->status |= MGPBD_STATUS_NAN;
+      if (bad) {
+        st->done = 1;
+      } else {
+        if (pap <= 0.0) st->status |= MGPBD_STATUS_PAP_NONPOS;
+        st->alpha = *a;
+      }
+    }
+    return !bad;
+  });
 }
 
 __device__ bool cg_check(CgState* st, const double* p, int blocks) {
-  const double rr = sum_partials(p, blocks);
-  const bool nan = !isfinite(rr), stop = nan || rr < st->tol2;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->rr = rr;
-    if (stop) {
-      if (nan) st->status |= MGPBD_STATUS_NAN;
-      else st->iters += 1;
-      st->done = 1;
+  double unused;
+  return cg_scalar(st, p, blocks, &unused, [&](double rr, double*) {
+    const bool nan = !isfinite(rr), stop = nan || rr < st->tol2;
+    if (blockIdx.x == 0) {
+      st->rr = rr;
+      if (stop) {
+        if (nan) st->status |= MGPBD_STATUS_NAN;
+        else st->iters += 1;
+        st->done = 1;
+      }
     }
-  }
-  return !stop;
+    return !stop;
+  });
 }
 
 // rz of the next iteration is left in rz_new (the others still read rz), and
 // moved by the next iteration's SpMV
 __device__ bool cg_beta(CgState* st, const double* p, int blocks, double* beta) {
-  const double rzn = sum_partials(p, blocks), rz = st->rz;
-  const bool bad = fabs(rz) < 1e-30;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->rz_new = rzn;
-    st->iters += 1;
-    if (bad) {
-      st->done = 1;
-    } else {
-      st->beta = rzn / rz;
-      if (st->iters >= st->maxiter) {
+  return cg_scalar(st, p, blocks, beta, [&](double rzn, double* b) {
+    const double rz = st->rz;
+    const bool bad = fabs(rz) < 1e-30;
+    *b = rzn / rz;
+    if (blockIdx.x == 0) {
+      st->rz_new = rzn;
+      st->iters += 1;
+      if (bad) {
         st->done = 1;
-        st->status |= MGPBD_STATUS_CG_MAXITER;
+      } else {
+        st->beta = *b;
+        if (st->iters >= st->maxiter) {
+          st->done = 1;
+          st->status |= MGPBD_STATUS_CG_MAXITER;
+        }
       }
     }
-  }
-  *beta = rzn / rz;
-  return !bad;
+    return !bad;
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -658,8 +686,7 @@ __global__ void __launch_bounds__(kThreads)
                const float* __restrict__ b, const float* __restrict__ dinv, float* __restrict__ y,
                float w, const float* __restrict__ wp, double* __restrict__ partials,
                CgState* st, const double* __restrict__ check, int check_blocks) {
-  if (st && st->done) return;
-  if (check && !cg_check(st, check, check_blocks)) return;
+  if (check ? !cg_check(st, check, check_blocks) : st && st->done) return;
   if (OP == kSpmvDot && blockIdx.x == 0 && threadIdx.x == 0) st->rz = st->rz_new;
   if (wp) w = *wp;
   // The loop bound is uniform per warp (all 32/G rows of a warp advance
@@ -721,8 +748,7 @@ __global__ void __launch_bounds__(kThreads)
                    const float* __restrict__ dinv, float* __restrict__ y, float w,
                    const float* __restrict__ wp, double* __restrict__ partials,
                    CgState* st, const double* __restrict__ check, int check_blocks) {
-  if (st && st->done) return;
-  if (check && !cg_check(st, check, check_blocks)) return;
+  if (check ? !cg_check(st, check, check_blocks) : st && st->done) return;
   if (OP == kSpmvDot && blockIdx.x == 0 && threadIdx.x == 0) st->rz = st->rz_new;
   if (wp) w = *wp;
   const int lane = threadIdx.x % G;
@@ -945,7 +971,6 @@ __global__ void k_cg_update_xr(CgState* st, const double* __restrict__ pap, int 
                                float* __restrict__ x, float* __restrict__ r, int64_t n,
                                double* __restrict__ partials, const float* __restrict__ dinv,
                                const float* __restrict__ wp, float* __restrict__ z) {
-  if (st->done) return;
   double alpha;
   if (!cg_alpha(st, pap, blocks, &alpha)) return;
   float a = (float)alpha;
@@ -966,7 +991,7 @@ __global__ void k_cg_update_xr(CgState* st, const double* __restrict__ pap, int 
 
 // the stopping test where no row operator follows
 __global__ void k_cg_check(CgState* st, const double* __restrict__ p, int blocks) {
-  if (!st->done) cg_check(st, p, blocks);
+  cg_check(st, p, blocks);
 }
 
 // Restart of a CG solve from its current iterate: rz from the partials,
@@ -988,7 +1013,7 @@ __global__ void k_cg_update_p(CgState* st, const double* __restrict__ rz, int bl
                               const float* __restrict__ z, float* __restrict__ p, int64_t n,
                               cudaGraphConditionalHandle handle, int loop) {
   double beta = 0.0;
-  const bool go = !st->done && cg_beta(st, rz, blocks, &beta);
+  const bool go = cg_beta(st, rz, blocks, &beta);
   if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
     st->body_runs += 1;
     cudaGraphSetConditional(handle, st->done ? 0u : 1u);
