@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <algorithm>
 #include <cmath>
 
 #include "common.h"
@@ -679,6 +680,38 @@ __device__ bool cg_beta(CgState* st, const double* p, int blocks, double* beta) 
 // check: the partials of CG's r.r, when its stopping test is still to be made.
 enum RowOp { kSpmv = 0, kJacobi = 1, kResidual = 2, kSpmvDot = 3, kJacobiZero = 4, kJacobiDot = 5 };
 
+// The products of a dot operator's rows.  A float64 multiply-add occupies its
+// pipe for a whole warp however few lanes take part: with the first of a row's G
+// lanes finishing it, the products of 718,520 rows took 24 us beside 105 of the
+// sweep itself.  TURNS: the lanes take turns at finishing a row, and their
+// products are added when each has one.
+template <int G, bool TURNS>
+struct RowDot {
+  double acc = 0.0;
+  float f = 0.0f, g = 0.0f;
+  int turn = 0;
+  __device__ void put(float a, float b) {
+    if (TURNS) {
+      f = a;
+      g = b;
+    } else {
+      acc += (double)a * (double)b;
+    }
+  }
+  __device__ void next() {
+    if (TURNS && ++turn == G) flush();
+  }
+  __device__ void flush() {
+    acc += (double)f * (double)g;
+    f = g = 0.0f;
+    turn = 0;
+  }
+  __device__ double sum() {
+    if (TURNS) flush();
+    return acc;
+  }
+};
+
 template <int G, int OP>
 __global__ void __launch_bounds__(kThreads)
     k_csr_rows(int32_t n, const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
@@ -691,11 +724,12 @@ __global__ void __launch_bounds__(kThreads)
   if (wp) w = *wp;
   // The loop bound is uniform per warp (all 32/G rows of a warp advance
   // together), so every lane reaches the shuffles.
+  constexpr bool kDot = OP == kSpmvDot || OP == kJacobiDot;
   const int lane = threadIdx.x % G;
   constexpr int kRowsPerWarp = 32 / G;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kRowsPerWarp;
-  double dacc = 0.0;
+  RowDot<G, false> dot;
   for (int64_t base = warp * kRowsPerWarp; base < n; base += stride) {
     const int64_t row = base + (threadIdx.x & 31) / G;
     const bool valid = row < n;
@@ -713,7 +747,7 @@ __global__ void __launch_bounds__(kThreads)
         y[row] = sum;
       } else if (OP == kSpmvDot) {
         y[row] = sum;
-        dacc += (double)x[row] * (double)sum;
+        dot.put(x[row], sum);
       } else if (OP == kResidual) {
         y[row] = b[row] - sum;
       } else if (OP == kJacobi) {
@@ -721,14 +755,14 @@ __global__ void __launch_bounds__(kThreads)
       } else if (OP == kJacobiDot) {
         const float v = x[row] + w * dinv[row] * (b[row] - sum);
         y[row] = v;
-        dacc += (double)b[row] * (double)v;
+        dot.put(b[row], v);
       } else {  // x = 0: A x = 0 exactly for finite A
         y[row] = w * dinv[row] * b[row];
       }
     }
   }
-  if (OP == kSpmvDot || OP == kJacobiDot) {
-    dacc = block_sum(dacc);
+  if (kDot) {
+    const double dacc = block_sum(dot.sum());
     if (threadIdx.x == 0) partials[blockIdx.x] = dacc;
   }
 }
@@ -740,7 +774,7 @@ __global__ void __launch_bounds__(kThreads)
 // The arrays carry >= 4 padding elements, so the last window stays inside
 // the allocation.  All U loads of a pass are issued before the first use,
 // which keeps 2*U*16 bytes per lane in flight.
-template <int G, int U, int OP>
+template <int G, int U, int OP, bool TURNS>
 __global__ void __launch_bounds__(kThreads)
     k_csr_rows_vec(int32_t n, const int32_t* __restrict__ indptr,
                    const int32_t* __restrict__ indices, const float* __restrict__ data,
@@ -751,11 +785,12 @@ __global__ void __launch_bounds__(kThreads)
   if (check ? !cg_check(st, check, check_blocks) : st && st->done) return;
   if (OP == kSpmvDot && blockIdx.x == 0 && threadIdx.x == 0) st->rz = st->rz_new;
   if (wp) w = *wp;
+  constexpr bool kDot = OP == kSpmvDot || OP == kJacobiDot;
   const int lane = threadIdx.x % G;
   constexpr int kRowsPerWarp = 32 / G;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kRowsPerWarp;
-  double dacc = 0.0;
+  RowDot<G, TURNS> dot;
   for (int64_t base = warp * kRowsPerWarp; base < n; base += stride) {
     const int64_t row = base + (threadIdx.x & 31) / G;
     const bool valid = row < n;
@@ -788,23 +823,24 @@ __global__ void __launch_bounds__(kThreads)
     }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
-    if (valid && lane == 0) {
+    if (valid && lane == (TURNS ? dot.turn : 0)) {
       if (OP == kSpmv) {
         y[row] = sum;
       } else if (OP == kSpmvDot) {
         y[row] = sum;
-        dacc += (double)x[row] * (double)sum;
+        dot.put(x[row], sum);
       } else if (OP == kResidual) {
         y[row] = b[row] - sum;
       } else {
         const float v = x[row] + w * dinv[row] * (b[row] - sum);
         y[row] = v;
-        if (OP == kJacobiDot) dacc += (double)b[row] * (double)v;
+        if (OP == kJacobiDot) dot.put(b[row], v);
       }
     }
+    if (kDot) dot.next();
   }
-  if (OP == kSpmvDot || OP == kJacobiDot) {
-    dacc = block_sum(dacc);
+  if (kDot) {
+    const double dacc = block_sum(dot.sum());
     if (threadIdx.x == 0) partials[blockIdx.x] = dacc;
   }
 }
@@ -819,16 +855,22 @@ constexpr int kRowShapeG[kNumRowShapes] = {4, 4, 4, 2, 2, 4, 8, 8};
 constexpr int kRowShapeU[kNumRowShapes] = {6, 4, 8, 4, 8, 2, 2, 4};
 
 // (the launches return their blocks: the partials of the dot operators)
-template <int OP>
+template <int OP, bool TURNS = false>
 int launch_vec_shape(int idx, const CsrView& a, const float* x, const float* b, float* y,
                       float w, double* partials, CgState* st, cudaStream_t s, const float* wp = nullptr,
                      const CgCheck& check = {}) {
   const int G = kRowShapeG[idx];
   const int grid = grid_for(a.n, kThreads / G);
+  // From three rounds of rows on the lanes of a dot operator take turns (us an
+  // iteration without / with: 248,612 rows, 3.2 rounds 440 / 436, 718,520 991 /
+  // 975); below, it only takes registers (91,660 rows 245.4 / 248.0).
+  if constexpr ((OP == kSpmvDot || OP == kJacobiDot) && !TURNS)
+    if (a.n >= 3LL * grid * (kThreads / G))
+      return launch_vec_shape<OP, true>(idx, a, x, b, y, w, partials, st, s, wp, check);
   switch (idx) {
 #define MGPBD_VEC_CASE(I, GG, UU)                                                            \
   case I:                                                                                    \
-    k_csr_rows_vec<GG, UU, OP><<<grid, kThreads, 0, s>>>(a.n, a.indptr, a.indices, a.data, x, \
+    k_csr_rows_vec<GG, UU, OP, TURNS><<<grid, kThreads, 0, s>>>(a.n, a.indptr, a.indices, a.data, x, \
                                                          b, a.diag_inv, y, w, wp, partials, st, \
                                                          check.partials, check.blocks); \
     break;
@@ -1328,13 +1370,19 @@ void launch_cg_init(CgState* st, const double* partials_rz, int blocks, double t
   k_cg_init<<<1, kThreads, 0, s>>>(st, partials_rz, blocks, tol_abs, tol_rel, maxiter);
   MGPBD_CHECK_LAUNCH();
 }
+// blocks of the CG's vector updates, each of which adds the partials of a dot
+// product first: with 8 a SM those float64 additions take as long as the update
+// (718,520 rows: 991 us an iteration with 1,216 blocks, 988 with 608, 994 with
+// 304)
+static int vector_blocks(int64_t n) { return std::min(grid_for(n, kThreads), kMaxReduceBlocks / 2); }
+
 int launch_cg_update_xr(CgState* st, const double* pap, int blocks, const float* p, const float* ap,
                         float* x, float* r, int64_t n, double* partials, const float* dinv,
                         const float* w_dev, float* z, cudaStream_t s) {
-  k_cg_update_xr<<<reduce_blocks(n), kThreads, 0, s>>>(st, pap, blocks, p, ap, x, r, n, partials,
+  k_cg_update_xr<<<vector_blocks(n), kThreads, 0, s>>>(st, pap, blocks, p, ap, x, r, n, partials,
                                                        dinv, w_dev, z);
   MGPBD_CHECK_LAUNCH();
-  return reduce_blocks(n);
+  return vector_blocks(n);
 }
 void launch_cg_check(CgState* st, const CgCheck& check, cudaStream_t s) {
   k_cg_check<<<1, kThreads, 0, s>>>(st, check.partials, check.blocks);
@@ -1347,7 +1395,7 @@ void launch_cg_restart(CgState* st, const double* p, int blocks, int32_t clear_m
 }
 void launch_cg_update_p(CgState* st, const double* rz, int blocks, const float* z, float* p, int64_t n,
                         const cudaGraphConditionalHandle* loop, cudaStream_t s) {
-  k_cg_update_p<<<grid_for(n, kThreads), kThreads, 0, s>>>(st, rz, blocks, z, p, n, loop ? *loop : 0,
+  k_cg_update_p<<<vector_blocks(n), kThreads, 0, s>>>(st, rz, blocks, z, p, n, loop ? *loop : 0,
                                                            loop != nullptr);
   MGPBD_CHECK_LAUNCH();
 }
