@@ -39,9 +39,10 @@
 // hexes, before / after: n = 10 68 / 27 (cluster), 20 70 / 39, 28 77 / 45,
 // 40 141 / 67; 80x20x80 332 / 135; ARAP 23x17x29 63 / 39.
 //
-// Arithmetic per element, the reductions and the scalar logic are those of
-// k_jcg (jcg.cu): float32 per element, float32 within a warp and float64
-// across warps and blocks, Kahan-compensated solution.  Sums run in a fixed
+// Arithmetic per element, the reductions and the scalar logic of the CG are
+// those of k_jcg (jcg.cu): float32 per element, float32 within a warp and
+// float64 across warps and blocks, Kahan-compensated solution.  The sums of the
+// estimate, which k_lz_apply (jform.cu) makes in float64, have 48 bits.  Sums run in a fixed
 // order, so results repeat bit for bit.
 //
 // Every wait is bounded as there; the blocks of a cluster meet once more at
@@ -218,6 +219,29 @@ __device__ __forceinline__ bool bounded_wait(const DArgs& a, F there) {
   }
   return ok;
 }
+
+// A sum in two float32 words, about 48 bits: the products and the errors of the
+// additions are kept exactly (Knuth's two-sum, a fused multiply-add for the
+// product).  (In float64, whose pipe is slow, the sums of a Lanczos step would
+// take as long as the application of A.)
+struct Sum2 {
+  float hi = 0.0f, lo = 0.0f;
+  __device__ __forceinline__ void add(float v) {
+    const float s = __fadd_rn(hi, v), t = __fsub_rn(s, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(v, t)));
+    hi = s;
+  }
+  __device__ __forceinline__ void add_product(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    lo = __fadd_rn(lo, __fmaf_rn(a, b, -p));
+    add(p);
+  }
+  __device__ __forceinline__ void add_lane(int o) {
+    const float h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+    lo = __fadd_rn(lo, l);
+    add(h);
+  }
+};
 
 __device__ __forceinline__ float dot3(float x, float y, float z, float4 u) {
   return x * u.x + y * u.y + z * u.z;
@@ -421,6 +445,11 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
     v = warp_sum_f(v);
     if (lane == 0) s_red[k][wid] = static_cast<double>(v);
   };
+  // ... in two words, which publish adds: a conversion occupies the float64 pipe
+  // for the whole warp, so not one in each
+  auto put2 = [&](int k, const Sum2& v) {
+    if (lane == 0) *reinterpret_cast<float2*>(&s_red[k][wid]) = make_float2(v.hi, v.lo);
+  };
   // x += alpha p, compensated (x and its low part of 4-slot rounds in tensor
   // memory)
   auto kahan = [&](float al, float p, float& s, float& c) {
@@ -588,8 +617,8 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   // ---- the last warp's part ----
   uint32_t gen = 0, nsum = 0;  // exchanges, sums
   // Publishes the block's partials of the planes in mask (arrive: once the
-  // other warps have arrived with theirs)
-  auto publish = [&](int mask, bool arrive) {
+  // other warps have arrived with theirs; words2: from put2)
+  auto publish = [&](int mask, bool arrive, bool words2 = false) {
     ++nsum;
     if (arrive) bar_sync1();
     __syncwarp();
@@ -598,7 +627,12 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
 #pragma unroll 1
     for (int k = 0; k < 3; ++k)
       if (mask >> k & 1) {
-        const double v = warp_sum_d(lane < nw ? s_red[k][lane] : 0.0);
+        double v = 0.0;
+        if (lane < nw) {
+          const float2 w = *reinterpret_cast<const float2*>(&s_red[k][lane]);
+          v = words2 ? static_cast<double>(w.x) + static_cast<double>(w.y) : s_red[k][lane];
+        }
+        v = warp_sum_d(v);
         if (CLUSTER) {
           if (lane < G)
             send_f64(map_rank(smem_u32(&s_sum[nsum & 1][k][rank]), base + lane), map_rank(sbar, base + lane), v);
@@ -718,19 +752,24 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   // The Chebyshev interval of this problem: lambda_max of S = D^-1/2 A D^-1/2
   // by Lanczos steps from a fixed start vector (Golub & Van Loan, sec. 10.1).
   // One application and one sum a step: with q.w, w.w and q.q of
-  // w = S q - b q_prev, a = q.w / q.q and b = |w - a q| follow together.  As
+  // w = S q - b q_prev, a = q.w / q.q and b = |w - a q| follow together, from
+  // sums of 48 bits.  (q.q has to be summed: taken as 1, or carried on from the
+  // step before, its error grows by a^2 / b^2 a step.)  Where little is left of
+  // the difference b is summed from the vector itself: a small b does not say
+  // that the space is exhausted (a uniform spectrum with one stiff constraint has
+  // one in the first step).  As
   // kernels of their own the 24 steps and the interval took 730 us a Newton
   // iteration, here 245 us (72,000 ARAP constraints on the grid): a step costs
   // two meetings, not four launches.
   auto estimate = [&]() {
     auto sqd = [&](int c) { return a.unit_dinv ? 1.0f : sqrtf(ad(c).y); };
     {
-      float qq = 0.0f;
+      Sum2 qq;
       auto seed = [&](int c) {
         uint32_t h = static_cast<uint32_t>(perm(c)) * 2654435761u;
         h ^= h >> 15;
         const float v = 0.5f + (h & 0xffff) * (1.0f / 65536.0f);
-        qq += v * v;
+        qq.add_product(v, v);
         return v;
       };
       rounds([&](int c, bool ok, uint32_t t, uint32_t) { tm_st2(t, 0.0f, ok ? seed(c) : 0.0f); });
@@ -739,11 +778,13 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         gd(c) = seed(c);
       });
       tm_wait_st();
-      put(2, qq);
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) qq.add_lane(o);
+      put2(2, qq);
       if (!syncw) {
         bar_arrive1();
       } else {
-        publish(4, true);
+        publish(4, true, true);
         bool ok = true;
         const double v = total(2, ok);
         if (lane == 0) {
@@ -756,6 +797,11 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
       __syncthreads();
       if (!s_ok) return false;
     }
+    auto set_b = [&](int j, double b) {
+      s_lb[j] = b;
+      s_inv = b > 0.0 ? static_cast<float>(1.0 / b) : 0.0f;
+      s_bprev = static_cast<float>(b);
+    };
 #pragma unroll 1
     for (int j = 0; j < kLanczosSteps; ++j) {
       const float aj = s_scal, inv = s_inv, bprev = s_bprev;
@@ -774,40 +820,71 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
       rest([&](int c) { next(c, gr(c), gd(c)); });
       tm_wait_st();
       __syncthreads();
-      float qw = 0.0f, ww = 0.0f, qq = 0.0f;
+      Sum2 qw, ww, qq;
       auto epi = [&](int c, float q, float d, float y) {
         const float w = sqd(c) * (y + ad(c).x * sm_f(a.o.x, c)) - bprev * d;
-        qw += q * w;
-        ww += w * w;
-        qq += q * q;
+        qw.add_product(q, w);
+        ww.add_product(w, w);
+        qq.add_product(q, q);
         return w;
       };
       if (!apply(false, epi, []() {}, []() {})) return false;
-      put(0, qw);
-      put(1, ww);
-      put(2, qq);
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) {
+        qw.add_lane(o);
+        ww.add_lane(o);
+        qq.add_lane(o);
+      }
+      put2(0, qw);
+      put2(1, ww);
+      put2(2, qq);
       if (!syncw) {
         bar_arrive1();
       } else {
-        publish(7, true);
+        publish(7, true, true);
         bool ok = true;
         const double tqw = total(0, ok), tww = total(1, ok), tqq = total(2, ok);
         if (lane == 0) {
           if (!ok) s_ok = 0;
           const double av = tqq > 0.0 ? tqw / tqq : 0.0;
-          // below 1e-5 w.w the difference is the rounding of the float32
-          // vectors: the space is exhausted
-          const double b2 = tww - 2.0 * av * tqw + av * av * tqq;
-          const double bv = b2 > 1e-5 * tww ? sqrt(b2) : (b2 == b2 ? 0.0 : b2);
+          const double b2 = tww - (2.0 * tqw - av * tqq) * av;
           s_la[j] = av;
-          s_lb[j] = bv;
           s_scal = static_cast<float>(av);
-          s_inv = bv > 0.0 ? static_cast<float>(1.0 / bv) : 0.0f;
-          s_bprev = static_cast<float>(bv);
+          // (in the limits, so that the squares' float32 words hold)
+          s_stop = !(b2 > 1e-6 * tww && tww > 1e-20 && tww < 1e30);
+          if (!s_stop) set_b(j, sqrt(b2));
         }
       }
       __syncthreads();
       if (!s_ok) return false;
+      if (s_stop) {  // |w - a q| from the vector
+        const float av = s_scal;
+        double yy = 0.0;
+        auto left = [&](float q, float w) {
+          const double y = w - av * q;
+          yy += y * y;
+        };
+        rounds([&](int c, bool ok, uint32_t t, uint32_t) {
+          const float2 v = tm_ld2(t);
+          if (ok) left(v.x, v.y);
+        });
+        rest([&](int c) { left(gr(c), gd(c)); });
+        yy = warp_sum_d(yy);
+        if (lane == 0) s_red[0][wid] = yy;
+        if (!syncw) {
+          bar_arrive1();
+        } else {
+          publish(1, true);
+          bool ok = true;
+          const double v = total(0, ok);
+          if (lane == 0) {
+            if (!ok) s_ok = 0;
+            set_b(j, sqrt(v));
+          }
+        }
+        __syncthreads();
+        if (!s_ok) return false;
+      }
     }
     if (syncw) {
       const double lmax = lanczos_lmax(s_la, s_lb, kLanczosSteps);
