@@ -17,6 +17,7 @@
 #include "local.cuh"
 #include "mpnn.cuh"
 #include "rap.cuh"
+#include "cheb_dev.cuh"
 #include "dcg_plan.h"
 #include "solver.h"
 #include "structure.h"
@@ -703,6 +704,12 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
       std::memcpy(contrib_off, g.contrib_off.data(), sizeof(int32_t) * g.contrib_off.size());
     }
   });
+}
+
+int mgpbd_host_lanczos_lmax(const double* a, const double* b, int32_t k, double* lmax) {
+  if (!a || !b || k < 1 || k > mgpbd::kMaxLanczos || !lmax) return MGPBD_EINVAL;
+  *lmax = mgpbd::jdev::host_lanczos_lmax(a, b, k);
+  return MGPBD_OK;
 }
 
 int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv,

@@ -16,8 +16,11 @@ namespace jdev {
 // off-diagonal b) lie below x: the leading minors of T - x I alternate in sign,
 // starting negative.  The minors by their three-term recurrence, T scaled by
 // 1 / s (s bounds its eigenvalues, so the minors of 32 rows stay in range): no
-// division, whose latency was most of the search's time.
-__device__ inline bool all_below(const double* a, const double* b, int k, double x, double inv_s) {
+// division, whose latency was most of the search's time.  (Eigenvalues that all
+// lie within 1e-13 s of x, of 24 rows, or 3e-10 s, of 32, may make a minor 0: x
+// then counts as not above them.)
+__host__ __device__ inline bool all_below(const double* a, const double* b, int k, double x,
+                                          double inv_s) {
   double p0 = 1.0, p1 = (a[0] - x) * inv_s;
   bool ok = p1 < 0.0;
   for (int i = 1; i < k; ++i) {
@@ -56,6 +59,29 @@ __device__ inline double lanczos_lmax(const double* a, const double* b, int k) {
     const int f = all ? __ffs(all) - 1 : 32;
     const double nlo = f == 0 ? lo : __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
     const double nhi = f == 32 ? hi : __shfl_sync(0xffffffffu, x, f < 32 ? f : 31);
+    lo = nlo;
+    hi = nhi;
+  }
+  return hi;
+}
+
+// ... on the host, one point after the other
+inline double host_lanczos_lmax(const double* a, const double* b, int k) {
+  double lo = 1e300, hi = -1e300;
+  for (int i = 0; i < k; ++i) {
+    const double r = (i > 0 ? std::fabs(b[i - 1]) : 0.0) + (i + 1 < k ? std::fabs(b[i]) : 0.0);
+    lo = std::fmin(lo, a[i] - r);
+    hi = std::fmax(hi, a[i] + r);
+  }
+  const double s = std::fmax(std::fabs(lo), std::fabs(hi));
+  if (!(hi >= lo) || !std::isfinite(hi) || !std::isfinite(lo)) return NAN;
+  const double inv_s = s > 0.0 ? 1.0 / s : 1.0;
+  for (int it = 0; it < 60 && hi - lo > 1e-12 * std::fmax(1.0, std::fabs(hi)); ++it) {
+    const double step = (hi - lo) * (1.0 / 33.0);
+    auto point = [&](int l) { return l == 31 ? hi - step : lo + step * (l + 1); };
+    int f = 0;
+    while (f < 32 && !all_below(a, b, k, point(f), inv_s)) ++f;
+    const double nlo = f == 0 ? lo : point(f - 1), nhi = f == 32 ? hi : point(f);
     lo = nlo;
     hi = nhi;
   }

@@ -641,6 +641,11 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
                         int32_t* c_indices, int32_t* contrib_idx,
                         int32_t* contrib_off);
 
+/* Largest eigenvalue of the symmetric tridiagonal (diagonal a (k), off-diagonal
+ * b (k - 1)), k <= 32, by the search of the Chebyshev interval's kernels, its
+ * points one after the other.  Host arrays. */
+int mgpbd_host_lanczos_lmax(const double* a, const double* b, int32_t k, double* lmax);
+
 /* y = (J W J^T + alpha~) x in float64 by way of the spatial partition that
  * the persistent dual CG runs on: nt constraints t_i (nt,4), the length
  * constraints from n4 on, rest positions x_ref (nv,3), prob (nt, or NULL) the
