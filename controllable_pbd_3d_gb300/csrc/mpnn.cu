@@ -396,6 +396,9 @@ __global__ void __launch_bounds__(kT) k_net_out_bwd(NetGraph g, const float* __r
 // are read once for them, with v and u of a row side by side (a launch each,
 // with the roots and quotients in every thread, took 28 us a sample).
 constexpr int kNetSamples = 8;
+// the norms of as many samples at once (along grid.y)
+constexpr int kNetNorms = 256;
+constexpr int kNormBlocks = 64;  // most blocks of a norm
 
 // u and v of samples s0 .. of a row: uv[row][0..7] = v, uv2[row][0..7] = u
 __global__ void k_net_uv(NetGraph g, NetFields f, int s0, int ns, const NetSigma* __restrict__ sg,
@@ -818,8 +821,8 @@ void CoarseNet::ensure(const NetGraph& g) {
   wcap_.alloc(n);
   wv_.alloc(n);
   dw_.alloc(n);
-  vs_.alloc((int64_t)n * kNetSamples);
-  us_.alloc((int64_t)n * kNetSamples);
+  sigs_.alloc(kNetNorms);
+  spart_.alloc(kNetNorms * kNormBlocks);
   wpart_.alloc((int64_t)kWgradBlocks * kBigPart);
   cap_ = n;
 }
@@ -929,25 +932,27 @@ void CoarseNet::loss_grad(const NetGraph& g, const float* samples, int32_t n_sam
     k_net_squash<<<ceil_div(n, kT), kT, 0, s>>>(n, y_.p, wcap_.p, wv_.p, dw_.p);
     MGPBD_CHECK_LAUNCH();
     MGPBD_CUDA(cudaMemsetAsync(gy_.p, 0, sizeof(float) * n, s));
-    const int sb = std::min(64, std::max(1, ceil_div(n, kT)));
-    const NetFields fields{samples, first % n_samples, n_samples};
-    if (S > sig_cap_) {
-      sigs_.alloc(S);
-      spart_.alloc((int64_t)S * 64);
-      sig_cap_ = S;
-    }
-    k_net_sumsq<<<dim3(sb, S), kT, 0, s>>>(n, fields, g.diag_inv, spart_.p);
-    MGPBD_CHECK_LAUNCH();
-    k_net_sigma<<<S, kT, 0, s>>>(spart_.p, sb, n, sigs_.p);
-    MGPBD_CHECK_LAUNCH();
-    for (int32_t k = 0; k < S; k += kNetSamples) {
-      const int ns = std::min(kNetSamples, S - k);
-      k_net_uv<<<ceil_div(n, kT), kT, 0, s>>>(g, fields, k, ns, sigs_.p, wv_.p, vs_.p, us_.p);
+    const int sb = std::min(kNormBlocks, std::max(1, ceil_div(n, kT)));
+    // w u and u of the samples: workspace that the layers' backward pass fills
+    // afterwards
+    static_assert(kNetSamples <= kNetF, "the samples' workspace");
+    float *vs = gself_.p, *us = q_.p;
+    for (int32_t k0 = 0; k0 < S; k0 += std::min(kNetNorms, S - k0)) {
+      const int nk = std::min(kNetNorms, S - k0);
+      const NetFields fields{samples, (int32_t)((first + (int64_t)k0) % n_samples), n_samples};
+      k_net_sumsq<<<dim3(sb, nk), kT, 0, s>>>(n, fields, g.diag_inv, spart_.p);
       MGPBD_CHECK_LAUNCH();
-      k_net_wloss<<<ob, kT, 0, s>>>(g, ah_.p, dw_.p, ns, vs_.p, us_.p, scale, gy_.p, part_.p);
+      k_net_sigma<<<nk, kT, 0, s>>>(spart_.p, sb, n, sigs_.p);
       MGPBD_CHECK_LAUNCH();
-      k_net_sum<<<1, kT, 0, s>>>(part_.p, ob, loss_dev, 1);
-      MGPBD_CHECK_LAUNCH();
+      for (int k = 0; k < nk; k += kNetSamples) {
+        const int ns = std::min(kNetSamples, nk - k);
+        k_net_uv<<<ceil_div(n, kT), kT, 0, s>>>(g, fields, k, ns, sigs_.p, wv_.p, vs, us);
+        MGPBD_CHECK_LAUNCH();
+        k_net_wloss<<<ob, kT, 0, s>>>(g, ah_.p, dw_.p, ns, vs, us, scale, gy_.p, part_.p);
+        MGPBD_CHECK_LAUNCH();
+        k_net_sum<<<1, kT, 0, s>>>(part_.p, ob, loss_dev, 1);
+        MGPBD_CHECK_LAUNCH();
+      }
     }
     k_net_head_bwd<<<ceil_div((int64_t)n * kNetF, kT), kT, 0, s>>>(n, gy_.p, h3_.p, p_.p, gz_.p);
     MGPBD_CHECK_LAUNCH();

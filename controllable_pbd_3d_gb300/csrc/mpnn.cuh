@@ -101,9 +101,7 @@ class CoarseNet {
   int32_t cap_ = -1;
   // workspace (cap_ rows)
   DevBuf<double> part_, spart_;
-  DevBuf<NetSigma> sigma_, sigs_;  // of the forward field, of a batch
-  int32_t sig_cap_ = 0;
-  DevBuf<float> vs_, us_;  // w u and u of eight samples side by side
+  DevBuf<NetSigma> sigma_, sigs_;  // of the forward field, of some of a batch
   DevBuf<float> u_, a1_, y_, e_, h3_, gy_, gz_, gself_, q_, wpart_;
   DevBuf<float> ah_;    // Ah = S A S per nonzero, written by layer 1
   DevBuf<float> feat_;  // the feature field sqrt(diag A)
