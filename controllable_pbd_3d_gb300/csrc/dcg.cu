@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
         return w;
       };
       if (!apply(false, epi, []() {}, []() {})) return false;
-#pragma unroll 1
+#pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         qw.add_lane(o);
         ww.add_lane(o);
