@@ -34,7 +34,7 @@ struct DcgDev {
   const DWarp* warps = nullptr;
   unsigned char* rows = nullptr;  // kDRow bytes each
   float4* tg = nullptr;           // 3 planes of nc float4 (length constraints: plane 0 only)
-  float2* ad = nullptr;           // (nc) alpha~, 1/diag in plan order
+  float2* ad = nullptr;           // (nc) alpha~ (as of the solve), 1/diag in plan order
   float* x = nullptr;             // (nc) CG vectors in plan order
   float* xc = nullptr;
   float* r = nullptr;
