@@ -717,11 +717,16 @@ int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32
                                int32_t n_blocks, int32_t cluster, int32_t threads,
                                int32_t smem_limit, const float* gradC, const float* invm,
                                const float* alpha, const float* x, double* y, int32_t* info) {
-  if (!t_i || nt <= 0 || n4 < 0 || n4 > nt || nv <= 0 || !x_ref || n_prob <= 0 || n_blocks < 0 || (n_blocks == 0 && (!cluster || !prob)) ||
-      n_blocks > (cluster ? mgpbd::kDMaxCluster : 255) || threads < 128 ||
-      threads > mgpbd::kDMaxThreads || threads % 128 != 0 || !gradC || !invm || !alpha || !x || !y ||
-      !info)
+  if (!t_i || nt <= 0 || n4 < 0 || n4 > nt || nv <= 0 || !x_ref || n_prob <= 0 || n_blocks < 0 ||
+      (n_blocks == 0 && (!cluster || !prob)) || n_blocks > (cluster ? mgpbd::kDMaxCluster : 255) ||
+      threads < 128 || threads > mgpbd::kDMaxThreads || threads % 128 != 0 || !gradC || !invm ||
+      !alpha || !x || !y || !info)
     return MGPBD_EINVAL;
+  for (int32_t c = 0; c < nt; ++c) {
+    if (prob && (prob[c] < 0 || prob[c] >= n_prob)) return MGPBD_EINVAL;
+    for (int l = 0; l < (c < n4 ? 4 : 2); ++l)
+      if (t_i[4LL * c + l] < 0 || t_i[4LL * c + l] >= nv) return MGPBD_EINVAL;
+  }
   return guarded([&] {
     mgpbd::DcgPlan p;
     mgpbd::DcgPlaces places = mgpbd::dcg_places(n_prob, std::max(n_blocks, 1));
