@@ -722,10 +722,15 @@ int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32
       threads < 128 || threads > mgpbd::kDMaxThreads || threads % 128 != 0 || !gradC || !invm ||
       !alpha || !x || !y || !info)
     return MGPBD_EINVAL;
+  std::vector<int32_t> owner(nv, -1);
   for (int32_t c = 0; c < nt; ++c) {
-    if (prob && (prob[c] < 0 || prob[c] >= n_prob)) return MGPBD_EINVAL;
-    for (int l = 0; l < (c < n4 ? 4 : 2); ++l)
-      if (t_i[4LL * c + l] < 0 || t_i[4LL * c + l] >= nv) return MGPBD_EINVAL;
+    const int32_t body = prob ? prob[c] : 0;
+    if (body < 0 || body >= n_prob) return MGPBD_EINVAL;
+    for (int l = 0; l < (c < n4 ? 4 : 2); ++l) {
+      const int32_t v = t_i[4LL * c + l];
+      if (v < 0 || v >= nv || (owner[v] >= 0 && owner[v] != body)) return MGPBD_EINVAL;
+      owner[v] = body;
+    }
   }
   return guarded([&] {
     mgpbd::DcgPlan p;

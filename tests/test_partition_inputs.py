@@ -40,3 +40,9 @@ def test_a_vertex_that_is_not_there_is_refused(bad):
   xr, c, n4, prob, g, w, alpha, x = pack()
   c[5, 3] = bad
   assert run_plan(xr, c, n4, prob, 2, 4, True, 256, SMEM, g, w, alpha, x)[0] == -1
+
+
+def test_bodies_that_share_a_vertex_are_refused():
+  xr, c, n4, prob, g, w, alpha, x = pack()
+  c[-1, 2] = c[0, 0]
+  assert run_plan(xr, c, n4, prob, 2, 4, True, 256, SMEM, g, w, alpha, x)[0] == -1
