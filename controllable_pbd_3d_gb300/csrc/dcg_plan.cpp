@@ -249,7 +249,9 @@ bool build_dcg_plan(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv, cons
       for (int k = 0; k < 3; ++k) {
         float s = 0.0f;
         for (int l = 0; l < n; ++l) s += x_ref[3LL * t_i[4LL * c + l] + k];
-        a.c[k] = s / n;
+        // (a coordinate that is not finite has no place; ordered by it, the
+        // bisection would take one constraint a pass)
+        a.c[k] = std::isfinite(s) ? s / n : 0.0f;
       }
     }
   }

@@ -46,3 +46,26 @@ def test_bodies_that_share_a_vertex_are_refused():
   xr, c, n4, prob, g, w, alpha, x = pack()
   c[-1, 2] = c[0, 0]
   assert run_plan(xr, c, n4, prob, 2, 4, True, 256, SMEM, g, w, alpha, x)[0] == -1
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf, 3e38])
+def test_rest_positions_that_are_not_finite(bad):
+  """They are only where the mesh is cut: any place will do, and it takes no
+  longer (ordered by NaN, 100,000 constraints took 15 s)."""
+  import time
+  xr, t = meshgen.hex_grid_tets(27, 27, 27)
+  c = np.ascontiguousarray(np.asarray(t, np.int32).reshape(-1, 4))
+  rng = np.random.default_rng(1)
+  g = rng.standard_normal((len(c), 4, 3)).astype(np.float32)
+  w = np.ones(len(xr), np.float32)
+  alpha = rng.random(len(c)).astype(np.float32)
+  x = rng.standard_normal(len(c)).astype(np.float32)
+  for part in (slice(None), slice(0, 40)):
+    xx = xr.astype(np.float32)
+    xx[part] = bad
+    t0 = time.perf_counter()
+    rc, y, _ = run_plan(xx, c, len(c), None, 1, 152, False, 512, SMEM, g, w, alpha, x)
+    assert time.perf_counter() - t0 < 5.0
+    assert rc == 0
+    ref, size = apply64(c, len(c), g, w, alpha, x)
+    assert np.all(np.abs(y - ref) <= 1e-13 * size)
