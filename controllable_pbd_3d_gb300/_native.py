@@ -182,6 +182,7 @@ _SIGS = {
     'mgpbd_host_aggregate': (C.c_int, [vp, i32, i32, vp, P_i32]),
     'mgpbd_host_tet_hierarchy': (C.c_int, [vp, i32, i32, i32, P_i32, vp, vp]),
     'mgpbd_host_lanczos_lmax': (C.c_int, [vp, vp, i32, vp]),
+    'mgpbd_host_place_bodies': (C.c_int, [i32, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp]),
     'mgpbd_host_partition_apply': (C.c_int, [vp, i32, i32, i32, vp, vp, i32, i32, i32, i32, i32, vp,
                                              vp, vp, vp, vp, vp]),
     'mgpbd_host_galerkin': (C.c_int, [i32, vp, vp, vp, vp, i32, P_i64, P_i64, vp, vp, vp, vp]),

@@ -712,6 +712,26 @@ int mgpbd_host_lanczos_lmax(const double* a, const double* b, int32_t k, double*
   return MGPBD_OK;
 }
 
+int mgpbd_host_place_bodies(int32_t n, const double* entries, const double* softness, int32_t n16,
+                            int32_t n8, int32_t n4, int32_t choice, int32_t* n_choices,
+                            int32_t* cluster, int32_t* blocks, int32_t* first, int32_t* size) {
+  if (n <= 0 || !entries || n16 < 0 || n8 < 0 || n4 < 0 || choice < 0 || !n_choices || !cluster ||
+      !blocks || !first || !size)
+    return MGPBD_EINVAL;
+  return guarded([&] {
+    const auto all = mgpbd::dcg_place_bodies(
+        std::vector<double>(entries, entries + n),
+        softness ? std::vector<double>(softness, softness + n) : std::vector<double>(), n16, n8, n4);
+    *n_choices = static_cast<int32_t>(all.size());
+    if (choice >= *n_choices) return;
+    const mgpbd::DcgPlaces& p = all[choice];
+    *cluster = p.cluster;
+    *blocks = p.blocks;
+    std::copy(p.first.begin(), p.first.end(), first);
+    std::copy(p.size.begin(), p.size.end(), size);
+  });
+}
+
 int mgpbd_host_partition_apply(const int32_t* t_i, int32_t nt, int32_t n4, int32_t nv,
                                const float* x_ref, const int32_t* prob, int32_t n_prob,
                                int32_t n_blocks, int32_t cluster, int32_t threads,

@@ -646,6 +646,16 @@ int mgpbd_host_galerkin(int32_t n, const int32_t* indptr, const int32_t* indices
  * points one after the other.  Host arrays. */
 int mgpbd_host_lanczos_lmax(const double* a, const double* b, int32_t k, double* lmax);
 
+/* How the per-body CG arranges n packed bodies on clusters of 16, 8 or 4 blocks
+ * of which n16, n8 and n4 are resident at once (0: none), from their vertex
+ * entries and, if not NULL, their softness: the arrangement `choice` of
+ * n_choices, best first -- body k on size[k] of `blocks` blocks from first[k]
+ * on, in clusters of `cluster`.  Host arrays. */
+int mgpbd_host_place_bodies(int32_t n, const double* entries, const double* softness,
+                            int32_t n16, int32_t n8, int32_t n4, int32_t choice,
+                            int32_t* n_choices, int32_t* cluster, int32_t* blocks,
+                            int32_t* first, int32_t* size);
+
 /* y = (J W J^T + alpha~) x in float64 by way of the spatial partition that
  * the persistent dual CG runs on: nt constraints t_i (nt,4), the length
  * constraints from n4 on, rest positions x_ref (nv,3), prob (nt, or NULL) the
