@@ -98,7 +98,10 @@ class BodyBatch:
     self.per_body = fast_cheb if per_body is None else bool(per_body)
     if self.per_body:
       self.solver.set_bodies(self.vert_off, self.segments())
-      self.solver.set_body_compliance([b.compliance for b in self.bodies])
+      # (a hint: bodies whose compliance is no measure of their stiffness go without)
+      hint = np.array([b.compliance for b in self.bodies], np.float64).astype(np.float32)
+      if np.isfinite(hint).all() and (hint >= 0).all():
+        self.solver.set_body_compliance(hint)
 
   def constraint_body(self) -> np.ndarray:
     """Body id of every constraint: one per tet (ARAP), or the volume
