@@ -2307,6 +2307,9 @@ void Solver::solve_bodies_graph() {
                              cudaMemcpyDeviceToHost, s));
   MGPBD_CUDA(cudaStreamSynchronize(s));
   const BodyLoop& L = *h_body_loop_;
+  // each body had an interval of its own; a solve of the whole pack that comes
+  // next needs one of all (a replayed graph does not pass jform_setup)
+  if (dcg_ready_ && p_.body_cg) estimate_next_ = true;
   g_launches.fetch_add(body_graph_init_launches_ + body_graph_body_launches_ * L.ite);
   status_ = L.status;
   stats_.newton_iters = L.ite;

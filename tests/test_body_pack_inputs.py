@@ -1,4 +1,5 @@
-"""Packed bodies whose compliances say nothing about stiffness."""
+"""Packed bodies: compliances that say nothing about stiffness, and direct solves
+beside the captured substep."""
 
 import numpy as np
 import pytest
@@ -23,3 +24,26 @@ def test_any_compliance_is_taken(cuda, compliance):
   if compliance < 1.0:  # (1e39 is not a float32)
     b.step(0)
     assert bool(cuda.isfinite(b.x).all())
+
+
+@pytest.mark.gpu
+def test_direct_solves_between_substeps(cuda):
+  """A solve of the whole pack after a substep that ran from its graph: the
+  interval has to be that of all bodies, also of the one a hundred times
+  lighter than the first."""
+  from test_dual_partition import residual
+  torch = cuda
+  bodies = random_bodies(2, seed=6, dims=(5, 7), compliance=(1.0, 1.0))
+  bodies[1].invm = bodies[1].invm * np.float32(100.0)
+  b = BodyBatch(bodies, G, DT, **KW)
+  b.init()
+  s = b.solver
+  n4 = int((s.constraint_types != 1).sum())
+  for i in range(3):
+    b.step(i)
+    s._b_gpu.copy_(torch.randn(s.n_tets, device='cuda', generator=torch.Generator('cuda').manual_seed(i)))
+    its = s._gpu_solver.solve(s._b_gpu, s._dlam_gpu)
+    rel, floor = residual(s, n4)
+    print('its', i, its, rel, floor)
+    assert its < 3000
+    assert rel <= 1e-6 + floor
