@@ -395,14 +395,23 @@ def roofline_from_steps(st, nt, nv, degree, hbm_peak, peak_kind, size=40, constr
 def roofline_of_solver(*args):
   """`roofline_from_steps` for the solvers timed here: their dual solves run
   on the partitioned kernel (`k_dcg`), which holds its part of the operator on
-  the chip, so the DRAM traffic measured on `k_jcg` says nothing of it."""
+  the chip.  Neither the DRAM traffic measured on `k_jcg` nor a fraction of the
+  HBM rate says anything of it (DRAM is idle): what bounds it is the meetings of
+  the blocks, degree + 2 a CG iteration, so the line gives the time of one.  The
+  library's `cg_path`, the memory an SM's share would take of `k_jcg`, is left
+  out for the same reason."""
   roof = roofline_from_steps(*args)
+  degree = args[3]
   for r in (roof, roof.get('other') or {}):
     if r.get('kernel', '').startswith('k_jcg'):
       r['kernel'] = r['kernel'].replace('k_jcg<0>', 'k_dcg').replace('k_jcg<1>', 'k_dcg')
       for k in ('traffic_source', 'traffic_over_algorithmic', 'dram_gbs', 'dram_frac'):
         r.pop(k, None)
-      r['traffic'] = None
+      r['algorithmic_gbs'] = r['achieved']
+      r.update(bound='exchange between blocks', achieved=None, peak=None, unit=None, frac=None,
+               peak_kind=None, traffic=None, meetings_per_cg_iteration=degree + 2,
+               us_per_meeting=round(r['us_per_cg_iteration'] / (degree + 2), 2))
+      r.pop('cg_path', None)
       r['working_set_note'] = ('operator data in tensor and shared memory as far as they hold it, the '
                                'rest from L2: the rate is on-chip, not HBM')
   return roof
