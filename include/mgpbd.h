@@ -231,9 +231,12 @@ typedef struct mgpbd_stats {
 } mgpbd_stats;
 
 #define MGPBD_CGPATH_KERNELS 0      /* one kernel (or graph node) per operation */
-#define MGPBD_CGPATH_PERSISTENT 1   /* one persistent kernel per solve, the
-                                       operator (persistent 1: what does not
-                                       fit on the chip) read from L2           */
+#define MGPBD_CGPATH_PERSISTENT 1   /* one persistent kernel per solve; an SM's
+                                       share of the operator is more than its
+                                       shared memory.  (persistent 2 reads it
+                                       from L2; persistent 1 has tensor memory
+                                       beside and reads from L2 only what both
+                                       do not hold)                            */
 #define MGPBD_CGPATH_STAGED 2       /* the same, an SM's share of the operator
                                        fits in its shared memory               */
 #define MGPBD_CGPATH_PRIMAL 3       /* primal system, one cooperative kernel    */
