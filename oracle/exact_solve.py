@@ -155,16 +155,19 @@ class ExactDualSolve:
 
 
 def chebyshev_pcg(apply_A, b, degree=8, lo=1e-3, scale=None, rel_tol=1e-6, tol_abs=0.0,
-                  maxiter=6000, lmax=None, x0=None):
+                  maxiter=6000, lmax=None, x0=None, work=np.longdouble):
   """CG preconditioned by a degree-`degree` Chebyshev polynomial in S A
   (S = diag(scale), or the identity) on [lo * 1.02 lmax, 1.02 lmax], lmax
   the largest eigenvalue of S A (Lanczos to 1e-10 unless given), from
   x = 0 (or x0: the library's warm start), until |r| < max(tol_abs,
   rel_tol |b|): the linear solve of the library's FAST mode in float64.
+  work: the vectors' type.  On a stiff system the iterations of a float64 CG
+  follow its rounding (the order of a row's products alone moves 460 of them by
+  up to 3 %), so counts that are to be compared need more.
   Returns (x, iterations)."""
-  b = np.asarray(b, np.float64)
+  b = np.asarray(b, work)
   n = len(b)
-  sc = np.ones(n) if scale is None else np.asarray(scale, np.float64)
+  sc = np.ones(n, work) if scale is None else np.asarray(scale, work)
   if lmax is None:
     op = sla.LinearOperator((n, n), matvec=lambda v: np.sqrt(sc) * apply_A(np.sqrt(sc) * v),
                             dtype=np.float64)
@@ -187,7 +190,7 @@ def chebyshev_pcg(apply_A, b, degree=8, lo=1e-3, scale=None, rel_tol=1e-6, tol_a
       rho = rho_n
     return x
 
-  x = np.zeros(n) if x0 is None else np.array(x0, np.float64)
+  x = np.zeros(n, work) if x0 is None else np.array(x0, work)
   r = b.copy() if x0 is None else b - apply_A(x)
   tol = max(tol_abs, rel_tol * np.linalg.norm(b))
   if np.linalg.norm(r) < tol:
@@ -210,14 +213,15 @@ def chebyshev_pcg(apply_A, b, degree=8, lo=1e-3, scale=None, rel_tol=1e-6, tol_a
 
 
 def chebyshev_pcg_bodies(apply_A, b, bodies, degree=8, lo=1e-3, rel_tol=1e-6, tol_abs=0.0,
-                         maxiter=6000, lmax=None):
+                         maxiter=6000, lmax=None, work=np.longdouble):
   """One Chebyshev-preconditioned CG per body on a block-diagonal A, in
   lockstep with one shared polynomial (lmax of the whole A), as the
   library's per-body kernel runs them: each body's dot products, alpha,
   beta and stopping test (|r_b| < max(tol_abs, rel_tol |b_b|)) are its own,
   and a body that stops keeps its x and r.  bodies: one index array per
-  body (together a partition).  Returns (x, per-body iterations)."""
-  b = np.asarray(b, np.float64)
+  body (together a partition).  work: as above.  Returns (x, per-body
+  iterations)."""
+  b = np.asarray(b, work)
   n = len(b)
   if lmax is None:
     op = sla.LinearOperator((n, n), matvec=apply_A, dtype=np.float64)
@@ -241,7 +245,7 @@ def chebyshev_pcg_bodies(apply_A, b, bodies, degree=8, lo=1e-3, rel_tol=1e-6, to
     return x
 
   nb = len(bodies)
-  x = np.zeros(n)
+  x = np.zeros(n, work)
   r = b.copy()
   tol = [max(tol_abs, rel_tol * np.linalg.norm(b[ix])) for ix in bodies]
   done = [bool(np.linalg.norm(r[ix]) < tol[k]) for k, ix in enumerate(bodies)]

@@ -771,7 +771,7 @@ class MGPBDOracle:
         x0 = self.dlam_prev if (self.warm_substep and ite == 0) else None
         dlam, it = chebyshev_pcg(lambda v: al * v + J @ (w3 * (Jt @ v)), b,
                                  rel_tol=self.rel_tol_cg, tol_abs=self.tol_cg,
-                                 maxiter=self.maxiter_cg, x0=x0)
+                                 maxiter=self.maxiter_cg, x0=x0, work=np.float64)
         if self.warm_substep and ite == 0:
           self.dlam_prev = dlam.copy()
       else:
