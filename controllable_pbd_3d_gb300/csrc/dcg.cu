@@ -759,8 +759,8 @@ __global__ void __launch_bounds__(kDMaxThreads, 1) k_dcg(DArgs a) {
   // that the space is exhausted (a uniform spectrum with one stiff constraint has
   // one in the first step).  As
   // kernels of their own the 24 steps and the interval took 730 us a Newton
-  // iteration, here 245 us (72,000 ARAP constraints on the grid): a step costs
-  // two meetings, not four launches.
+  // iteration, here 245 us (72,000 ARAP constraints on the grid; 250 with the
+  // sums' second words): a step costs two meetings, not four launches.
   auto estimate = [&]() {
     auto sqd = [&](int c) { return a.unit_dinv ? 1.0f : sqrtf(ad(c).y); };
     {

@@ -681,10 +681,10 @@ __device__ bool cg_beta(CgState* st, const double* p, int blocks, double* beta) 
 enum RowOp { kSpmv = 0, kJacobi = 1, kResidual = 2, kSpmvDot = 3, kJacobiZero = 4, kJacobiDot = 5 };
 
 // The products of a dot operator's rows.  A float64 multiply-add occupies its
-// pipe for a whole warp however few lanes take part: with the first of a row's G
-// lanes finishing it, the products of 718,520 rows took 24 us beside 105 of the
-// sweep itself.  TURNS: the lanes take turns at finishing a row, and their
-// products are added when each has one.
+// pipe for a whole warp however few lanes take part.  TURNS: the lanes take turns
+// at finishing a row, and their products are added when each has one (718,520
+// rows, us a launch with the first of the four lanes / with turns: sweep and
+// product 129 / 125, SpMV and product 128 / 120; a sweep alone 105).
 template <int G, bool TURNS>
 struct RowDot {
   double acc = 0.0;

@@ -1,5 +1,7 @@
-// Device helpers of the cooperative persistent CG kernels (jcg.cu, pcg.cu):
-// the bounded grid barrier and the fixed-order block/grid reductions.
+// Device helpers of the kernels whose blocks wait on one another: the bounded
+// grid barrier and the fixed-order block/grid reductions of the cooperative CG
+// kernels (jcg.cu, pcg.cu), and the timer and the tagged 16-byte accesses of
+// those that wait without a barrier (dcg.cu, sweep.cu, local.cu).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -889,7 +889,7 @@ void Solver::jform_setup(uint32_t* dev_status) {
   launch_jform_prepare(j, inc_ent_.p, gV_.p, jdinv_.p, gT_.p,
                        p_.cheb_scale == MGPBD_CHEB_UNSCALED, stream_);
   if (dcg_ready_) launch_dcg_pack(j, ddev_, dplan_.n_rows, stream_);
-  // k_dcg makes the estimate of its systems itself (245 us against 730 at
+  // k_dcg makes the estimate of its systems itself (250 us against 730 at
   // 72,000 constraints).  After a primal warm start the solve begins up to 1e6
   // |b| away, where the 8th digit of the interval shows in the solution: there
   // it comes from the kernels that always made it.
