@@ -199,6 +199,7 @@ _SIGS = {
     'mgpbd_xpbd_preupdate': (C.c_int, [vp]),
     'mgpbd_xpbd_update': (C.c_int, [vp, i32]),
     'mgpbd_xpbd_synchronize': (C.c_int, [vp]),
+    'mgpbd_xpbd_set_barrier_limit': (C.c_int, [vp, C.c_double]),
     'mgpbd_xpbd_lambdas': (C.c_int, [vp, C.POINTER(vp), C.POINTER(vp)]),
     'mgpbd_xpbd_n_colors': (C.c_int, [vp, P_i32]),
     'mgpbd_vbd_create': (C.c_int, [C.POINTER(VbdParams), C.POINTER(vp)]),
@@ -211,6 +212,7 @@ _SIGS = {
     'mgpbd_vbd_update_vel': (C.c_int, [vp]),
     'mgpbd_vbd_step': (C.c_int, [vp]),
     'mgpbd_vbd_synchronize': (C.c_int, [vp]),
+    'mgpbd_vbd_set_barrier_limit': (C.c_int, [vp, C.c_double]),
     'mgpbd_vbd_omegas': (C.c_int, [vp, vp]),
     'mgpbd_vbd_field': (C.c_int, [vp, i32, C.POINTER(vp), P_i64]),
     'mgpbd_vbd_n_colors': (C.c_int, [vp, P_i32]),

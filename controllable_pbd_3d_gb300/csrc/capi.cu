@@ -904,6 +904,11 @@ int mgpbd_xpbd_synchronize(mgpbd_xpbd_handle h) {
   return guarded([&] { h->impl.synchronize(); });
 }
 
+int mgpbd_xpbd_set_barrier_limit(mgpbd_xpbd_handle h, double seconds) {
+  if (!h) return MGPBD_EINVAL;
+  return guarded([&] { h->impl.set_barrier_limit(seconds); });
+}
+
 int mgpbd_xpbd_lambdas(mgpbd_xpbd_handle h, float** hydro, float** devia) {
   if (!h || !hydro || !devia) return MGPBD_EINVAL;
   *hydro = h->impl.lambda_h();
@@ -935,6 +940,11 @@ int mgpbd_vbd_set_mesh(mgpbd_vbd_handle h, float* x, const float* x_ref, const f
                        const int32_t* t_i, int32_t nv, int32_t nt) {
   if (!h) return MGPBD_EINVAL;
   return guarded([&] { h->impl.set_mesh(x, x_ref, invm, t_i, nv, nt); });
+}
+
+int mgpbd_vbd_set_barrier_limit(mgpbd_vbd_handle h, double seconds) {
+  if (!h) return MGPBD_EINVAL;
+  return guarded([&] { h->impl.set_barrier_limit(seconds); });
 }
 
 int mgpbd_vbd_init(mgpbd_vbd_handle h) {

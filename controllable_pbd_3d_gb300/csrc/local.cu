@@ -33,7 +33,6 @@ constexpr int kVbdWarps = 16;  // (8: 313 us over 32^3 hexes, 16: 232)
 // 24 (with four lanes 10 iterations over 24^3 hexes take 244 us, with eight 196,
 // with sixteen 207, and 302, 313, 463 over 32^3)
 constexpr int kVL = 8;
-constexpr unsigned long long kSpinNs = 4000000000ull;  // grid barrier limit
 
 // 3x3 helpers (row-major m[r][c]); determinant by the first column's
 // cofactors, inverse = adjugate / det
@@ -262,6 +261,7 @@ struct FlowArgs {
   float4* xt;        // position and count of updates of each vertex
   int32_t n_chunks;  // 32 tets of one colour each
   int32_t passes;
+  unsigned long long spin_ns;
   GridSync* gs;
   int32_t* status;
 };
@@ -269,17 +269,19 @@ struct FlowArgs {
 // Waits until each of K vertices has had the update it is wanted with (all are
 // polled at once: one after the other, each would add its own round trip);
 // false once a wait of the grid gave up
-// (a null vertex is one that is not waited for)
+// (a null vertex is one that is not waited for; a limit of 0 gives up at the first
+// poll that finds one missing)
 template <int K>
 __device__ __forceinline__ bool wait_vertices(const float4* const (&p)[K], const uint32_t (&want)[K],
-                                              uint4 (&v)[K], GridSync* gs, int32_t* status) {
+                                              uint4 (&v)[K], unsigned long long spin_ns,
+                                              GridSync* gs, int32_t* status) {
 #pragma unroll
   for (int l = 0; l < K; ++l) {
     v[l].w = want[l];
     if (p[l]) v[l] = pdev::get_tagged(p[l]);
   }
   unsigned long long t0 = 0;
-  for (uint32_t n = 1;; ++n) {
+  for (uint32_t n = spin_ns == 0 ? 1024 : 1;; ++n) {
     bool ready = true;
 #pragma unroll
     for (int l = 0; l < K; ++l) ready = ready && v[l].w == want[l];
@@ -291,7 +293,7 @@ __device__ __forceinline__ bool wait_vertices(const float4* const (&p)[K], const
       if (pdev::ld_relaxed(&gs->err) != 0u) return false;
       const unsigned long long t = pdev::global_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kSpinNs) {
+      if (t - t0 >= spin_ns) {
         atomicExch(&gs->err, 1u);
         atomicOr(reinterpret_cast<unsigned int*>(status), MGPBD_STATUS_SYNC_TIMEOUT);
         return false;
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(32 * kXpbdWarps) k_xpbd_flow(XArgs a, FlowArgs
 #pragma unroll
         for (int l = 0; l < 4; ++l) ver[l] += (uint32_t)s * deg[l];
         uint4 v[4];
-        ok = wait_vertices(at, ver, v, c.gs, c.status);
+        ok = wait_vertices(at, ver, v, c.spin_ns, c.gs, c.status);
         if (ok) {
 #pragma unroll
           for (int l = 0; l < 4; ++l) {
@@ -394,6 +396,7 @@ struct ColorArgs {
   const int32_t* off;
   int32_t n_colors;
   int32_t passes;
+  unsigned long long spin_ns;
   GridSync* gs;
   int32_t* status;
 };
@@ -407,7 +410,7 @@ __global__ void __launch_bounds__(kLT) k_xpbd_color(XArgs a, ColorArgs c) {
       const int32_t b = c.off[col], e = c.off[col + 1];
       for (int64_t i = b + tid; i < e; i += stride) xpbd_update<false>(a, XTet(a, c.order[i]));
       const bool last = s == c.passes - 1 && col == c.n_colors - 1;
-      if (!last && !pdev::grid_sync(c.gs, c.status, kSpinNs, gen)) return;
+      if (!last && !pdev::grid_sync(c.gs, c.status, c.spin_ns, gen)) return;
     }
 }
 
@@ -619,6 +622,7 @@ struct VFlowArgs {
   int32_t n_iter;
   float rho;
   const float* om;
+  unsigned long long spin_ns;
   GridSync* gs;
   int32_t* status;
 };
@@ -671,7 +675,7 @@ __global__ void __launch_bounds__(32 * kVbdWarps) k_vbd_flow(VArgs a, VFlowArgs 
           at[k] = some ? (u & 1 ? c.xa : c.xb) + (u >> 1) : nullptr;
           want[k] = n + (some ? u & 1 : 0);
         }
-        ok = wait_vertices(at, want, v, c.gs, c.status);
+        ok = wait_vertices(at, want, v, c.spin_ns, c.gs, c.status);
 #pragma unroll
         for (int k = 0; k < K; ++k)
           if (at[k])
@@ -729,6 +733,7 @@ struct VColorArgs {
   int32_t n_iter;
   float rho;
   const float* om;
+  unsigned long long spin_ns;
   GridSync* gs;
   int32_t* status;
 };
@@ -764,11 +769,11 @@ __global__ void __launch_bounds__(kLT) k_vbd_color(VArgs a, VColorArgs c) {
         if (gl == 0 && w != 0.0f) vbd_finish(a, vi, w, f, H);
       }
       const bool last = n == c.n_iter - 1 && col == c.n_colors - 1 && !cheb;
-      if (!last && !pdev::grid_sync(c.gs, c.status, kSpinNs, gen)) return;
+      if (!last && !pdev::grid_sync(c.gs, c.status, c.spin_ns, gen)) return;
     }
     if (cheb) {
       vbd_chebyshev(a, c.om[n], tid, stride);
-      if (n != c.n_iter - 1 && !pdev::grid_sync(c.gs, c.status, kSpinNs, gen)) return;
+      if (n != c.n_iter - 1 && !pdev::grid_sync(c.gs, c.status, c.spin_ns, gen)) return;
     }
   }
 }
@@ -865,7 +870,7 @@ LazyStatus::~LazyStatus() {
   if (host_) cudaFreeHost(host_);
 }
 
-void LazyStatus::record(const int32_t* dev, cudaStream_t s) {
+void LazyStatus::record(int32_t* dev, cudaStream_t s) {
   if (!host_) {
     MGPBD_CUDA(cudaMallocHost(&host_, sizeof(int32_t)));
     *host_ = 0;
@@ -873,6 +878,8 @@ void LazyStatus::record(const int32_t* dev, cudaStream_t s) {
   }
   MGPBD_CUDA(cudaMemcpyAsync(host_, dev, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   MGPBD_CUDA(cudaEventRecord(ev_, s));
+  dev_ = dev;
+  stream_ = s;
   pending_ = true;
 }
 
@@ -882,8 +889,11 @@ void LazyStatus::check(const char* what) {
   if (e == cudaErrorNotReady) return;
   MGPBD_CUDA(e);
   pending_ = false;
-  if (static_cast<uint32_t>(*host_) & MGPBD_STATUS_SYNC_TIMEOUT)
+  if (static_cast<uint32_t>(*host_) & MGPBD_STATUS_SYNC_TIMEOUT) {
+    // reported once: the next launch starts afresh
+    MGPBD_CUDA(cudaMemsetAsync(dev_, 0, sizeof(int32_t), stream_));
     throw Error(MGPBD_ECUDA, std::string(what) + ": a grid barrier wait timed out");
+  }
 }
 
 void LazyStatus::wait(const char* what) {
@@ -1020,6 +1030,7 @@ void Xpbd::update(int32_t passes) {
     f.xt = xt_.p;
     f.n_chunks = n_chunks_;
     f.passes = passes;
+    f.spin_ns = spin_ns_;
     f.gs = gs_.p;
     f.status = status_.p;
     k_flow_start<<<blocks_for(nv_), kLT, 0, s>>>(x_, xt_.p, nv_);
@@ -1033,6 +1044,7 @@ void Xpbd::update(int32_t passes) {
     c.off = offsets_.p;
     c.n_colors = n_colors_;
     c.passes = passes;
+    c.spin_ns = spin_ns_;
     c.gs = gs_.p;
     c.status = status_.p;
     void* args[] = {&a, &c};
@@ -1276,6 +1288,7 @@ void Vbd::solve() {
     f.n_iter = p_.n_iterations;
     f.rho = p_.rho;
     f.om = om_.p;
+    f.spin_ns = spin_ns_;
     f.gs = gs_.p;
     f.status = status_.p;
     if (n_steps_ > 0) {
@@ -1299,6 +1312,7 @@ void Vbd::solve() {
     c.n_iter = p_.n_iterations;
     c.rho = p_.rho;
     c.om = om_.p;
+    c.spin_ns = spin_ns_;
     c.gs = gs_.p;
     c.status = status_.p;
     void* args[] = {&a, &c};

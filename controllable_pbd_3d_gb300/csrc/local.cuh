@@ -26,17 +26,31 @@ class LazyStatus {
   LazyStatus(const LazyStatus&) = delete;
   LazyStatus& operator=(const LazyStatus&) = delete;
   ~LazyStatus();
-  void record(const int32_t* dev, cudaStream_t s);
+  void record(int32_t* dev, cudaStream_t s);
   void check(const char* what);
   void wait(const char* what);
 
  private:
   int32_t* host_ = nullptr;
   cudaEvent_t ev_ = nullptr;
+  int32_t* dev_ = nullptr;
+  cudaStream_t stream_ = nullptr;
   bool pending_ = false;
 };
 
-class Xpbd {
+// The limit of the colour kernels' waits (mgpbd_set_barrier_limit)
+class WaitLimit {
+ public:
+  void set_barrier_limit(double seconds) {
+    require(seconds >= 0.0 && seconds <= 60.0, MGPBD_EINVAL, "barrier limit must be in [0, 60] s");
+    spin_ns_ = static_cast<unsigned long long>(seconds * 1e9);
+  }
+
+ protected:
+  unsigned long long spin_ns_ = 4000000000ull;
+};
+
+class Xpbd : public WaitLimit {
  public:
   explicit Xpbd(const mgpbd_xpbd_params& p);
   void set_stream(cudaStream_t s) { stream_ = s; }
@@ -69,7 +83,7 @@ class Xpbd {
   int grid_ = 0;
 };
 
-class Vbd {
+class Vbd : public WaitLimit {
  public:
   explicit Vbd(const mgpbd_vbd_params& p);
   void set_stream(cudaStream_t s) { stream_ = s; }

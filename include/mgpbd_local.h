@@ -83,6 +83,8 @@ int mgpbd_xpbd_preupdate(mgpbd_xpbd_handle h);
 int mgpbd_xpbd_update(mgpbd_xpbd_handle h, int32_t n_passes);
 /* waits for the last update and reports its status */
 int mgpbd_xpbd_synchronize(mgpbd_xpbd_handle h);
+/* wait limit of the colour kernel, as mgpbd_set_barrier_limit */
+int mgpbd_xpbd_set_barrier_limit(mgpbd_xpbd_handle h, double seconds);
 /* device pointers of hydro_lambda / devia_lambda (nt each) */
 int mgpbd_xpbd_lambdas(mgpbd_xpbd_handle h, float** hydro, float** devia);
 /* colours of the graph colouring method (0 for the other methods) */
@@ -125,6 +127,8 @@ int mgpbd_vbd_step(mgpbd_vbd_handle h);            /* :168-172 */
 /* waits for the last solve and reports its status (solve, like update
  * above, is asynchronous on the handle's stream) */
 int mgpbd_vbd_synchronize(mgpbd_vbd_handle h);
+/* wait limit of the colour kernel, as mgpbd_set_barrier_limit */
+int mgpbd_vbd_set_barrier_limit(mgpbd_vbd_handle h, double seconds);
 /* the omega of each iteration of solve (n_iterations values, 1 where the
  * Chebyshev step is off), as the reference records it */
 int mgpbd_vbd_omegas(mgpbd_vbd_handle h, float* omegas);
