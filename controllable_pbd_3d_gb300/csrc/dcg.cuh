@@ -64,9 +64,11 @@ void launch_dcg(const JView& j, const JcgVecs& v, const DcgPlan& plan, const Dcg
 // A mesh of at most this many vertex entries (4 per 4-slot, 2 per length
 // constraint) runs on one cluster of 16 blocks, a larger one on the whole
 // grid.  A cluster's exchanges go through distributed shared memory, a grid's
-// through L2, but it has a tenth of the SMs.  Measured on cubes of n^3 hexes,
-// length + volume, us per CG iteration cluster / grid: n = 10 (34k entries)
-// 27 / 39, 14 (91k) 34 / 40, 17 (163k) 42 / 38, 20 (263k) 71 / 39.
+// through L2, but it has a tenth of the SMs.  Measured on cubes of n^3 hexes, us
+// per CG iteration cluster / grid, length + volume: n = 10 (34k entries) 27 / 34,
+// 14 (91k) 35 / 33, 17 (163k) 43 / 35, 20 (263k) 73 / 37; on another box the grid
+// took 39 / 40 / 38 / 39 of these.  ARAP: 10 (20k) 23 / 32, 14 (55k) 27 / 30, 17
+// (98k) 31 / 32, 18 (117k) 36 / 32, 20 (160k) 42 / 33.
 constexpr double kDClusterEntries = 120e3;
 // From this many constraints a block on it runs 768 threads, below 512: more
 // warps hide more of the shared-memory latency, fewer have less to issue

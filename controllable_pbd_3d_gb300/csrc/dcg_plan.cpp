@@ -102,7 +102,11 @@ DcgPlaces dcg_places(int32_t nprob, int32_t nblk) {
 // the bodies that everything else waits for can have more SMs than the others:
 // 16 bodies of 6..18 hexes a side, compliances 1e-7..1e-5, three draws: 93 / 83
 // / 109 ms a substep, on clusters of 8 each 132 / 111 / 169; 24 bodies of 8..17:
-// 105 / 114 / 99 and 149 / 167 / 161.
+// 105 / 114 / 99 and 149 / 167 / 161.  The model is of length + volume bodies in
+// that range; ARAP packs and softer ones follow the same rule (ms a substep, the
+// pack in lockstep over the grid / by this rule): ARAP, 16 bodies of 6..18,
+// 1e-7..1e-5 257 / 72, 1e-5..1e-3 39 / 12; 40 of 4..12 249 / 61 and 40 / 11;
+// length + volume, 16 of 6..18, 1e-5..1e-3 34 / 10.
 std::vector<DcgPlaces> dcg_place_bodies(const std::vector<double>& entries,
                                         const std::vector<double>& softness, int n16, int n8, int n4) {
   constexpr int kHardness = 16;
